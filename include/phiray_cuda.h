@@ -431,15 +431,21 @@ int32_t phx_tracer_create_instanced(phx_ctx ctx, const phx_scene* scene, const p
  * has no instances. Stream-ordered. */
 int32_t phx_tracer_reinstance(phx_tracer tr, const phx_instance* insts, uint32_t ninsts);
 int32_t phx_tracer_destroy(phx_tracer tr);
-/* Which kernel traces a frame. All compute the same image bit for bit:
- * PHX_KERNEL_MEGAKERNEL (the default) is shade.wgsl's main as one thread per
- * pixel with the walk called from every site that traces;
- * PHX_KERNEL_STATE_MACHINE is a persistent kernel whose lanes take pixels from a
- * counter and run the bounce loop as a state machine around one walk, so
- * lanes at different points of their paths still traverse together. Its
- * _6 and _8 forms cap registers for 6 or 8 resident 128-thread blocks per
- * SM (more warps, path state spilled to local memory); phx_tracer_autotune
- * times them on the scene and keeps the fastest. */
+/* Which kernel traces a frame. All compute the same image bit for bit. A
+ * tracer whose kernel was neither set nor autotuned takes the pooled render
+ * where it can run and PHX_KERNEL_MEGAKERNEL elsewhere.
+ * PHX_KERNEL_MEGAKERNEL is shade.wgsl's main as one thread per pixel with the
+ * walk called from every site that traces;
+ * PHX_KERNEL_STATE_MACHINE and its _6 and _8 forms are the pooled render with
+ * blocks of 512, 256 and 128 threads: each block keeps a pool of sample
+ * paths in device memory and alternates between tracing all of their rays
+ * and shading all of their hits by kind. It runs single-instance scenes whose
+ * materials transmit no light, not inside a graph capture (but for a batch's
+ * own) nor with adaptive sampling; PHX_KERNEL_MEGAKERNEL runs the other
+ * frames. Scenes of instances and frames with the floor grid take a
+ * persistent kernel under these ids, whose lanes take pixels from a counter
+ * and run the bounce loop as a state machine around one walk.
+ * phx_tracer_autotune times them on the scene and keeps the fastest. */
 #define PHX_KERNEL_MEGAKERNEL 0u
 #define PHX_KERNEL_STATE_MACHINE 1u
 #define PHX_KERNEL_STATE_MACHINE_6 2u

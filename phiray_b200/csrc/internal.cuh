@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <cstdarg>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -37,6 +38,11 @@ struct DevMem {
     ~DevMem() { release(); }
 };
 
+// The pooled render's path states and sample terms (render_pool.cuh).
+struct PoolScratch {
+    DevMem state, out;
+};
+
 struct Ctx {
     int device = 0;
     int sms = 148;
@@ -46,6 +52,8 @@ struct Ctx {
     uint32_t* status = nullptr;     // device status word
     cudaMemPool_t pool = nullptr;   // device memory of the context's objects
     DevMem denoise_scratch;         // guide and ping-pong planes of phx_denoise
+    PoolScratch path_pool;          // the pooled render's buffers
+    std::mutex path_pool_lock;      // from sizing them to the launches that use them
     int live = 0;                   // buffers, passes, BVHs, tracers not yet freed
 };
 

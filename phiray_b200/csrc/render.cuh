@@ -42,18 +42,31 @@ struct WfBuffers {
     uint32_t* host_lens;  // pinned, 3 words
 };
 
+// The pooled render's buffers (render_pool.cuh): the state of `slots` paths,
+// and the terms of `spp` samples of every pixel of the launch.
+struct PoolBuffers {
+    uint32_t* pools;
+    uint64_t slots;
+    uint32_t* out;
+    uint32_t spp;
+};
+// Bytes of one path's state; words of one sample's terms.
+size_t pool_slot_bytes();
+uint32_t pool_out_words();
+// The pooled render, by kernel id 1-3 (render_pool.cu).
+int32_t render_pooled(uint32_t kernel, bool stats, const RenderLaunch& L, const PoolBuffers& B);
+
 constexpr uint32_t WF_SLOTS = 1u << 20;  // path slots of the wavefront render (at most)
 // 32-bit words of one wavefront path slot (Path, Sums, phase).
 uint32_t wf_slot_words();
 
 // The single-instance render kernels by id: ids 0 and 4-8 (render_flat_a.cu),
-// 9-12 (render_flat_b.cu), 13-15 (render_flat_c.cu), 17-19 (render_flat_r.cu),
-// 1-3 (render_sm.cu).
+// 9-12 (render_flat_b.cu), 13-15 (render_flat_c.cu), 17-19 (render_flat_r.cu);
+// 1-3 are render_pooled below.
 int32_t render_flat_a(uint32_t kernel, bool stats, const RenderLaunch& L);
 int32_t render_flat_b(uint32_t kernel, bool stats, const RenderLaunch& L);
 int32_t render_flat_c(uint32_t kernel, bool stats, const RenderLaunch& L);
 int32_t render_flat_r(uint32_t kernel, bool stats, const RenderLaunch& L);
-int32_t render_flat_sm(uint32_t kernel, bool stats, const RenderLaunch& L);
 // Scenes of instances and frames with the floor grid (render_full.cu).
 int32_t render_full(uint32_t kernel, bool stats, const RenderLaunch& L);
 // The wavefront render (render_wf.cu).
@@ -89,7 +102,7 @@ struct Sums {
 };
 
 __device__ __forceinline__ float srgb_to_linear1(float c) {
-    return c <= 0.04045f ? c / 12.92f : pm_pow((c + 0.055f) / 1.055f, 2.4f);
+    return c <= 0.04045f ? dv(c, 12.92f) : pow_of(dv(c + 0.055f, 1.055f), 2.4f);
 }
 
 __device__ __forceinline__ f3 env_at(const Frame& F) { return F.env; }
@@ -98,22 +111,15 @@ __device__ __forceinline__ f3 env_at(const Frame& F) { return F.env; }
 template <int STATS>
 __device__ __noinline__ f3 direct(const Scene& S, const Frame& F, const Surf& s, uint32_t& seed, bool with_env,
                                   f3 sun, Count& cnt) {
-    const bool rig = uses_rig(F);
-    f3 sum = rig ? rig_fill(F, s) : mk(0.0f);
-    for (uint32_t k = 0; k < 4u; k++) {
-        Shadowed q = unshadowed();
-        if (k == 0u) {
-            q = rig ? rig_query(F, 0u, s, seed, sun) : lamp_query(F, s, seed);
-        } else if (k == 1u) {
-            if (rig) q = rig_query(F, 1u, s, seed, sun);
-        } else if (k == 2u) {
-            q = glow_query<STATS>(S, s, seed);
-        }
-        // k == 3: env_query needs an environment image's table (env_cdf),
-        // which the host refuses; it returns unshadowed without a draw.
-        if (maxc(q.c) > 0.0f) {
-            const float vis = trace<STATS>(S, s.pos, q.dir, q.dist, true, cnt).tri != NONE ? 0.0f : 1.0f;
-            sum += q.c * vis;
+    f3 sum = uses_rig(F) ? rig_fill(F, s) : mk(0.0f);
+#pragma unroll 1
+    for (uint32_t k = 0; k < 3u; k++) {
+        const Query q = light_query<STATS>(S, F, k, s, seed, sun);
+        if (!q.met) continue;
+        const f3 c = brdf(s, q.l, q.e) * q.scale;
+        if (maxc(c) > 0.0f) {
+            const float vis = trace<STATS>(S, s.pos, q.l, q.dist, true, cnt).tri != NONE ? 0.0f : 1.0f;
+            sum += c * vis;
         }
     }
     return sum;
@@ -125,7 +131,7 @@ __device__ __forceinline__ f3 glow_mis(const Scene& S, const Geo& g, f3 emit, co
     const float chance = lamp_chance<M>(S, h.tri, (M & MODE_FULL) ? h.inst : 0u);
     if (chance <= 0.0f) return emit;
     const f3 cr = cross(g.b - g.a, g.c - g.a);
-    const float pl = chance * h.t * h.t / fmaxf(0.5f * length(cr) * fabsf(dot(normalize(cr), dir)), 1e-8f);
+    const float pl = chance * h.t * h.t / fmaxf(0.5f * length(cr) * fabsf(dot(unit(cr), dir)), 1e-8f);
     const float pb = fmaxf(dot(from_n, dir), 0.0f) / PI;
     return emit * pb * pb / fmaxf(pb * pb + pl * pl, 1e-12f);
 }
@@ -150,10 +156,11 @@ __device__ __forceinline__ f3 indirect(const Scene& S, const Frame& F, f3 pos, f
     bool through = false;
     f3 dir = mk(0.0f, 0.0f, 1.0f);
     float pb = 1.0f;
+#pragma unroll 1
     for (uint32_t b = 0; b < depth; b++) {
         if (!through) {
             dir = cosine_dir(nrm, seed);
-            pb = fmaxf(dot(nrm, dir), 0.0f) / PI;
+            pb = dv(fmaxf(dot(nrm, dir), 0.0f), PI);
         }
         through = false;
         min_pdf = fminf(min_pdf, pb);
@@ -165,7 +172,7 @@ __device__ __forceinline__ f3 indirect(const Scene& S, const Frame& F, f3 pos, f
         if (!bounce) break;
         const Geo g = geo_at<STATS>(S, h.tri, (STATS & MODE_FULL) ? h.inst : 0u);
         const Mat t = mat_at(S, g.mat);
-        const f3 ng0 = normalize(cross(g.b - g.a, g.c - g.a));
+        const f3 ng0 = unit(cross(g.b - g.a, g.c - g.a));
         const f3 ng = dot(ng0, dir) < 0.0f ? ng0 : -ng0;
         const f3 hit = org + dir * h.t + ng * (F.eps + h.t * 1e-5f);
         const f3 base = vmax(mk(t.color.x, t.color.y, t.color.z), mk(0.0f));
@@ -190,7 +197,7 @@ __device__ __forceinline__ f3 indirect(const Scene& S, const Frame& F, f3 pos, f
         if (b + 1u < depth) {
             const float keep = clampf(maxc(thr), 0.0f, 0.95f);
             if (keep < 1e-4f || rnd(seed) > keep) break;
-            thr = thr / keep;
+            thr = dv(thr, keep);
         }
         org = hit;
         nrm = ng;
@@ -204,7 +211,7 @@ __device__ __forceinline__ f3 bounce_light(const Scene& S, const Frame& F, const
                                            uint32_t& seed, f3 sun, Count& cnt) {
     const Geo g = geo_at<STATS>(S, h.tri, (STATS & MODE_FULL) ? h.inst : 0u);
     const Mat t = mat_at(S, g.mat);
-    const f3 ng0 = normalize(cross(g.b - g.a, g.c - g.a));
+    const f3 ng0 = unit(cross(g.b - g.a, g.c - g.a));
     const f3 ng = dot(ng0, d) < 0.0f ? ng0 : -ng0;
     const f3 pos = org + d * h.t + ng * (F.eps + h.t * 1e-5f);
     const f3 base = vmax(mk(t.color.x, t.color.y, t.color.z), mk(0.0f));
@@ -227,18 +234,18 @@ struct CamRay {
 };
 
 __device__ __forceinline__ CamRay camera_ray(const Frame& F, uint32_t i, uint32_t& seed) {
-    const float su = ((float)(i % F.w) + 0.5f) / (float)F.w - 0.5f;
-    const float sv = ((float)(i / F.w) + 0.5f) / (float)F.h - 0.5f;
+    const float su = dv((float)(i % F.w) + 0.5f, (float)F.w) - 0.5f;
+    const float sv = dv((float)(i / F.w) + 0.5f, (float)F.h) - 0.5f;
     const float jox = rnd(seed) - 0.5f;
     const float joy = rnd(seed) - 0.5f;
-    const float jx = jox / (float)F.w;
-    const float jy = joy / (float)F.h;
-    const float vx = (su + jx - F.pan_x) / F.scale;
-    const float vy = -((sv + jy) / F.aspect - F.pan_y) / F.scale;
+    const float jx = dv(jox, (float)F.w);
+    const float jy = dv(joy, (float)F.h);
+    const float vx = dv(su + jx - F.pan_x, F.scale);
+    const float vy = dv(-(dv(sv + jy, F.aspect) - F.pan_y), F.scale);
     CamRay r;
     if (F.persp != 0u) {
         r.o = F.pivot + F.back * (F.dist / F.units);
-        r.d = normalize(F.right * vx + F.up * vy - F.back * F.dist);
+        r.d = unit(F.right * vx + F.up * vy - F.back * F.dist);
     } else {
         r.o = F.pivot + (F.right * vx + F.up * vy + F.back * 1.0e4f) / F.units;
         r.d = -F.back;
@@ -301,12 +308,12 @@ __device__ void sample(const Scene& S, const Frame& F, uint32_t i, uint32_t fram
         const Mat t = mat_at(S, g.mat);
         const float w = 1.0f - h.u - h.v;
         const f3 hit = o + d * h.t;
-        const f3 ngw = normalize(cross(g.b - g.a, g.c - g.a));
+        const f3 ngw = unit(cross(g.b - g.a, g.c - g.a));
         const f3 ng0 = g.mirror ? -ngw : ngw;  // world_ng (layout.wgsl:97-101)
         const bool front = dot(ng0, d) < 0.0f;
         const f3 ng = front ? ng0 : -ng0;
         f3 n = g.na * w + g.nb * h.u + g.nc * h.v;
-        n = dot(n, n) > 1e-12f ? normalize(n) * (front ? 1.0f : -1.0f) : ng;
+        n = dot(n, n) > 1e-12f ? unit(n) * (front ? 1.0f : -1.0f) : ng;
         if (dot(n, -d) < 0.0f) n = ng;
         const f3 off = ng * hit_lift(F, h.t);
         const f3 past = ng * through_lift(F, hit, h.t);
@@ -348,23 +355,23 @@ __device__ void sample(const Scene& S, const Frame& F, uint32_t i, uint32_t fram
         const f3 diffuse_weight = vmix(s.albedo, s.albedo * s.sss_tint, bleed) * opaque;
         const f3 lw = mk(0.2126f, 0.7152f, 0.0722f);
         const float ndv = fmaxf(dot(n, -d), 1e-4f);
-        const f3 gloss_guess = s.f0 + (mk(1.0f) - s.f0) * pm_pow(1.0f - ndv, 5.0f);
+        const f3 gloss_guess = s.f0 + (mk(1.0f) - s.f0) * pow_of(1.0f - ndv, 5.0f);
         const float pd = dot(vmax(diffuse_weight, mk(0.0f)), lw);
         const float pg = glossy_on ? dot(gloss_guess, lw) : 0.0f;
-        float p_diffuse = pd + pg > 0.0f ? pd / (pd + pg) : 1.0f;
+        float p_diffuse = pd + pg > 0.0f ? dv(pd, pd + pg) : 1.0f;
         if (pd > 0.0f && pg > 0.0f) p_diffuse = clampf(p_diffuse, 0.15f, 0.85f);
         const bool take_diffuse = rnd(seed) < p_diffuse;
         if (take_diffuse && pd > 0.0f)
             bounced += diffuse_weight * indirect<STATS>(S, F, pos, n, seed, diffuse_on, sun, cnt) / p_diffuse;
         const f3 v = -d;
-        const f3 tx = normalize(onb(n, 1.0f, 0.0f));
+        const f3 tx = unit(onb(n, 1.0f, 0.0f));
         const f3 ty = cross(n, tx);
         const float ggx_a = s.rough * s.rough;
         const f3 wi_local = mk(dot(v, tx), dot(v, ty), dot(v, n));
         const float r1 = rnd(seed);
         const float r2 = rnd(seed);
         const f3 h_local = ggx_sample_vndf(wi_local, ggx_a, r1, r2);
-        const f3 hw = normalize(tx * h_local.x + ty * h_local.y + n * h_local.z);
+        const f3 hw = unit(tx * h_local.x + ty * h_local.y + n * h_local.z);
         const f3 refl = reflect(d, hw);
         const float cos_hi = fmaxf(dot(hw, v), 0.0f);
         const float cos_no = dot(n, refl);
@@ -392,7 +399,7 @@ __device__ void sample(const Scene& S, const Frame& F, uint32_t i, uint32_t fram
             o = hit - past;
             thr *= mk(sqrtf(base.x), sqrtf(base.y), sqrtf(base.z)) * tw * (mk(1.0f) - fres);
         }
-        d = cone_dir(normalize(nd), s.rough * s.rough, seed);
+        d = cone_dir(unit(nd), s.rough * s.rough, seed);
         if (maxc(thr) < 0.01f) break;
     }
     // emit (util.wgsl:101-145); the overlay was added at the first hit.
@@ -774,20 +781,15 @@ __device__ __forceinline__ uint32_t set_ray(Path& P, f3 o, f3 d, float tmax, boo
 template <int STATS>
 __device__ __forceinline__ uint32_t start_direct(const Scene& S, const Frame& F, Path& P, const Surf& s, uint32_t cont,
                                                  f3 sun) {
-    const bool rig = uses_rig(F);
-    P.dsum = rig ? rig_fill(F, s) : mk(0.0f);
+    P.dsum = uses_rig(F) ? rig_fill(F, s) : mk(0.0f);
     P.qn = 0;
-    for (uint32_t k = 0; k < 4u; k++) {
-        Shadowed q = unshadowed();
-        if (k == 0u) {
-            q = rig ? rig_query(F, 0u, s, P.seed, sun) : lamp_query(F, s, P.seed);
-        } else if (k == 1u) {
-            if (rig) q = rig_query(F, 1u, s, P.seed, sun);
-        } else if (k == 2u) {
-            q = glow_query<STATS>(S, s, P.seed);
-        }
-        if (maxc(q.c) > 0.0f) {
-            P.put(P.qn, q.c, q.dir, q.dist);
+#pragma unroll 1
+    for (uint32_t k = 0; k < 3u; k++) {
+        const Query q = light_query<STATS>(S, F, k, s, P.seed, sun);
+        if (!q.met) continue;
+        const f3 c = brdf(s, q.l, q.e) * q.scale;
+        if (maxc(c) > 0.0f) {
+            P.put(P.qn, c, q.l, q.dist);
             P.qn++;
         }
     }
@@ -851,12 +853,12 @@ __device__ __forceinline__ uint32_t step(const Scene& S, const Frame& F, Path& P
             const Mat t = mat_at(S, g.mat);
             const float w = 1.0f - h.u - h.v;
             const f3 hit = P.o + P.d * h.t;
-            const f3 ngw = normalize(cross(g.b - g.a, g.c - g.a));
+            const f3 ngw = unit(cross(g.b - g.a, g.c - g.a));
             const f3 ng0 = g.mirror ? -ngw : ngw;  // world_ng
             const bool front = dot(ng0, P.d) < 0.0f;
             const f3 ng = front ? ng0 : -ng0;
             f3 n = g.na * w + g.nb * h.u + g.nc * h.v;
-            n = dot(n, n) > 1e-12f ? normalize(n) * (front ? 1.0f : -1.0f) : ng;
+            n = dot(n, n) > 1e-12f ? unit(n) * (front ? 1.0f : -1.0f) : ng;
             if (dot(n, -P.d) < 0.0f) n = ng;
             const f3 off = ng * hit_lift(F, h.t);
             const f3 past = ng * through_lift(F, hit, h.t);
@@ -913,10 +915,10 @@ __device__ __forceinline__ uint32_t step(const Scene& S, const Frame& F, Path& P
             P.diffuse_weight = vmix(s.albedo, s.albedo * s.sss_tint, bleed) * P.opaque;
             const f3 lw = mk(0.2126f, 0.7152f, 0.0722f);
             const float ndv = fmaxf(dot(s.n, -P.d), 1e-4f);
-            const f3 gloss_guess = s.f0 + (mk(1.0f) - s.f0) * pm_pow(1.0f - ndv, 5.0f);
+            const f3 gloss_guess = s.f0 + (mk(1.0f) - s.f0) * pow_of(1.0f - ndv, 5.0f);
             const float pd = dot(vmax(P.diffuse_weight, mk(0.0f)), lw);
             const float pg = dot(gloss_guess, lw);
-            float p_diffuse = pd + pg > 0.0f ? pd / (pd + pg) : 1.0f;
+            float p_diffuse = pd + pg > 0.0f ? dv(pd, pd + pg) : 1.0f;
             if (pd > 0.0f && pg > 0.0f) p_diffuse = clampf(p_diffuse, 0.15f, 0.85f);
             P.p_diffuse = p_diffuse;
             P.take_diffuse = rnd(P.seed) < p_diffuse ? 1u : 0u;
@@ -970,7 +972,7 @@ __device__ __forceinline__ uint32_t step(const Scene& S, const Frame& F, Path& P
             const Geo g = geo_at<STATS>(S, h.tri, (STATS & MODE_FULL) ? h.inst : 0u);
             const Mat t = mat_at(S, g.mat);
             const f3 dir = P.idir;
-            const f3 ng0 = normalize(cross(g.b - g.a, g.c - g.a));
+            const f3 ng0 = unit(cross(g.b - g.a, g.c - g.a));
             const f3 ng = dot(ng0, dir) < 0.0f ? ng0 : -ng0;
             const f3 hit = P.iorg + dir * h.t + ng * (F.eps + h.t * 1e-5f);
             const f3 base = vmax(mk(t.color.x, t.color.y, t.color.z), mk(0.0f));
@@ -1026,14 +1028,14 @@ __device__ __forceinline__ uint32_t step(const Scene& S, const Frame& F, Path& P
         case PH_GLOSSY: {
             const Surf& s = P.s;
             const f3 v = -P.d;
-            const f3 tx = normalize(onb(s.n, 1.0f, 0.0f));
+            const f3 tx = unit(onb(s.n, 1.0f, 0.0f));
             const f3 ty = cross(s.n, tx);
             P.ggx_a = s.rough * s.rough;
             const f3 wi_local = mk(dot(v, tx), dot(v, ty), dot(v, s.n));
             const float r1 = rnd(P.seed);
             const float r2 = rnd(P.seed);
             const f3 h_local = ggx_sample_vndf(wi_local, P.ggx_a, r1, r2);
-            const f3 hw = normalize(tx * h_local.x + ty * h_local.y + s.n * h_local.z);
+            const f3 hw = unit(tx * h_local.x + ty * h_local.y + s.n * h_local.z);
             const f3 refl = reflect(P.d, hw);
             const float cos_hi = fmaxf(dot(hw, v), 0.0f);
             P.cos_no = dot(s.n, refl);
@@ -1051,7 +1053,7 @@ __device__ __forceinline__ uint32_t step(const Scene& S, const Frame& F, Path& P
             const Geo g = geo_at<STATS>(S, h.tri, (STATS & MODE_FULL) ? h.inst : 0u);
             const Mat t = mat_at(S, g.mat);
             const f3 d = P.rd;
-            const f3 ng0 = normalize(cross(g.b - g.a, g.c - g.a));
+            const f3 ng0 = unit(cross(g.b - g.a, g.c - g.a));
             const f3 ng = dot(ng0, d) < 0.0f ? ng0 : -ng0;
             const f3 pos = P.ro + d * h.t + ng * (F.eps + h.t * 1e-5f);
             const f3 base = vmax(mk(t.color.x, t.color.y, t.color.z), mk(0.0f));
@@ -1087,7 +1089,7 @@ __device__ __forceinline__ uint32_t step(const Scene& S, const Frame& F, Path& P
                 P.o = P.hit - P.past;
                 P.thr *= mk(sqrtf(P.base.x), sqrtf(P.base.y), sqrtf(P.base.z)) * tw * (mk(1.0f) - P.fres);
             }
-            P.d = cone_dir(normalize(nd), P.s.rough * P.s.rough, P.seed);
+            P.d = cone_dir(unit(nd), P.s.rough * P.s.rough, P.seed);
             if (maxc(P.thr) < 0.01f) return PH_EMIT_END;
             P.bounce++;
             if (P.bounce < passes) return set_ray(P, P.o, P.d, INF, false, PH_ON_BOUNCE);
@@ -1399,30 +1401,6 @@ int32_t launch_mk(const RenderLaunch& L) {
                                                                      L.counters);
     return cuda_check(cudaGetLastError(), "render");
 }
-
-// Single-instance scenes: every form the autotuner times.
-template <int M>
-int32_t launch_flat(uint32_t kernel, const RenderLaunch& L) {
-    switch (kernel) {
-        case PHX_KERNEL_STATE_MACHINE: return launch_sm<M, 4>(L);
-        case PHX_KERNEL_STATE_MACHINE_6: return launch_sm<M, 6>(L);
-        case PHX_KERNEL_STATE_MACHINE_8: return launch_sm<M, 8>(L);
-        case PHX_KERNEL_MEGAKERNEL_3: return launch_mk<M, 3, false>(L);
-        case PHX_KERNEL_MEGAKERNEL_2: return launch_mk<M, 2, false>(L);
-        case PHX_KERNEL_MEGAKERNEL_SYNC: return launch_mk<M, 4, true>(L);
-        case PHX_KERNEL_MEGAKERNEL_2_SYNC: return launch_mk<M, 2, true>(L);
-        case PHX_KERNEL_MEGAKERNEL_5: return launch_mk<M, 5, false>(L);
-        case PHX_KERNEL_MEGAKERNEL_6: return launch_mk<M, 6, false>(L);
-        case PHX_KERNEL_MEGAKERNEL_6_SYNC: return launch_mk<M, 6, true>(L);
-        case PHX_KERNEL_MEGAKERNEL_8: return launch_mk<M, 8, false>(L);
-        case PHX_KERNEL_MEGAKERNEL_8_SYNC: return launch_mk<M, 8, true>(L);
-        case PHX_KERNEL_MEGAKERNEL_10_SYNC: return launch_mk<M, 10, true>(L);
-        case PHX_KERNEL_MEGAKERNEL_12_SYNC: return launch_mk<M, 12, true>(L);
-        case PHX_KERNEL_MEGAKERNEL_16_SYNC: return launch_mk<M, 16, true>(L);
-        default: return launch_mk<M, 4, false>(L);
-    }
-}
-
 
 // The wavefront render: each pass runs the logic kernel over every path
 // slot, then walks the primary, extension and shadow queues; the host reads

@@ -230,7 +230,11 @@ int32_t phx_ctx_destroy(phx_ctx ctx) {
         g_ctxs.erase(&c);
     }
     if (t_current == &c) t_current = nullptr;
-    if (c.stream) c.denoise_scratch.release();
+    if (c.stream) {
+        c.denoise_scratch.release();
+        c.path_pool.state.release();
+        c.path_pool.out.release();
+    }
     if (c.stream) cudaStreamSynchronize(c.stream);
     if (c.own) cudaStreamSynchronize(c.own);
     if (c.status) cudaFree(c.status);

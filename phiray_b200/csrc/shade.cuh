@@ -6,7 +6,7 @@
 // env_at, visible, lamp_query, area_query, spot_mask, lamp_reach,
 // lamp_chance, glow_query, hit_lift, through_lift), brdf.wgsl (GGX, Surf,
 // fresnel_of, dielectric_f0, under_layer(_real), env_brdf, brdf_w,
-// ggx_pdf, glossy_floor), util.wgsl (hash, rnd, unit_disk), view.wgsl.
+// glossy_floor), util.wgsl (hash, rnd, unit_disk), view.wgsl.
 //
 // A scene is either one identity instance (every mesh in world space: the
 // reference's top-tree walk plus one trace_blas is then a single walk of the
@@ -138,6 +138,30 @@ struct Frame {
     uint32_t grid_hide;
 };
 
+// ---- shared code kept out of line ----
+//
+// Instruction fetch bounds the render kernels: with every helper inlined the
+// megakernel's code was 390 KB, and "no instruction" was its largest stall
+// (11.7 warps an issue against 7.6 waiting on memory). So the long helpers
+// that several sites use — a normalise is three IEEE divides and a square
+// root — are one copy each: 190 KB, and 16 spp of the 1.3 M-face mesh at
+// 1080p went from 48.7 to 46.1 ms in the 16-block form, 67.4 to 56.9 in the
+// 4-block one.
+static __device__ __noinline__ f3 unit(f3 a) { return normalize(a); }
+// The IEEE divide and square root (each some ten instructions and a branch
+// to its slow path wherever it is inlined).
+static __device__ __noinline__ float dv(float a, float b) { return a / b; }
+static __device__ __noinline__ f3 dv(f3 a, float b) { return a / b; }
+static __device__ __noinline__ float rt(float x) { return sqrtf(x); }
+static __device__ __noinline__ float pow_of(float x, float y) { return pm_pow(x, y); }
+static __device__ __noinline__ float exp2_of(float x) { return pm_exp2(x); }
+// (sine, cosine)
+static __device__ __noinline__ float2 sincos_of(float x) {
+    float2 r;
+    pm_sincos(x, &r.x, &r.y);
+    return r;
+}
+
 // ---- util.wgsl ----
 
 __device__ __forceinline__ uint32_t hash(uint32_t x) {
@@ -158,14 +182,13 @@ __device__ __forceinline__ float2 unit_disk(float ru, float rv) {
     float r, phi;
     if (a * a > b * b) {
         r = a;
-        phi = (PI / 4.0f) * (b / a);
+        phi = (PI / 4.0f) * dv(b, a);
     } else {
         r = b;
-        phi = (PI / 2.0f) - (PI / 4.0f) * (a / b);
+        phi = (PI / 2.0f) - (PI / 4.0f) * dv(a, b);
     }
-    float s, c;
-    pm_sincos(phi, &s, &c);
-    return make_float2(r * c, r * s);
+    const float2 sc = sincos_of(phi);
+    return make_float2(r * sc.y, r * sc.x);
 }
 
 // ---- bvh.wgsl ----
@@ -328,6 +351,7 @@ __device__ __forceinline__ bool walk_tree(const Tree S, f3 o, f3 d, Hit& best, b
     uint32_t nd = S.root;
     for (;;) {
         if (nd & LEAF) {
+#pragma unroll 1
             for (uint32_t id = nd & ~LEAF; id < S.nslots; id++) {
                 const float4 A = __ldg(S.tris + 3 * (size_t)id);
                 const float4 B = __ldg(S.tris + 3 * (size_t)id + 1);
@@ -500,6 +524,7 @@ __device__ __forceinline__ Hit walk_wide(const Tree& T, const float4* __restrict
     uint32_t nd = (T.root & LEAF) ? T.root : 0u;
     for (;;) {
         if (nd & LEAF) {
+#pragma unroll 1
             for (uint32_t id = nd & ~LEAF; id < T.nslots; id++) {
                 const float4 A = __ldg(T.tris + 3 * (size_t)id);
                 const float4 B = __ldg(T.tris + 3 * (size_t)id + 1);
@@ -692,31 +717,31 @@ struct Surf {
 };
 
 __device__ __forceinline__ float ggx_lambda(float alpha2, float cos_n) {
-    const float t = alpha2 * fmaxf(1.0f / fmaxf(cos_n * cos_n, 1e-8f) - 1.0f, 0.0f);
-    return 0.5f * (sqrtf(1.0f + t) - 1.0f);
+    const float t = alpha2 * fmaxf(dv(1.0f, fmaxf(cos_n * cos_n, 1e-8f)) - 1.0f, 0.0f);
+    return 0.5f * (rt(1.0f + t) - 1.0f);
 }
 
 __device__ __forceinline__ f3 ggx_sample_vndf(f3 wi, float alpha, float r1, float r2) {
-    const f3 wi_ = normalize(mk(alpha * wi.x, alpha * wi.y, wi.z));
+    const f3 wi_ = unit(mk(alpha * wi.x, alpha * wi.y, wi.z));
     const float lensq = wi_.x * wi_.x + wi_.y * wi_.y;
     f3 t1, t2;
     if (lensq > 1e-7f) {
-        t1 = mk(-wi_.y, wi_.x, 0.0f) / sqrtf(lensq);
+        t1 = dv(mk(-wi_.y, wi_.x, 0.0f), rt(lensq));
         t2 = cross(wi_, t1);
     } else {
         t1 = mk(1.0f, 0.0f, 0.0f);
         t2 = mk(0.0f, 1.0f, 0.0f);
     }
     float2 t = unit_disk(r1, r2);
-    t.y = mixf(sqrtf(fmaxf(1.0f - t.x * t.x, 0.0f)), t.y, 0.5f * (1.0f + wi_.z));
-    const f3 h_ = t1 * t.x + t2 * t.y + wi_ * sqrtf(fmaxf(0.0f, 1.0f - t.x * t.x - t.y * t.y));
-    return normalize(mk(alpha * h_.x, alpha * h_.y, fmaxf(0.0f, h_.z)));
+    t.y = mixf(rt(fmaxf(1.0f - t.x * t.x, 0.0f)), t.y, 0.5f * (1.0f + wi_.z));
+    const f3 h_ = t1 * t.x + t2 * t.y + wi_ * rt(fmaxf(0.0f, 1.0f - t.x * t.x - t.y * t.y));
+    return unit(mk(alpha * h_.x, alpha * h_.y, fmaxf(0.0f, h_.z)));
 }
 
 __device__ __forceinline__ float ggx_weight(float alpha2, float cos_ni, float cos_no) {
     const float li = ggx_lambda(alpha2, cos_ni);
     const float lo = ggx_lambda(alpha2, cos_no);
-    return (1.0f + li) / (1.0f + li + lo);
+    return dv(1.0f + li, 1.0f + li + lo);
 }
 
 __device__ __forceinline__ Surf plain_surf(f3 pos, f3 n, f3 v, f3 albedo, f3 f0, float rough) {
@@ -728,17 +753,17 @@ __device__ __forceinline__ float fresnel_dielectric_cos(float cosi, float eta) {
     const float c = fabsf(cosi);
     float g = eta * eta - 1.0f + c * c;
     if (g <= 0.0f) return 1.0f;
-    g = sqrtf(g);
-    const float a = (g - c) / (g + c);
-    const float b = (c * (g + c) - 1.0f) / (c * (g - c) + 1.0f);
+    g = rt(g);
+    const float a = dv(g - c, g + c);
+    const float b = dv(c * (g + c) - 1.0f, c * (g - c) + 1.0f);
     return 0.5f * a * a * (1.0f + b * b);
 }
 
-__device__ __forceinline__ f3 fresnel_of(const Surf& s, float cs) {
-    const float schlick = pm_pow(1.0f - cs, 5.0f);
+static __device__ __noinline__ f3 fresnel_of(const Surf& s, float cs) {
+    const float schlick = pow_of(1.0f - cs, 5.0f);
     f3 f = s.f0 + (mk(1.0f) - s.f0) * schlick;
     if (s.eta > 1.0f && s.dielectric > 0.0f) {
-        const float r = (s.eta - 1.0f) / (s.eta + 1.0f);
+        const float r = dv(s.eta - 1.0f, s.eta + 1.0f);
         const float face_on = r * r;
         f += mk(s.dielectric * (fresnel_dielectric_cos(cs, s.eta) - face_on - (1.0f - face_on) * schlick));
     }
@@ -747,7 +772,7 @@ __device__ __forceinline__ f3 fresnel_of(const Surf& s, float cs) {
 
 __device__ __forceinline__ f3 scatter_tint(f3 radius) {
     const float m = fmaxf(fmaxf(radius.x, radius.y), fmaxf(radius.z, 1e-6f));
-    return vmix(mk(1.0f), radius / m, 0.85f);
+    return vmix(mk(1.0f), dv(radius, m), 0.85f);
 }
 
 __device__ __forceinline__ float scatter_bleed(float weight, f3 radius) {
@@ -758,19 +783,19 @@ __device__ __forceinline__ float scatter_bleed(float weight, f3 radius) {
 __device__ __forceinline__ float charlie(float nh, float rough) {
     const float inv = 1.0f / fmaxf(rough * rough, 0.005f);
     const float sin2 = fmaxf(1.0f - nh * nh, 0.0f);
-    return (2.0f + inv) * pm_pow(sin2, inv * 0.5f) / (2.0f * PI);
+    return (2.0f + inv) * pow_of(sin2, inv * 0.5f) / (2.0f * PI);
 }
 
 __device__ __forceinline__ f3 env_brdf(f3 f0, float rough, float nv) {
     const float rx = rough * -1.0f + 1.0f, ry = rough * -0.0275f + 0.0425f, rz = rough * -0.572f + 1.04f,
                 rw = rough * 0.022f + -0.04f;
-    const float a004 = fminf(rx * rx, pm_exp2(-9.28f * nv)) * rx + ry;
+    const float a004 = fminf(rx * rx, exp2_of(-9.28f * nv)) * rx + ry;
     const float abx = -1.04f * a004 + rz, aby = 1.04f * a004 + rw;
     return f0 * abx + mk(aby);
 }
 
 __device__ __forceinline__ f3 dielectric_f0(float ior) {
-    const float r = (ior - 1.0f) / (ior + 1.0f);
+    const float r = dv(ior - 1.0f, ior + 1.0f);
     return mk(r * r);
 }
 
@@ -780,97 +805,87 @@ __device__ __forceinline__ float under_layer(f3 f0, float rough, float nv) {
 }
 
 __device__ __forceinline__ float under_layer_real(float eta, float rough, float nv) {
-    const float r = (eta - 1.0f) / (eta + 1.0f);
+    const float r = dv(eta - 1.0f, eta + 1.0f);
     const float face_on = r * r;
     const float climb = env_brdf(mk(0.0f), rough, nv).x;
     const float flat = env_brdf(mk(1.0f), rough, nv).x - climb;
-    const float schlick = (1.0f - face_on) * pm_pow(1.0f - nv, 5.0f);
+    const float schlick = (1.0f - face_on) * pow_of(1.0f - nv, 5.0f);
     const float real = fresnel_dielectric_cos(nv, eta) - face_on;
-    const float scale = clampf(real / fmaxf(schlick, 1e-5f), 0.0f, 1.0f);
+    const float scale = clampf(dv(real, fmaxf(schlick, 1e-5f)), 0.0f, 1.0f);
     return clampf(1.0f - (face_on * flat + climb * scale), 0.0f, 1.0f);
 }
 
 // glossy_floor with phiray's own integrator (integrator.x 0): 0.3.
 __device__ __forceinline__ float glossy_floor() { return 0.3f; }
 
-__device__ __forceinline__ float ggx_pdf(const Surf& s, f3 l) {
-    const f3 h = normalize(l + s.v);
-    const float nh = fmaxf(dot(s.n, h), 0.0f);
-    const float a2 = fmaxf(s.rough * s.rough * s.rough * s.rough, 1e-4f);
-    const float dd = nh * nh * (a2 - 1.0f) + 1.0f;
-    const float dist = a2 / (PI * dd * dd);
-    const float nv = fmaxf(dot(s.n, s.v), 1e-4f);
-    const float g1 = 1.0f / (1.0f + ggx_lambda(a2, nv));
-    return g1 * dist / (4.0f * nv);
-}
-
-__device__ __forceinline__ f3 brdf_w(const Surf& s, f3 l, f3 e, float wd, float ws) {
+static __device__ __noinline__ f3 brdf(const Surf& s, f3 l, f3 e) {
     const float raw = dot(s.n, l);
     const float w = s.bleed * 0.75f;
-    const float nl = fmaxf((raw + w) / (1.0f + w), 0.0f) / (1.0f + w * 0.5f);
+    const float nl = dv(fmaxf(dv(raw + w, 1.0f + w), 0.0f), 1.0f + w * 0.5f);
     f3 thru = mk(0.0f);
-    if (s.bleed != 0.0f) thru = s.albedo * s.bleed * s.sss_tint * pm_pow(fmaxf(dot(s.v, -l), 0.0f), 3.0f) * 0.35f;
-    if (nl <= 0.0f) return thru * e * wd;
-    const f3 hv = normalize(l + s.v);
+    if (s.bleed != 0.0f) thru = s.albedo * s.bleed * s.sss_tint * pow_of(fmaxf(dot(s.v, -l), 0.0f), 3.0f) * 0.35f;
+    if (nl <= 0.0f) return thru * e;
+    const f3 hv = unit(l + s.v);
     const float nh = fmaxf(dot(s.n, hv), 0.0f);
     const float hvv = fmaxf(dot(hv, s.v), 0.0f);
     const float a2 = fmaxf(s.rough * s.rough * s.rough * s.rough, 1e-4f);
     const float dd = nh * nh * (a2 - 1.0f) + 1.0f;
-    const float dist = a2 / (PI * dd * dd);
+    const float dist = dv(a2, PI * dd * dd);
     const f3 fres = fresnel_of(s, hvv);
     const float nv = fmaxf(dot(s.n, s.v), 1e-4f);
-    const float g2 = 1.0f / (1.0f + ggx_lambda(a2, nv) + ggx_lambda(a2, fmaxf(raw, 1e-4f)));
-    const f3 spec = fres * dist * g2 * 0.25f / nv;
-    const f3 diffuse = vmix(s.albedo, s.albedo * s.sss_tint, s.bleed) / PI;
-    f3 sum = diffuse * wd + spec * ws;
+    const float g2 = dv(1.0f, 1.0f + ggx_lambda(a2, nv) + ggx_lambda(a2, fmaxf(raw, 1e-4f)));
+    const f3 spec = dv(fres * dist * g2 * 0.25f, nv);
+    const f3 diffuse = dv(vmix(s.albedo, s.albedo * s.sss_tint, s.bleed), PI);
+    f3 sum = diffuse + spec;
     if (s.sheen != 0.0f) sum += s.sheen_tint * s.sheen * charlie(nh, s.sheen_rough);
     if (s.coat != 0.0f) {
         const float ca2 = fmaxf(s.coat_rough * s.coat_rough * s.coat_rough * s.coat_rough, 1e-4f);
         const float cd = nh * nh * (ca2 - 1.0f) + 1.0f;
-        const float coat_f = 0.04f + 0.96f * pm_pow(1.0f - hvv, 5.0f);
-        const float coat = s.coat * coat_f * (ca2 / (PI * cd * cd)) * 0.25f;
+        const float coat_f = 0.04f + 0.96f * pow_of(1.0f - hvv, 5.0f);
+        const float coat = s.coat * coat_f * dv(ca2, PI * cd * cd) * 0.25f;
         const float under = 1.0f - s.coat * coat_f;
         sum = sum * under + mk(coat);
     }
     f3 out = sum * e * nl;
-    if (s.bleed != 0.0f) out += thru * e * wd;
+    if (s.bleed != 0.0f) out += thru * e;
     return out;
 }
 
-__device__ __forceinline__ f3 brdf(const Surf& s, f3 l, f3 e) { return brdf_w(s, l, e, 1.0f, 1.0f); }
-
 // ---- light.wgsl ----
 
-__device__ __forceinline__ f3 onb(f3 n, float a, float b) {
-    const f3 tx = normalize(fabsf(n.z) > 0.9f ? cross(n, mk(1.0f, 0.0f, 0.0f)) : cross(n, mk(0.0f, 0.0f, 1.0f)));
+static __device__ __noinline__ f3 onb(f3 n, float a, float b) {
+    const f3 tx = unit(fabsf(n.z) > 0.9f ? cross(n, mk(1.0f, 0.0f, 0.0f)) : cross(n, mk(0.0f, 0.0f, 1.0f)));
     const f3 ty = cross(n, tx);
     return tx * a + ty * b;
 }
 
 __device__ __forceinline__ f3 cone_dir(f3 axis, float ang, uint32_t& seed) {
     if (ang <= 0.0f) return axis;
-    const float r = ang * sqrtf(rnd(seed));
+    const float r = ang * rt(rnd(seed));
     const float ph = 2.0f * PI * rnd(seed);
-    float s, c;
-    pm_sincos(ph, &s, &c);
-    return normalize(axis + onb(axis, r * c, r * s));
+    const float2 sc = sincos_of(ph);
+    return unit(axis + onb(axis, r * sc.y, r * sc.x));
 }
 
 __device__ __forceinline__ f3 cosine_dir(f3 n, uint32_t& seed) {
     const float r1 = rnd(seed);
-    const float rr = sqrtf(r1);
+    const float rr = rt(r1);
     const float ph = 2.0f * PI * rnd(seed);
-    float s, c;
-    pm_sincos(ph, &s, &c);
-    return normalize(onb(n, rr * c, rr * s) + n * sqrtf(fmaxf(0.0f, 1.0f - r1)));
+    const float2 sc = sincos_of(ph);
+    return unit(onb(n, rr * sc.y, rr * sc.x) + n * rt(fmaxf(0.0f, 1.0f - r1)));
 }
 
-struct Shadowed {
-    f3 c, dir;
-    float dist;
+// A light query before its BRDF: the direction to the light and the distance
+// its shadow ray runs, the light arriving (zero: none), and the factor the
+// reflected light is scaled by. The queries leave the BRDF to their caller,
+// so that its code is there once for all of them.
+struct Query {
+    f3 l, e;
+    float dist, scale;
+    bool met;
 };
 
-__device__ __forceinline__ Shadowed unshadowed() { return Shadowed{mk(0.0f), mk(0.0f, 0.0f, 1.0f), 0.0f}; }
+__device__ __forceinline__ Query no_query() { return Query{mk(0.0f, 0.0f, 1.0f), mk(0.0f), 0.0f, 0.0f, false}; }
 
 __device__ __forceinline__ float spot_mask(const phx_light& li, f3 l) {
     const f3 dir = mk(li.dir[0], li.dir[1], li.dir[2]);
@@ -893,33 +908,33 @@ __device__ __forceinline__ float lamp_reach(const phx_light& li, f3 at, float ao
     if (li.kind == 0u) return lum;
     const f3 to = mk(li.pos[0], li.pos[1], li.pos[2]) - at;
     const float nr = fmaxf(li.size * 0.5f, ao * 0.05f);
-    return lum / ((4.0f * PI) * (dot(to, to) + nr * nr));
+    return dv(lum, (4.0f * PI) * (dot(to, to) + nr * nr));
 }
 
-__device__ __forceinline__ Shadowed area_query(const Surf& s, const phx_light& li, float weight, float r1, float r2,
+__device__ __forceinline__ Query area_query(const Surf& s, const phx_light& li, float weight, float r1, float r2,
                                                float pick) {
     const f3 lpos = mk(li.pos[0], li.pos[1], li.pos[2]), ldir = mk(li.dir[0], li.dir[1], li.dir[2]),
              lright = mk(li.right[0], li.right[1], li.right[2]);
     const float height = dot(s.pos - lpos, ldir);
-    if (height <= 0.0f) return unshadowed();
+    if (height <= 0.0f) return no_query();
     const bool round = li.shape == 4u || li.shape == 5u;
     const float hx = li.size * 0.5f, hy = li.size_y * 0.5f;
     const float area = fmaxf(li.size * li.size_y * (round ? 0.25f * PI : 1.0f), 1e-8f);
     const f3 up = cross(ldir, lright);
     const f3 off = s.pos - lpos;
-    const float near = area / (area + PI * dot(off, off));
+    const float near = dv(area, area + PI * dot(off, off));
     float onx, ony;
-    float sn, cs;
-    pm_sincos(2.0f * PI * r2, &sn, &cs);
+    const float2 sc = sincos_of(2.0f * PI * r2);
+    const float sn = sc.x, cs = sc.y;
     if (pick < near) {
-        const float spread = sqrtf(r1 / fmaxf(1.0f - r1, 1e-6f)) * height;
+        const float spread = rt(dv(r1, fmaxf(1.0f - r1, 1e-6f))) * height;
         onx = cs * spread + dot(off, lright);
         ony = sn * spread + dot(off, up);
-        const float ux = onx / fmaxf(hx, 1e-8f), uy = ony / fmaxf(hy, 1e-8f);
+        const float ux = dv(onx, fmaxf(hx, 1e-8f)), uy = dv(ony, fmaxf(hy, 1e-8f));
         const bool inside = round ? (ux * ux + uy * uy <= 1.0f) : (fmaxf(fabsf(ux), fabsf(uy)) <= 1.0f);
-        if (!inside) return unshadowed();
+        if (!inside) return no_query();
     } else {
-        const float sq = sqrtf(r1);
+        const float sq = rt(r1);
         if (round) {
             onx = cs * sq * hx;
             ony = sn * sq * hy;
@@ -930,51 +945,53 @@ __device__ __forceinline__ Shadowed area_query(const Surf& s, const phx_light& l
     }
     const f3 to = lpos + lright * onx + up * ony - s.pos;
     const float d2 = fmaxf(dot(to, to), 1e-6f);
-    const f3 l = to / sqrtf(d2);
+    const float far = rt(d2);
+    const f3 l = dv(to, far);
     const float facing = fmaxf(dot(-l, ldir), 0.0f);
-    const float pdf = (1.0f - near) / area + near * facing * facing / (PI * d2);
-    const f3 e = mk(li.color[0], li.color[1], li.color[2]) / (PI * area) * facing / d2 / fmaxf(pdf, 1e-12f);
-    if (maxc(e) < 1e-5f) return unshadowed();
-    return Shadowed{brdf(s, l, e) * weight, l, sqrtf(d2) * 0.999f};
+    const float pdf = dv(1.0f - near, area) + dv(near * facing * facing, PI * d2);
+    const f3 e = dv(dv(dv(mk(li.color[0], li.color[1], li.color[2]), PI * area) * facing, d2), fmaxf(pdf, 1e-12f));
+    if (maxc(e) < 1e-5f) return no_query();
+    return Query{l, e, far * 0.999f, weight, true};
 }
 
-__device__ __forceinline__ Shadowed lamp_query(const Frame& F, const Surf& s, uint32_t& seed) {
+__device__ __forceinline__ Query lamp_query(const Frame& F, const Surf& s, uint32_t& seed) {
     float total = 0.0f, held = 0.0f;
     uint32_t idx = 0;
     float u = rnd(seed);
+#pragma unroll 1
     for (uint32_t k = 0; k < F.count; k++) {
         const float w = lamp_reach(F.lights[k], s.pos, F.ao);
         if (w <= 0.0f) continue;
         total += w;
-        const float share = w / total;
-        if (u < share) {
+        const float share = dv(w, total);
+        const bool take = u < share;
+        if (take) {
             idx = k;
             held = w;
-            u = u / share;
-        } else {
-            u = (u - share) / (1.0f - share);
         }
+        u = dv(take ? u : u - share, take ? share : 1.0f - share);
     }
-    if (total <= 0.0f || held <= 0.0f) return unshadowed();
+    if (total <= 0.0f || held <= 0.0f) return no_query();
     const phx_light& li = F.lights[idx];
-    const float weight = total / held;
+    const float weight = dv(total, held);
     const f3 color = mk(li.color[0], li.color[1], li.color[2]);
     if (li.kind == 0u) {
         const f3 l = cone_dir(-mk(li.dir[0], li.dir[1], li.dir[2]), li.size * 0.5f, seed);
-        return Shadowed{brdf(s, l, color) * weight, l, INF};
+        return Query{l, color, INF, weight, true};
     }
     const float r1 = rnd(seed);
     const float r2 = rnd(seed);
     if (li.kind == 3u) return area_query(s, li, weight, r1, r2, rnd(seed));
     const f3 lpos = mk(li.pos[0], li.pos[1], li.pos[2]);
-    const f3 aim = lpos + onb(normalize(s.pos - lpos), (r1 - 0.5f) * li.size, (r2 - 0.5f) * li.size);
+    const f3 aim = lpos + onb(unit(s.pos - lpos), (r1 - 0.5f) * li.size, (r2 - 0.5f) * li.size);
     const f3 to = aim - s.pos;
     const float d2 = fmaxf(dot(to, to), 1e-6f);
-    const f3 l = to / sqrtf(d2);
-    f3 e = color / ((4.0f * PI) * d2);
+    const float far = rt(d2);
+    const f3 l = dv(to, far);
+    f3 e = dv(color, (4.0f * PI) * d2);
     if (li.kind == 2u) e *= spot_mask(li, l);
-    if (maxc(e) < 1e-5f) return unshadowed();
-    return Shadowed{brdf(s, l, e) * weight, l, sqrtf(d2) * 0.999f};
+    if (maxc(e) < 1e-5f) return no_query();
+    return Query{l, e, far * 0.999f, weight, true};
 }
 
 // lamp_chance (light.wgsl:259-271): the table share of the hit's (face,
@@ -985,6 +1002,7 @@ __device__ __forceinline__ float lamp_chance(const Scene& S, uint32_t slot, uint
     if (count == 0u) return 0.0f;
     const bool placed = (M & MODE_FULL) && S.lamp_inst;
     uint32_t lo = 0, hi = count - 1u;
+#pragma unroll 1
     while (lo < hi) {
         const uint32_t mid = (lo + hi) / 2u;
         const uint32_t f = __ldg(S.lamp_slot + mid);
@@ -998,11 +1016,12 @@ __device__ __forceinline__ float lamp_chance(const Scene& S, uint32_t slot, uint
 }
 
 template <int M>
-__device__ __forceinline__ Shadowed glow_query(const Scene& S, const Surf& s, uint32_t& seed) {
+__device__ __forceinline__ Query glow_query(const Scene& S, const Surf& s, uint32_t& seed) {
     const uint32_t count = S.lamp_count;
-    if (count == 0u) return unshadowed();
+    if (count == 0u) return no_query();
     const float u = rnd(seed);
     uint32_t lo = 0, hi = count - 1u;
+#pragma unroll 1
     while (lo < hi) {
         const uint32_t mid = (lo + hi) / 2u;
         if (__ldg(S.lamp_cdf + mid) < u) lo = mid + 1u;
@@ -1024,13 +1043,14 @@ __device__ __forceinline__ Shadowed glow_query(const Scene& S, const Surf& s, ui
     const float area = 0.5f * length(cr);
     const f3 to = q - s.pos;
     const float d2 = fmaxf(dot(to, to), 1e-6f);
-    const f3 l = to / sqrtf(d2);
-    const float cos_l = fabsf(dot(normalize(cr), l));
-    const f3 e = t.emit * cos_l * area / (chance * d2);
-    const float pl = chance * d2 / fmaxf(area * cos_l, 1e-8f);
-    const float pb = fmaxf(dot(s.n, l), 0.0f) / PI;
-    const float w = pl * pl / fmaxf(pl * pl + pb * pb, 1e-12f);
-    return Shadowed{brdf(s, l, e) * w, l, sqrtf(d2) * 0.999f};
+    const float far = rt(d2);
+    const f3 l = dv(to, far);
+    const float cos_l = fabsf(dot(unit(cr), l));
+    const f3 e = dv(t.emit * cos_l * area, chance * d2);
+    const float pl = dv(chance * d2, fmaxf(area * cos_l, 1e-8f));
+    const float pb = dv(fmaxf(dot(s.n, l), 0.0f), PI);
+    const float w = dv(pl * pl, fmaxf(pl * pl + pb * pb, 1e-12f));
+    return Query{l, e, far * 0.999f, w, true};
 }
 
 __device__ __forceinline__ float hit_lift(const Frame& F, float t) {
@@ -1046,13 +1066,30 @@ __device__ __forceinline__ float through_lift(const Frame& F, f3 pos, float t) {
 
 __device__ __forceinline__ bool uses_rig(const Frame& F) { return F.count == 0u && !(dot(F.env, F.env) > 0.0f); }
 
-__device__ __forceinline__ Shadowed rig_query(const Frame& F, uint32_t k, const Surf& s, uint32_t& seed, f3 sun) {
+__device__ __forceinline__ Query rig_query(const Frame& F, uint32_t k, const Surf& s, uint32_t& seed, f3 sun) {
     if (k == 0u) {
         const f3 key = cone_dir(sun, 0.06f, seed);
-        return Shadowed{brdf(s, key, mk(2.0f)), key, INF};
+        return Query{key, mk(2.0f), INF, 1.0f, true};
     }
-    const f3 rim = normalize(F.up * 0.6f - F.back * 0.8f + F.right * 0.2f);
-    return Shadowed{brdf(s, rim, mk(0.9f)), rim, INF};
+    const f3 rim = unit(F.up * 0.6f - F.back * 0.8f + F.right * 0.2f);
+    return Query{rim, mk(0.9f), INF, 1.0f, true};
+}
+
+__device__ __forceinline__ f3 rig_fill(const Frame& F, const Surf& s) {
+    const f3 fill = unit(-F.right * 0.8f + F.up * 0.2f + F.back * 0.6f);
+    return brdf(s, fill, mk(0.45f));
+}
+
+// direct()'s light query k (integrate.wgsl:66-85): 0 a lamp or the rig's key,
+// 1 the rig's rim, 2 an emitter. The fourth, env_query, needs an environment
+// image's table (env_cdf), which the host refuses; it returns no light
+// without a draw.
+template <int M>
+__device__ __forceinline__ Query light_query(const Scene& S, const Frame& F, uint32_t k, const Surf& s, uint32_t& seed,
+                                             f3 sun) {
+    if (k == 2u) return glow_query<M>(S, s, seed);
+    if (uses_rig(F)) return rig_query(F, k, s, seed, sun);
+    return k == 0u ? lamp_query(F, s, seed) : no_query();
 }
 
 // ---- util.wgsl:185-272: the floor grid as an overlay, premultiplied ----
@@ -1076,7 +1113,7 @@ __device__ __forceinline__ Over floor_over(const Frame& F, f3 o, f3 d, float t_h
     const float lg = pm_log2(fmaxf(want, 1e-9f)) / pm_log2(10.0f);
     const float lvl = floorf(lg);
     const float f = lg - lvl;
-    const float g0 = pm_pow(10.0f, lvl);
+    const float g0 = pow_of(10.0f, lvl);
     const float g1 = g0 * 10.0f;
     const float half_w = foot * 0.5f;
     const float aa = foot;
@@ -1132,11 +1169,6 @@ static __device__ __noinline__ Over grid_over(const Frame& F, f3 o, f3 d, float 
         g = Over{g.c * (1.0f - z.a) + z.c, g.a * (1.0f - z.a) + z.a};
     }
     return g;
-}
-
-__device__ __forceinline__ f3 rig_fill(const Frame& F, const Surf& s) {
-    const f3 fill = normalize(-F.right * 0.8f + F.up * 0.2f + F.back * 0.6f);
-    return brdf(s, fill, mk(0.45f));
 }
 
 }  // namespace shade

@@ -30,8 +30,9 @@ namespace {
 // arrays before any kernel indexes through them: out[0] the first face that
 // names a vertex or material out of range, out[1] the first material with a
 // texture or map (Mat words 12-16 not NO_TEX), out[2] the first with a
-// second lobe (word 30 not NO_MAT), all 0xFFFFFFFF when none; out[3] != 0
-// when some material emits (luminance of words 8-10 above zero).
+// second lobe (word 30 not NO_MAT), all 0xFFFFFFFF when none; out[3]
+// bit 0 when some material emits (luminance of words 8-10 above zero), bit 1
+// when some material transmits light (trans (1 - metal) not zero).
 __global__ void __launch_bounds__(256) k_check_scene(const uint4* __restrict__ faces, uint32_t nfaces, uint32_t nverts,
                                                      const float* __restrict__ mats, uint32_t nmats,
                                                      uint32_t* __restrict__ out) {
@@ -48,6 +49,7 @@ __global__ void __launch_bounds__(256) k_check_scene(const uint4* __restrict__ f
         if (tex) atomicMin(out + 1, i);
         if (__ldg(w + 30) != 0xFFFFFFFFu) atomicMin(out + 2, i);
         if (0.2126f * __ldg(m + 8) + 0.7152f * __ldg(m + 9) + 0.0722f * __ldg(m + 10) > 0.0f) atomicOr(out + 3, 1u);
+        if (!(__ldg(m + 6) * (1.0f - __ldg(m + 5)) == 0.0f)) atomicOr(out + 3, 2u);
     }
 }
 
@@ -689,6 +691,9 @@ struct Forest {
     DevMem rec, flags, mesh_of, placed_dev, mesh_rec, slots, order_all, lamp_inst, slot_mesh, mesh_off, mesh_list;
 };
 
+// A tracer whose render kernel was neither set nor autotuned (launch_frame).
+constexpr uint32_t KERNEL_UNSET = 0xFFFFFFFFu;
+
 struct phx_tracer_s {
     Ctx* ctx = nullptr;
     uint32_t nverts = 0, nfaces = 0, nmats = 0, leaf = 4;
@@ -703,12 +708,13 @@ struct phx_tracer_s {
     uint32_t* wf_host_lens = nullptr;  // pinned: the queue lengths the host polls
     bool has_normals = false;
     bool emissive = false;  // some material emits: the emitter table is built
+    bool transmits = false;  // some material transmits light (glass)
     DevMem verts, vnorm, faces, mats, tnodes, tris, tnorm, lamp_slot, lamp_power, lamp_cdf, info, px, rays, cam;
     BvhWork bvh;
     uint32_t w = 0, h = 0;
     uint32_t frame = 0, target = 32;  // Tracer::SAMPLE_COUNT (src/trace/mod.rs:129) until set_samples
-    uint32_t kernel = PHX_KERNEL_MEGAKERNEL;  // which render kernel traces a frame (the fastest measured)
-    DevMem next;                                 // the state-machine kernel's pixel counter
+    uint32_t kernel = KERNEL_UNSET;  // which render kernel traces a frame (set or autotuned)
+    DevMem next;                                 // the pooled and state-machine kernels' work counter
     uint32_t stack_place = PHX_STACK_LOCAL;      // where thread-per-ray walks keep their stack
     uint32_t walk = PHX_WALK_THREAD;             // ray walks: a thread per ray, persistent warps, sorted first
     DevMem rkeys, rsorted, rorder, ralt_k, ralt_v, rzero;  // the sorted walk's keys and radix-sort scratch
@@ -1106,6 +1112,26 @@ int32_t wf_buffers(phx_tracer tr, uint32_t count, WfBuffers& B) {
     return PHX_OK;
 }
 
+// The pooled render's buffers for `count` pixels and `spp` samples, out of
+// `scratch`: 8,192 path slots an SM (240 bytes each), and the terms of as
+// many samples as POOL_OUT_BYTES hold (one at least; the rest of the samples
+// run in further launches).
+constexpr size_t POOL_OUT_BYTES = (size_t)1 << 30;
+constexpr uint64_t POOL_SM_SLOTS = 8192;
+
+int32_t pool_buffers(Ctx* c, PoolScratch& scratch, uint32_t count, uint32_t spp, PoolBuffers& B) {
+    const size_t sample = (size_t)count * pool_out_words() * 4;
+    const uint32_t fit = (uint32_t)std::max<size_t>(POOL_OUT_BYTES / sample, 1);
+    const uint32_t launches = (spp + fit - 1) / fit;
+    B.slots = (uint64_t)c->sms * POOL_SM_SLOTS;
+    B.spp = (spp + launches - 1) / launches;
+    PHX_TRY(scratch.state.reserve(B.slots * pool_slot_bytes()));
+    PHX_TRY(scratch.out.reserve(sample * B.spp));
+    B.pools = (uint32_t*)scratch.state.ptr;
+    B.out = (uint32_t*)scratch.out.ptr;
+    return PHX_OK;
+}
+
 // Launches the tracer's render kernel over pixels [first_px, first_px +
 // count_px) of frame F, whose camera is already in tr->cam (no host copy:
 // the launch can be recorded into a graph).
@@ -1134,18 +1160,24 @@ int32_t ensure_wide(phx_tracer tr) {
     return read_status(c);
 }
 
-int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, uint32_t count_px, bool stats) {
+int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, uint32_t count_px, bool stats,
+                     PoolScratch* scratch = nullptr) {
     Ctx* c = tr->ctx;
+    const bool full = tr->forest || F.grid > 0.0f;
+    // The default: the pooled render where it can run (below), which on a
+    // 65,536-face cloud at 256 x 256, 16 spp took 4.9 ms against the 4-block
+    // megakernel's 27 ms, on the 1.3 M-face mesh at 1080p, 16 spp, 28 ms
+    // against 57, and on 64 x 48 pixels 0.6 against 0.8; else that megakernel.
     uint32_t kernel = tr->kernel;
+    if (kernel == KERNEL_UNSET) kernel = full ? PHX_KERNEL_MEGAKERNEL : PHX_KERNEL_STATE_MACHINE;
     const Scene S = scene_of(tr);
-    // Adaptive Sampling runs on the megakernel forms (the state machine
-    // fetches pixels by index, not from the open list); they all compute
-    // the same image, so an adaptive frame takes the default form instead.
+    // Adaptive Sampling runs on the megakernel forms (the others take pixels
+    // by index, not from the open list); they all compute the same image, so
+    // an adaptive frame takes the 4-block form instead.
     if (F.adapt_on && kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8)
         kernel = PHX_KERNEL_MEGAKERNEL;
     const RenderLaunch L{S,        F,       sun,    (uint32_t*)tr->px.ptr, first_px, count_px,
                          (unsigned long long*)tr->rays.ptr, (uint32_t*)tr->next.ptr, c->sms, c->stream};
-    const bool full = tr->forest || F.grid > 0.0f;
     if (kernel == PHX_KERNEL_WAVEFRONT) {
         // the host polls its queues between passes: not while a graph is recorded
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1159,7 +1191,24 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
         }
     }
     if (full) return render_full(kernel, stats, L);
-    if (kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8) return render_flat_sm(kernel, stats, L);
+    if (kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8) {
+        // The pooled render shades a path's one opaque camera hit, so it takes
+        // scenes whose materials transmit no light. Its buffers are the
+        // context's, which a recorded graph must not hold (they may grow
+        // before it is replayed), or the caller's `scratch`. Otherwise, and
+        // where there is no memory for them, the 4-block megakernel.
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        PHX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+        if (!tr->transmits && count_px && (scratch || cap == cudaStreamCaptureStatusNone)) {
+            std::unique_lock<std::mutex> lock(c->path_pool_lock, std::defer_lock);
+            if (!scratch) lock.lock();
+            PoolBuffers B;
+            const int32_t rc = pool_buffers(c, scratch ? *scratch : c->path_pool, count_px, F.spp, B);
+            if (rc >= 0) return render_pooled(kernel, stats, L, B);
+            if (rc != PHX_ERR_OOM && cap == cudaStreamCaptureStatusNone) return rc;
+        }
+        kernel = PHX_KERNEL_MEGAKERNEL;
+    }
     if (kernel >= PHX_KERNEL_MEGAKERNEL_6 && kernel <= PHX_KERNEL_MEGAKERNEL_8_SYNC) return render_flat_b(kernel, stats, L);
     if (kernel >= PHX_KERNEL_MEGAKERNEL_10_SYNC && kernel <= PHX_KERNEL_MEGAKERNEL_16_SYNC)
         return render_flat_c(kernel, stats, L);
@@ -1320,7 +1369,8 @@ int32_t create_tracer(phx_ctx ctx, const phx_scene* sc, const phx_mesh* meshes, 
             rc = fail(PHX_ERR_INVALID, "material %u uses a texture (not supported)", found[1]);
         if (rc == PHX_OK && found[2] != 0xFFFFFFFFu)
             rc = fail(PHX_ERR_INVALID, "material %u has a second lobe (not supported)", found[2]);
-        tr->emissive = found[3] != 0;
+        tr->emissive = (found[3] & 1u) != 0;
+        tr->transmits = (found[3] & 2u) != 0;
     }
     if (meshes && rc == PHX_OK) {
         tr->forest.reset(new Forest());
@@ -1995,6 +2045,7 @@ struct phx_batch_s {
     std::vector<uint32_t> order;  // jobs by decreasing per-tile cost
     uint32_t kind = PHX_BATCH_PERSISTENT, threads = 128, stack = PHX_STACK_LOCAL;
     DevMem djobs, next, counters, stamps, modes;
+    PoolScratch path_pool;        // the per-scene pooled launches' buffers (the captured graph holds them)
     uint32_t* host_modes = nullptr;  // pinned: the graph's per-replay copy source
     uint32_t ntiles = 0;
     cudaGraphExec_t exec = nullptr;
@@ -2064,7 +2115,8 @@ int32_t batch_trace(phx_batch b) {
             BatchJob& bj = b->jobs[j];
             const Frame F = frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp);
             PHX_CUDA(cudaMemsetAsync(bj.tr->rays.ptr, 0, 8, c->stream));
-            PHX_TRY(launch_frame(bj.tr, F, mk(bj.cam.sun[0], bj.cam.sun[1], bj.cam.sun[2]), 0, bj.w * bj.h, false));
+            PHX_TRY(launch_frame(bj.tr, F, mk(bj.cam.sun[0], bj.cam.sun[1], bj.cam.sun[2]), 0, bj.w * bj.h, false,
+                                 &b->path_pool));
             PHX_CUDA(cudaMemcpyAsync((unsigned long long*)b->counters.ptr + 3 * j, bj.tr->rays.ptr, 8,
                                      cudaMemcpyDeviceToDevice, c->stream));
         }

@@ -240,7 +240,8 @@ class Tracer:
         return chosen.value, list(ms)
 
     def set_kernel(self, kind: int) -> None:
-        """Render kernel: Tracer.MEGAKERNEL or Tracer.STATE_MACHINE (same image)."""
+        """Render kernel, one of the ids above (same image). Unset, the pooled
+        render (STATE_MACHINE) where it can run, else MEGAKERNEL."""
         N.check(N.lib().phx_tracer_set_kernel(self.handle, kind))
 
     STACK_LOCAL = 0
