@@ -202,63 +202,79 @@ __global__ void k_root(const float4* __restrict__ nodes, uint32_t n, float4* inf
     info[1] = make_float4(b.x, b.y, b.z, ext);
 }
 
+// The power of slot s (lamp.rs: world area x emitted luminance), 0 for one
+// that emits nothing.
+__device__ __forceinline__ float lamp_glow(const float4* __restrict__ tris, const float4* __restrict__ mats, uint32_t s) {
+    const float4 B = __ldg(tris + 3 * (size_t)s + 1);
+    const float4 e = __ldg(mats + 8 * (size_t)__float_as_uint(B.w) + 2);
+    const float lum = 0.2126f * e.x + 0.7152f * e.y + 0.0722f * e.z;
+    if (!(lum > 0.0f)) return 0.0f;
+    const float4 A = __ldg(tris + 3 * (size_t)s), Cc = __ldg(tris + 3 * (size_t)s + 2);
+    const float e1x = B.x - A.x, e1y = B.y - A.y, e1z = B.z - A.z;
+    const float e2x = Cc.x - A.x, e2y = Cc.y - A.y, e2z = Cc.z - A.z;
+    const float cx = e1y * e2z - e1z * e2y, cy = e1z * e2x - e1x * e2z, cz = e1x * e2y - e1y * e2x;
+    float sq = 0.0f;
+    sq = sq + cx * cx;
+    sq = sq + cy * cy;
+    sq = sq + cz * cz;
+    return 0.5f * sqrtf(sq) * lum;
+}
+
+// Emissive slots of each run of 1,024, a block a run.
+__global__ void __launch_bounds__(1024) k_lamp_count(const float4* __restrict__ tris, const float4* __restrict__ mats,
+                                                     uint32_t n, uint32_t* __restrict__ counts) {
+    const uint32_t s = blockIdx.x * 1024u + threadIdx.x;
+    const uint32_t c = __syncthreads_count(s < n && lamp_glow(tris, mats, s) > 0.0f);
+    if (threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+
+// Rank of `on` among the block's threads in thread order, and the number of
+// them (1,024 threads).
+__device__ __forceinline__ uint32_t block_rank(bool on, uint32_t* s_warp, uint32_t& total) {
+    const uint32_t m = __ballot_sync(0xffffffffu, on), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0) s_warp[warp] = __popc(m);
+    __syncthreads();
+    const uint32_t c = s_warp[lane];
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? c : 0u);
+    total = __reduce_add_sync(0xffffffffu, c);
+    __syncthreads();
+    return before + __popc(m & ((1u << lane) - 1u));
+}
+
 // The emitter table (lamp.rs table_of, one instance): emissive slots in slot
-// order with their power (world area x emitted luminance) and its running
-// share. One block: counts per thread chunk, a block scan for positions,
-// then one thread sums in slot order so the CDF rounds as the CPU's does.
+// order with their power and its running share. One block, over the runs that
+// hold an emitter (k_lamp_count's counts, which sit where the CDF will);
+// then one thread sums in slot order so the CDF rounds as the CPU's does. A
+// scene's emitters are a few faces, and one block reading every slot took
+// 142 us for 65,540 faces (657 us for 120,000) where the two take 11.
 __global__ void __launch_bounds__(1024) k_lamps(const float4* __restrict__ tris, const float4* __restrict__ mats,
                                                 uint32_t n, uint32_t* __restrict__ slots, float* __restrict__ power,
-                                                float* __restrict__ cdf, float4* info) {
-    __shared__ uint32_t s_count[1024];
-    const uint32_t T = blockDim.x, t = threadIdx.x;
-    const uint32_t chunk = (n + T - 1) / T;
-    const uint32_t lo = t * chunk, hi = lo + chunk < n ? lo + chunk : n;
-    auto glow = [&](uint32_t s, float& p) -> bool {
-        const float4 A = __ldg(tris + 3 * (size_t)s), B = __ldg(tris + 3 * (size_t)s + 1),
-                     Cc = __ldg(tris + 3 * (size_t)s + 2);
-        const uint32_t m = __float_as_uint(B.w);
-        const float4 e = __ldg(mats + 8 * (size_t)m + 2);
-        const float lum = 0.2126f * e.x + 0.7152f * e.y + 0.0722f * e.z;
-        if (!(lum > 0.0f)) return false;
-        const float e1x = B.x - A.x, e1y = B.y - A.y, e1z = B.z - A.z;
-        const float e2x = Cc.x - A.x, e2y = Cc.y - A.y, e2z = Cc.z - A.z;
-        const float cx = e1y * e2z - e1z * e2y, cy = e1z * e2x - e1x * e2z, cz = e1x * e2y - e1y * e2x;
-        float sq = 0.0f;
-        sq = sq + cx * cx;
-        sq = sq + cy * cy;
-        sq = sq + cz * cz;
-        p = 0.5f * sqrtf(sq) * lum;
-        return p > 0.0f;
-    };
-    uint32_t c = 0;
-    for (uint32_t s = lo; s < hi; s++) {
-        float p;
-        if (glow(s, p)) c++;
-    }
-    s_count[t] = c;
-    __syncthreads();
-    if (t == 0) {
-        uint32_t run = 0;
-        for (uint32_t k = 0; k < T; k++) {
-            const uint32_t v = s_count[k];
-            s_count[k] = run;
-            run += v;
+                                                float* cdf, float4* info) {
+    __shared__ uint32_t s_warp[32], s_run[1024];
+    const uint32_t runs = (n + 1023u) / 1024u, t = threadIdx.x;
+    const uint32_t* counts = (const uint32_t*)cdf;
+    uint32_t count = 0;
+    for (uint32_t r0 = 0; r0 < runs; r0 += 1024u) {
+        uint32_t held = 0;
+        const bool holds = r0 + t < runs && counts[r0 + t] != 0u;
+        const uint32_t at = block_rank(holds, s_warp, held);
+        if (holds) s_run[at] = r0 + t;
+        __syncthreads();
+        for (uint32_t k = 0; k < held; k++) {
+            const uint32_t s = s_run[k] * 1024u + t;
+            const float p = s < n ? lamp_glow(tris, mats, s) : 0.0f;
+            uint32_t found = 0;
+            const uint32_t rank = block_rank(p > 0.0f, s_warp, found);
+            if (p > 0.0f) {
+                slots[count + rank] = s;
+                power[count + rank] = p;
+            }
+            count += found;
         }
-        info[2] = make_float4(__uint_as_float(run), 0.0f, 0.0f, 0.0f);
+        __syncthreads();
     }
-    __syncthreads();
-    uint32_t at = s_count[t];
-    for (uint32_t s = lo; s < hi; s++) {
-        float p;
-        if (glow(s, p)) {
-            slots[at] = s;
-            power[at] = p;
-            at++;
-        }
-    }
-    __syncthreads();
     if (t == 0) {
-        const uint32_t count = __float_as_uint(info[2].x);
+        info[2] = make_float4(__uint_as_float(count), 0.0f, 0.0f, 0.0f);
         float total = 0.0f;
         for (uint32_t k = 0; k < count; k++) total += power[k];
         float run = 0.0f;
@@ -735,6 +751,14 @@ namespace {
 
 int32_t prepare_nodes(phx_tracer tr);
 
+// The emitter table of a single-instance scene.
+void enqueue_lamps(phx_tracer tr, uint32_t n) {
+    const float4 *tris = (const float4*)tr->tris.ptr, *mats = (const float4*)tr->mats.ptr;
+    k_lamp_count<<<ceil_div(n, 1024), 1024, 0, tr->ctx->stream>>>(tris, mats, n, (uint32_t*)tr->lamp_cdf.ptr);
+    k_lamps<<<1, 1024, 0, tr->ctx->stream>>>(tris, mats, n, (uint32_t*)tr->lamp_slot.ptr, (float*)tr->lamp_power.ptr,
+                                             (float*)tr->lamp_cdf.ptr, (float4*)tr->info.ptr);
+}
+
 int32_t prepare(phx_tracer tr) {
     // After a build or refit: face boxes are in tr->bvh; gather, mark leaf
     // ends, then the walk's nodes, root info and emitter table.
@@ -783,9 +807,7 @@ int32_t prepare_nodes(phx_tracer tr) {
                                                       0u, 0u);
     k_root<<<1, 1, 0, s>>>((const float4*)w.nodes.ptr, n, (float4*)tr->info.ptr, 0u);
     if (tr->emissive)
-        k_lamps<<<1, 1024, 0, s>>>((const float4*)tr->tris.ptr, (const float4*)tr->mats.ptr, n,
-                                   (uint32_t*)tr->lamp_slot.ptr, (float*)tr->lamp_power.ptr, (float*)tr->lamp_cdf.ptr,
-                                   (float4*)tr->info.ptr);
+        enqueue_lamps(tr, n);
     else  // no material emits: an empty table (the count word of info[2])
         PHX_CUDA(cudaMemsetAsync((float4*)tr->info.ptr + 2, 0, sizeof(float4), s));
     return cuda_check(cudaGetLastError(), "tracer prepare");
@@ -970,9 +992,7 @@ int32_t prepare_sah(phx_tracer tr) {
     k_convert<<<ceil_div(m, 256), 256, 0, s>>>((const float4*)w.nodes.ptr, m, (float4*)tr->tnodes.ptr, 0u, 0u, 0u);
     k_root<<<1, 1, 0, s>>>((const float4*)w.nodes.ptr, n, (float4*)tr->info.ptr, 0u);
     if (tr->emissive)
-        k_lamps<<<1, 1024, 0, s>>>((const float4*)tr->tris.ptr, (const float4*)tr->mats.ptr, n,
-                                   (uint32_t*)tr->lamp_slot.ptr, (float*)tr->lamp_power.ptr, (float*)tr->lamp_cdf.ptr,
-                                   (float4*)tr->info.ptr);
+        enqueue_lamps(tr, n);
     else
         PHX_CUDA(cudaMemsetAsync((float4*)tr->info.ptr + 2, 0, sizeof(float4), s));
     return cuda_check(cudaGetLastError(), "SAH prepare");
@@ -1161,8 +1181,9 @@ int32_t ensure_wide(phx_tracer tr) {
 }
 
 int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, uint32_t count_px, bool stats,
-                     PoolScratch* scratch = nullptr) {
+                     PoolScratch* scratch = nullptr, cudaStream_t stream = nullptr) {
     Ctx* c = tr->ctx;
+    if (!stream) stream = c->stream;
     const bool full = tr->forest || F.grid > 0.0f;
     // The default: the pooled render where it can run (below), which on a
     // 65,536-face cloud at 256 x 256, 16 spp took 4.9 ms against the 4-block
@@ -1177,11 +1198,11 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
     if (F.adapt_on && kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8)
         kernel = PHX_KERNEL_MEGAKERNEL;
     const RenderLaunch L{S,        F,       sun,    (uint32_t*)tr->px.ptr, first_px, count_px,
-                         (unsigned long long*)tr->rays.ptr, (uint32_t*)tr->next.ptr, c->sms, c->stream};
+                         (unsigned long long*)tr->rays.ptr, (uint32_t*)tr->next.ptr, c->sms, stream};
     if (kernel == PHX_KERNEL_WAVEFRONT) {
         // the host polls its queues between passes: not while a graph is recorded
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        PHX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+        PHX_CUDA(cudaStreamIsCapturing(stream, &cap));
         if (cap != cudaStreamCaptureStatusNone || F.adapt_on) {
             kernel = PHX_KERNEL_MEGAKERNEL;
         } else {
@@ -1198,7 +1219,7 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
         // before it is replayed), or the caller's `scratch`. Otherwise, and
         // where there is no memory for them, the 4-block megakernel.
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        PHX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+        PHX_CUDA(cudaStreamIsCapturing(stream, &cap));
         if (!tr->transmits && count_px && (scratch || cap == cudaStreamCaptureStatusNone)) {
             std::unique_lock<std::mutex> lock(c->path_pool_lock, std::defer_lock);
             if (!scratch) lock.lock();
@@ -2045,7 +2066,16 @@ struct phx_batch_s {
     std::vector<uint32_t> order;  // jobs by decreasing per-tile cost
     uint32_t kind = PHX_BATCH_PERSISTENT, threads = 128, stack = PHX_STACK_LOCAL;
     DevMem djobs, next, counters, stamps, modes;
-    PoolScratch path_pool;        // the per-scene pooled launches' buffers (the captured graph holds them)
+    // The per-scene launches run on a few side streams, so that one scene's
+    // last paths end beside the next scene's first. The captured graph holds
+    // their buffers.
+    static constexpr int LANES = 3;
+    struct Lane {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t done = nullptr;
+        PoolScratch path_pool;
+    } lanes[LANES];
+    cudaEvent_t fork = nullptr;
     uint32_t* host_modes = nullptr;  // pinned: the graph's per-replay copy source
     uint32_t ntiles = 0;
     cudaGraphExec_t exec = nullptr;
@@ -2106,22 +2136,68 @@ int32_t batch_prepare(phx_batch b) {
     return wait_stream(c->stream, BATCH_WAIT_MS);  // the pageable sources are released on return
 }
 
+// One launch a scene, the largest first, each on the side stream with the
+// least work so far. The serving frame of six 256^2-512^2 scenes traced in
+// 26.1 ms on one stream, 22.5 on three.
+int32_t trace_per_scene(phx_batch b) {
+    Ctx* c = b->ctx;
+    const size_t nj = b->jobs.size();
+    auto work = [&](size_t j) { return (uint64_t)b->jobs[j].w * b->jobs[j].h * b->jobs[j].spp; };
+    std::vector<uint32_t> order(nj), lane_of(nj);
+    for (size_t j = 0; j < nj; j++) order[j] = (uint32_t)j;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return work(x) > work(y); });
+    uint64_t load[phx_batch_s::LANES] = {};
+    for (uint32_t j : order) {
+        uint32_t l = 0;
+        for (uint32_t k = 1; k < phx_batch_s::LANES; k++)
+            if (load[k] < load[l]) l = k;
+        lane_of[j] = l;
+        load[l] += work(j);
+    }
+    if (!b->fork) {
+        PHX_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+        for (auto& lane : b->lanes) {
+            PHX_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
+            PHX_CUDA(cudaEventCreateWithFlags(&lane.done, cudaEventDisableTiming));
+        }
+    }
+    // The buffers are sized on the context's stream before the side streams
+    // start (where there is no memory for them launch_frame does without).
+    for (size_t j = 0; j < nj; j++) {
+        const BatchJob& bj = b->jobs[j];
+        PoolBuffers B;
+        if (!bj.tr->forest && !bj.tr->transmits)
+            (void)pool_buffers(c, b->lanes[lane_of[j]].path_pool, bj.w * bj.h, bj.spp, B);
+    }
+    PHX_CUDA(cudaEventRecord(b->fork, c->stream));
+    for (auto& lane : b->lanes) PHX_CUDA(cudaStreamWaitEvent(lane.stream, b->fork, 0));
+    int32_t rc = PHX_OK;
+    for (uint32_t j : order) {
+        BatchJob& bj = b->jobs[j];
+        auto& lane = b->lanes[lane_of[j]];
+        const Frame F = frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp);
+        rc = cuda_check(cudaMemsetAsync(bj.tr->rays.ptr, 0, 8, lane.stream), "rays");
+        if (rc >= 0)
+            rc = launch_frame(bj.tr, F, mk(bj.cam.sun[0], bj.cam.sun[1], bj.cam.sun[2]), 0, bj.w * bj.h, false,
+                              &lane.path_pool, lane.stream);
+        if (rc >= 0)
+            rc = cuda_check(cudaMemcpyAsync((unsigned long long*)b->counters.ptr + 3 * j, bj.tr->rays.ptr, 8,
+                                            cudaMemcpyDeviceToDevice, lane.stream), "rays");
+        if (rc < 0) break;
+    }
+    // joined whatever happened: later work and frees follow all of it
+    for (auto& lane : b->lanes) {
+        PHX_CUDA(cudaEventRecord(lane.done, lane.stream));
+        PHX_CUDA(cudaStreamWaitEvent(c->stream, lane.done, 0));
+    }
+    return rc;
+}
+
 // The frame's traces, stream-ordered (capturable once batch_prepare ran).
 int32_t batch_trace(phx_batch b) {
     Ctx* c = b->ctx;
     PHX_CUDA(cudaMemsetAsync(b->counters.ptr, 0, b->jobs.size() * 3 * sizeof(unsigned long long), c->stream));
-    if (b->kind == PHX_BATCH_PER_SCENE) {
-        for (size_t j = 0; j < b->jobs.size(); j++) {
-            BatchJob& bj = b->jobs[j];
-            const Frame F = frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp);
-            PHX_CUDA(cudaMemsetAsync(bj.tr->rays.ptr, 0, 8, c->stream));
-            PHX_TRY(launch_frame(bj.tr, F, mk(bj.cam.sun[0], bj.cam.sun[1], bj.cam.sun[2]), 0, bj.w * bj.h, false,
-                                 &b->path_pool));
-            PHX_CUDA(cudaMemcpyAsync((unsigned long long*)b->counters.ptr + 3 * j, bj.tr->rays.ptr, 8,
-                                     cudaMemcpyDeviceToDevice, c->stream));
-        }
-        return PHX_OK;
-    }
+    if (b->kind == PHX_BATCH_PER_SCENE) return trace_per_scene(b);
     switch (b->threads) {
         case 64: return launch_batch<64>(b);
         case 128: return launch_batch<128>(b);
@@ -2195,6 +2271,11 @@ int32_t phx_batch_destroy(phx_batch b) {
     phx_batch_clear(b);
     if (b->host_modes) cudaFreeHost(b->host_modes);
     if (b->done) cudaEventDestroy(b->done);
+    if (b->fork) cudaEventDestroy(b->fork);
+    for (auto& lane : b->lanes) {
+        if (lane.done) cudaEventDestroy(lane.done);
+        if (lane.stream) cudaStreamDestroy(lane.stream);
+    }
     b->ctx->live--;
     delete b;
     return PHX_OK;

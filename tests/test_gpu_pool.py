@@ -7,7 +7,8 @@ import pytest
 
 import phiray_b200 as px
 from phiray_b200 import scenes
-from tests.test_gpu_trace import cam_of
+from tests import oracle_lib
+from tests.test_gpu_trace import cam_of, check_image
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +72,17 @@ def test_pooled_render_of_rows_and_a_tree_that_is_one_leaf(gpu):
         images.append(tr.image())
         tr.close()
     assert np.array_equal(images[0], images[1])
+
+
+# no emitter in a run of slots, one, runs full of them; a rest of a run
+@pytest.mark.parametrize("ntris,every", [(1500, 1), (3000, 700), (2047, 2047)])
+def test_emitter_table(gpu, orc, ntris, every):
+    s = scenes.c1_plain(ntris=ntris, width=32, height=24, spp=2)
+    s.mats[:ntris:every, 8:11] = 0.5
+    cam = cam_of(s, 32, 24)
+    want, rays = oracle_lib.TraceOracle(orc, s).trace(cam, 0, 2)
+    tr = px.Tracer.of(gpu, s)
+    tr.trace(cam, 32, 24, 0, 2)
+    check_image(tr.image(), want, 32 * 24)
+    assert tr.time()[1] == rays
+    tr.close()
