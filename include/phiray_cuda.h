@@ -218,8 +218,9 @@ typedef struct phx_bvh_s* phx_bvh;
  * numbering, bounds refit bottom up. All pointers are DEVICE memory:
  * prims (n phx_aabb), nodes (room for 2n - 1), order (n). Writes the node
  * count and depth; stream-ordered, waits once or twice per tree level.
- * Nodes under 64 slots are a thread's, 64-2,047 a block's, larger ones are
- * cut over blocks of 2,048 slots (1.3 M prims: ~9 ms). */
+ * A node under 128 slots and its whole subtree are a warp's, 128-2,047 slots
+ * a block's, larger ones are cut over blocks of 2,048 slots (1.3 M prims:
+ * ~5 ms). */
 int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32_t leaf, phx_node* nodes,
                           uint32_t* order, uint32_t* node_count, uint32_t* depth);
 

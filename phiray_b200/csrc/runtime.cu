@@ -91,16 +91,21 @@ int32_t wait_stream(cudaStream_t s, uint32_t timeout_ms) {
         cudaEventDestroy(ev);
         return cuda_check(e, "cudaEventRecord");
     }
-    const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeout_ms);
-    int spins = 0;
+    const auto began = std::chrono::steady_clock::now();
+    const auto deadline = began + std::chrono::milliseconds(timeout_ms);
+    // Polled without a pause for the first millisecond: a sleep of 50 us is
+    // late by as much again, and a build that waits once a level of the tree
+    // (16 waits) spent 1 of its 5.4 ms in them.
+    const auto patient = began + std::chrono::milliseconds(1);
     for (;;) {
         e = cudaEventQuery(ev);
         if (e != cudaErrorNotReady) break;
-        if (std::chrono::steady_clock::now() > deadline) {
+        const auto now = std::chrono::steady_clock::now();
+        if (now > deadline) {
             cudaEventDestroy(ev);
             return fail(PHX_ERR_TIMEOUT, "device did not drain within %u ms", timeout_ms);
         }
-        if (++spins > 64) std::this_thread::sleep_for(std::chrono::microseconds(50));
+        if (now > patient) std::this_thread::sleep_for(std::chrono::microseconds(50));
     }
     cudaEventDestroy(ev);
     return cuda_check(e, "stream wait");

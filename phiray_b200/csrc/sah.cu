@@ -1,19 +1,20 @@
 // The binned SAH builder on the device (phiray src/bvh/sah.rs:25-189,
 // Bvh::build_sah): the tree phiray's tracer walks, node for node.
 //
-// Level by level: every open node of a level is one thread that bins its
-// slots, sweeps the 3 x 15 planes, and either becomes a leaf or partitions
-// its slots in place (the reference's swap loop) and opens two children in
-// the next level's list. Temporary ids come from a counter; once the tree
-// is complete, inner-node counts (bottom up) and depth-first ranks (top
-// down) give every node the index the reference's work stack hands out,
-// and a last bottom-up pass writes the nodes with their bounds.
+// Top down, level by level, while nodes of SUB slots or more are open: each is
+// binned, swept over the 3 x 15 planes, and either becomes a leaf or partitions
+// its slots as the reference's swap loop does and opens two children in the
+// next level's list (temporary ids come from a counter). Nodes under SUB slots
+// wait as seeds: one launch then builds every seed's whole subtree, a warp
+// each. Once the tree is complete, inner-node counts (bottom up) and
+// depth-first ranks (top down) give every node the index the reference's work
+// stack hands out, and the nodes are written with their bounds, the subtrees
+// first.
 //
-// Nodes under MID slots are one thread each, running the per-node code of
-// sah_core.cuh; nodes of MID to BIG slots a block each (64 threads up to
+// Nodes of SUB to BIG slots are a block each (64 threads up to
 // LARGE slots, 256 above; bins by shared-memory atomics, the swap loop's
 // result by the queue model below, in shared memory). Nodes of BIG slots or more —
-// the top levels, where a node a thread or warp would leave the GPU idle —
+// the top levels, where a node a block would leave the GPU idle —
 // are cut over blocks of CHUNK slots: the box of centres and the bins are min/max and count reductions
 // (exact in any order) merged with atomics; one thread a node then makes
 // the reference's decision from those bins (sah_core.cuh decide); and the
@@ -45,23 +46,27 @@ __global__ void k_sah_init(const float* __restrict__ prims, uint32_t n, float* _
     order[i] = i;
 }
 
+// A TNode's `left` while it waits as a seed (its subtree is built, counted
+// and written by k_sah_subtree and k_sah_subtree_emit).
+constexpr uint32_t SEED = sah::NONE - 1u;
+
 __global__ void k_sah_count(const uint32_t* __restrict__ list, uint32_t count, const TNode* __restrict__ tn,
                             uint32_t* inner) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < count) sah::count_inner(list[k], tn, inner);
+    if (k < count && tn[list[k]].left != SEED) sah::count_inner(list[k], tn, inner);
 }
 
 __global__ void k_sah_place(const uint32_t* __restrict__ list, uint32_t count, const TNode* __restrict__ tn,
                             const uint32_t* __restrict__ inner, uint32_t* rank, uint32_t* final_index) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < count) sah::place(list[k], tn, inner, rank, final_index);
+    if (k < count && tn[list[k]].left != SEED) sah::place(list[k], tn, inner, rank, final_index);
 }
 
 __global__ void k_sah_emit(const uint32_t* __restrict__ list, uint32_t count, const TNode* __restrict__ tn,
                            const uint32_t* __restrict__ final_index, const float* __restrict__ prims,
                            const uint32_t* __restrict__ order, sah::Box* boxes, float* nodes) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < count) sah::emit(list[k], tn, final_index, prims, order, boxes, nodes);
+    if (k < count && tn[list[k]].left != SEED) sah::emit(list[k], tn, final_index, prims, order, boxes, nodes);
 }
 
 inline uint32_t blocks_of(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
@@ -73,11 +78,14 @@ constexpr uint32_t CHUNK_THREADS = 256;
 constexpr uint32_t CHUNK_ITEMS = 8;
 constexpr uint32_t CHUNK = CHUNK_THREADS * CHUNK_ITEMS;
 constexpr uint32_t HBINS = 3 * sah::BINS;
+constexpr uint32_t JUMPS = 64;  // hops and rounds of k_part_jump
+constexpr uint32_t JUMP_ROUNDS = 5;
 
 // A big node of the level and what is decided about it.
 struct BigNode {
     uint32_t t, start, end, depth;
     uint32_t cut, axis, at, m, first_right;
+    uint32_t chunk0, chunk1;  // its chunks in the level's table
     float lo[3], scale[3];
     uint32_t cbox[6];            // box of centres, as ordered words (lo xyz, hi xyz)
     uint32_t bcount[HBINS];      // per axis and bin: slots
@@ -97,6 +105,16 @@ __device__ __forceinline__ uint32_t ord(float f) {
 }
 __device__ __forceinline__ float unord(uint32_t w) {
     return __uint_as_float((w & 0x80000000u) ? (w & 0x7FFFFFFFu) : ~w);
+}
+
+// *p lowered (raised) to v: the word is read first, since once a few slots are
+// in, most lie inside their bin's box, and a word only ever moves one way, so
+// a stale reading never skips a change that counts.
+__device__ __forceinline__ void low_to(volatile uint32_t* p, uint32_t v) {
+    if (v < *p) atomicMin((uint32_t*)p, v);
+}
+__device__ __forceinline__ void high_to(volatile uint32_t* p, uint32_t v) {
+    if (v > *p) atomicMax((uint32_t*)p, v);
 }
 
 template <int THREADS = CHUNK_THREADS>
@@ -125,11 +143,11 @@ __device__ __forceinline__ uint32_t block_sum_exclusive(uint32_t v, uint32_t* to
     return before;
 }
 
-// ---- nodes of MID to BIG slots: a block a node ----
+// ---- nodes of SUB to BIG slots: a block a node ----
 
 // Two block forms: 256 threads for nodes of LARGE to BIG slots, 64 threads
-// for nodes of MID to LARGE (8 slots a thread either way).
-constexpr uint32_t MID = 64;
+// for nodes of SUB to LARGE (8 slots a thread either way).
+constexpr uint32_t SUB = 128;  // nodes under this many slots are seeds
 constexpr uint32_t LARGE = 512;
 constexpr uint32_t NODE_ITEMS = 8;  // slots a thread holds
 static_assert(256 * NODE_ITEMS == BIG && 64 * NODE_ITEMS == LARGE, "a block holds its largest node");
@@ -213,8 +231,8 @@ __global__ void __launch_bounds__(NODE_THREADS, 512 / NODE_THREADS) k_sah_block(
                     const uint32_t at = k * sah::BINS + sah::bin_of(centres + 3 * (uint64_t)i, glo, scale, k);
                     atomicAdd(&s_count[at], 1u);
                     for (int f = 0; f < 3; f++) {  // a NaN bound loses, as in f32::min / max
-                        if (p[f] == p[f]) atomicMin(&s_box[6 * at + f], ord(p[f]));
-                        if (p[4 + f] == p[4 + f]) atomicMax(&s_box[6 * at + 3 + f], ord(p[4 + f]));
+                        if (p[f] == p[f]) low_to(&s_box[6 * at + f], ord(p[f]));
+                        if (p[4 + f] == p[4 + f]) high_to(&s_box[6 * at + 3 + f], ord(p[4 + f]));
                     }
                 }
             }
@@ -320,51 +338,401 @@ __global__ void __launch_bounds__(NODE_THREADS, 512 / NODE_THREADS) k_sah_block(
     tn[t] = nd;
 }
 
-// The level's open nodes, split into the big ones (BIG slots or more, not
-// at the depth cap) and the rest.
-// (counts: small, big, mid, large, and in counts[4] the level's length.)
+// The level's open nodes, split by size; the small ones become seeds.
+// (counts: big, mid, large of this level, its length, the seeds so far; the
+// deepest seed node, the level's chunks and the marks of k_part_jump's rounds
+// are kept beside them.)
 // The length is `count`, or *dcount when given: the children the level
 // before opened, so the host learns them with this level's counts, in one
 // wait; the grid then covers an upper bound.
-__global__ void k_sah_classify(const uint32_t* __restrict__ list, uint32_t count, const uint32_t* dcount,
-                               const TNode* __restrict__ tn, uint32_t* small, uint32_t* big, uint32_t* mid,
-                               uint32_t* large, uint32_t* counts) {
+enum : uint32_t { LC_BIG = 0, LC_MID, LC_LARGE, LC_LEN, LC_SEEDS, LC_DEPTH, LC_CHUNKS, LC_PENDING, LC_WORDS = LC_PENDING + 6 };
+
+__global__ void k_sah_classify(const uint32_t* __restrict__ list, uint32_t count, const uint32_t* dcount, TNode* tn,
+                               uint32_t* seeds, uint32_t* big, uint32_t* mid, uint32_t* large, uint32_t* counts) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (dcount) count = *dcount;
-    if (k == 0) counts[4] = count;
+    if (k == 0) counts[LC_LEN] = count;
     if (k >= count) return;
     const uint32_t t = list[k];
     const TNode nd = tn[t];
     const uint32_t n = nd.end - nd.start;
-    const bool open = nd.depth + 1 < sah::MAX_DEPTH;
-    if (open && n >= BIG) big[atomicAdd(counts + 1, 1u)] = t;
-    else if (open && n >= LARGE) large[atomicAdd(counts + 3, 1u)] = t;
-    else if (open && n >= MID) mid[atomicAdd(counts + 2, 1u)] = t;
-    else small[atomicAdd(counts, 1u)] = t;
+    uint32_t kind = LC_SEEDS;
+    if (nd.depth + 1 < sah::MAX_DEPTH && n >= SUB) kind = n >= BIG ? LC_BIG : (n >= LARGE ? LC_LARGE : LC_MID);
+    // one atomic a warp and kind
+    const uint32_t m = __match_any_sync(__activemask(), kind), lane = threadIdx.x & 31u;
+    const uint32_t leader = __ffs(m) - 1u;
+    uint32_t at = 0;
+    if (lane == leader) at = atomicAdd(counts + kind, (uint32_t)__popc(m));
+    at = __shfl_sync(m, at, leader) + __popc(m & ((1u << lane) - 1u));
+    if (kind == LC_SEEDS) {
+        seeds[at] = t;
+        tn[t].left = SEED;
+    } else {
+        (kind == LC_BIG ? big : (kind == LC_LARGE ? large : mid))[at] = t;
+    }
 }
 
-// Nodes under MID slots (and nodes at the depth cap): a thread a node,
-// sah_core.cuh process as it is.
-struct DeviceAdd {
-    __device__ uint32_t operator()(uint32_t* p, uint32_t v) const { return atomicAdd(p, v); }
+// ---- whole subtrees of the seeds, a warp each ----
+//
+// A thread a node and a launch a level spent 2.9 of the 8.1 ms a 1.3 M-box
+// build took: serial loops over scattered slots, 12 levels of them (now 1.7 in
+// one launch, of a 4.9 ms build; seeds of 64 slots 1.5, with two more levels
+// of blocks above them, 5.2). What bounds it now is instructions: about 400 a
+// node and 54 a slot and node. Here a
+// seed's boxes and centres are read once into shared memory and the subtree
+// is built there, in the reference's depth-first order: each lane holds four
+// slots, the planes of the three axes are priced by a lane each (a loop over
+// the node's slots, every lane reading the same box), and the partition is
+// the queue model by bit masks. Depth-first numbering makes a node's final
+// index a function of the seed's rank. The nodes of a seed of n slots at
+// `start` are records loc[2 start ..): (start, end, parent's inner rank * 2 +
+// side or NONE, own inner rank or SUB_LEAF | depth << 8).
+constexpr uint32_t SUB_WARPS = 4;
+constexpr uint32_t SUB_LEAF = 255u;
+constexpr uint32_t SUB_LANE = SUB / 32;  // positions a lane holds
+
+struct SubShared {
+    float c[3][SUB], lo[3][SUB], hi[3][SUB];
+    uint32_t slot[SUB];
+    uint32_t stack[SUB];  // start | end << 8 | depth << 16 | side << 31; the code's rank beside it
+    uint8_t rank_of[SUB];
+    uint8_t idx[SUB];     // position -> the slot's place in the arrays above
+    uint8_t bin[3][SUB];
+    uint32_t lefts[SUB_LANE], before[SUB_LANE];  // the left slots' mask, lefts before each word
 };
 
-__global__ void k_sah_thread(const uint32_t* __restrict__ list, uint32_t count, TNode* tn,
-                             const float* __restrict__ prims, const float* __restrict__ centres, uint32_t* order,
-                             uint32_t leaf, uint32_t* tcount, uint32_t* next, uint32_t* next_count) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    sah::process(list[k], tn, prims, centres, order, leaf, tcount, next, next_count, DeviceAdd{});
+// Left slots before position x.
+__device__ __forceinline__ uint32_t lefts_before(const SubShared& w, uint32_t x) {
+    return w.before[x >> 5] + __popc(w.lefts[x >> 5] & ((1u << (x & 31u)) - 1u));
 }
 
-__global__ void k_big_setup(const uint32_t* __restrict__ big, uint32_t nb, const TNode* __restrict__ tn,
-                            BigNode* bn, uint2* spans) {
+// Area of the box (lo, hi) (sah.rs:32-35).
+__device__ __forceinline__ float area_of(const float* lo, const float* hi) {
+    sah::Box b;
+    for (int k = 0; k < 3; k++) {
+        b.lo[k] = lo[k];
+        b.hi[k] = hi[k];
+    }
+    return sah::area(b);
+}
+
+// A plane's two sides over positions j0, j0 + step, .. < j1: boxes and counts.
+struct Sides {
+    float llo[3], lhi[3], rlo[3], rhi[3];
+    uint32_t lc, rc;
+};
+
+__device__ __forceinline__ Sides sides_of(const SubShared& w, uint32_t axis, uint32_t at, uint32_t j0, uint32_t j1,
+                                          uint32_t step) {
+    constexpr float BIGF = 3.402823466e38f;
+    Sides s;
+    for (int k = 0; k < 3; k++) {
+        s.llo[k] = s.rlo[k] = BIGF;
+        s.lhi[k] = s.rhi[k] = -BIGF;
+    }
+    s.lc = s.rc = 0;
+    for (uint32_t j = j0; j < j1; j += step) {
+        const uint32_t i = w.idx[j];
+        const bool left = w.bin[axis][i] <= at;
+        for (int k = 0; k < 3; k++) {
+            const float lo = w.lo[k][i], hi = w.hi[k][i];
+            s.llo[k] = fminf(s.llo[k], left ? lo : BIGF);
+            s.lhi[k] = fmaxf(s.lhi[k], left ? hi : -BIGF);
+            s.rlo[k] = fminf(s.rlo[k], left ? BIGF : lo);
+            s.rhi[k] = fmaxf(s.rhi[k], left ? -BIGF : hi);
+        }
+        s.lc += left ? 1u : 0u;
+        s.rc += left ? 0u : 1u;
+    }
+    return s;
+}
+
+// An axis's sweep (sweep_axis) from its planes' costs, plane `at` in lane
+// first + at: the first plane with two sides if its cost is no number, else
+// the lowest cost, the lower plane on a tie. Every lane calls.
+__device__ __forceinline__ sah::AxisBest axis_best(bool priced, float cost, uint32_t first, uint32_t lane) {
+    const bool mine = lane >= first && lane < first + 15u && priced;
+    const uint32_t planes = __ballot_sync(0xffffffffu, mine);
+    const float c0 = __shfl_sync(0xffffffffu, cost, planes ? __ffs(planes) - 1 : 0);
+    if (!planes) return sah::AxisBest{false, 0.0f, 0u};
+    if (c0 != c0) return sah::AxisBest{true, c0, (uint32_t)__ffs(planes) - 1u - first};
+    // costs are sums of products of areas and counts: none is negative
+    const uint32_t key = mine && cost == cost ? __float_as_uint(cost) : 0xFFFFFFFFu;
+    const uint32_t low = __reduce_min_sync(0xffffffffu, key);
+    const uint32_t who = __ballot_sync(0xffffffffu, key == low);
+    return sah::AxisBest{true, __uint_as_float(low), (uint32_t)__ffs(who) - 1u - first};
+}
+
+__global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree(const uint32_t* __restrict__ seeds, uint32_t nseeds,
+                                                                const TNode* __restrict__ tn,
+                                                                const float* __restrict__ prims,
+                                                                const float* __restrict__ centres, uint32_t* order,
+                                                                uint32_t leaf, uint4* __restrict__ loc,
+                                                                uint32_t* __restrict__ loc_count, uint32_t* inner,
+                                                                uint32_t* max_depth) {
+    __shared__ SubShared shared[SUB_WARPS];
+    const uint32_t lane = threadIdx.x & 31u, k0 = blockIdx.x * SUB_WARPS + (threadIdx.x >> 5);
+    if (k0 >= nseeds) return;
+    SubShared& w = shared[threadIdx.x >> 5];
+    const uint32_t t = seeds[k0];
+    const TNode seed = tn[t];
+    const uint32_t total = seed.end - seed.start;
+    uint4* out = loc + 2 * (uint64_t)seed.start;
+    if (seed.depth + 1 >= sah::MAX_DEPTH || total <= 1u) {
+        if (lane == 0) {
+            out[0] = make_uint4(seed.start, seed.end, sah::NONE, SUB_LEAF | seed.depth << 8);
+            loc_count[k0] = 1u;
+            inner[t] = 0u;
+            atomicMax(max_depth, seed.depth);
+        }
+        return;
+    }
+    for (uint32_t j = lane; j < total; j += 32u) {
+        const uint32_t i = order[seed.start + j];
+        w.slot[j] = i;
+        w.idx[j] = (uint8_t)j;
+        const float4 a = __ldg((const float4*)prims + 2 * (uint64_t)i), b = __ldg((const float4*)prims + 2 * (uint64_t)i + 1);
+        w.lo[0][j] = a.x;
+        w.lo[1][j] = a.y;
+        w.lo[2][j] = a.z;
+        w.hi[0][j] = b.x;
+        w.hi[1][j] = b.y;
+        w.hi[2][j] = b.z;
+        for (int k = 0; k < 3; k++) w.c[k][j] = __ldg(centres + 3 * (uint64_t)i + k);
+    }
+    __syncwarp();
+    uint32_t sp = 0, ninner = 0, nrec = 0, deepest = seed.depth;
+    uint32_t s = 0, e = total, depth = seed.depth, code = sah::NONE;
+    for (;;) {
+        const uint32_t n = e - s;
+        uint32_t m = sah::NONE;
+        if (depth + 1 < sah::MAX_DEPTH && n > 1u) {
+            // this lane's positions s + lane, s + 32 + lane, ..
+            uint32_t mine[SUB_LANE];
+            bool held[SUB_LANE];
+            float lo[3], scale[3];
+            sah::Box cbox;
+#pragma unroll
+            for (uint32_t q = 0; q < SUB_LANE; q++) {
+                held[q] = q * 32u + lane < n;
+                mine[q] = 0u;
+                if (q * 32u < n && held[q]) mine[q] = w.idx[s + q * 32u + lane];  // (most nodes need one word)
+            }
+            for (int k = 0; k < 3; k++) {
+                uint32_t l = ord(3.402823466e38f), h = ord(-3.402823466e38f);
+#pragma unroll
+                for (uint32_t q = 0; q < SUB_LANE; q++) {
+                    if (q * 32u >= n) break;
+                    const float c = w.c[k][mine[q]];
+                    if (held[q] && c == c) {
+                        l = min(l, ord(c));
+                        h = max(h, ord(c));
+                    }
+                }
+                cbox.lo[k] = unord(__reduce_min_sync(0xffffffffu, l));
+                cbox.hi[k] = unord(__reduce_max_sync(0xffffffffu, h));
+            }
+            if (!sah::grid_of(cbox, lo, scale)) {
+                if (n > leaf) m = n / 2u;
+            } else {
+#pragma unroll
+                for (uint32_t q = 0; q < SUB_LANE; q++)
+                    if (q * 32u < n && held[q]) {
+                        const float c[3] = {w.c[0][mine[q]], w.c[1][mine[q]], w.c[2][mine[q]]};
+                        for (int k = 0; k < 3; k++) w.bin[k][mine[q]] = (uint8_t)sah::bin_of(c, lo, scale, k);
+                    }
+                __syncwarp();
+                // axes 0 and 1: a lane a plane; axis 2: two lanes a plane, each half the slots
+                sah::AxisBest axes[3];
+                sah::Box bounds;
+                {
+                    const uint32_t axis = lane < 15u ? 0u : 1u;
+                    const Sides d = sides_of(w, axis, lane < 30u ? lane - 15u * axis : 0u, s, e, 1u);
+                    const bool priced = d.lc != 0u && d.rc != 0u && (axis ? scale[1] : scale[0]) != 0.0f;
+                    const float cost = area_of(d.llo, d.lhi) * (float)d.lc + area_of(d.rlo, d.rhi) * (float)d.rc;
+                    axes[0] = axis_best(priced, cost, 0u, lane);
+                    axes[1] = axis_best(priced, cost, 15u, lane);
+                    for (int k = 0; k < 3; k++) {
+                        bounds.lo[k] = fminf(d.llo[k], d.rlo[k]);
+                        bounds.hi[k] = fmaxf(d.lhi[k], d.rhi[k]);
+                    }
+                }
+                {
+                    Sides d = sides_of(w, 2u, lane & 15u, s + (lane >> 4), e, 2u);
+                    for (int k = 0; k < 3; k++) {
+                        d.llo[k] = fminf(d.llo[k], __shfl_xor_sync(0xffffffffu, d.llo[k], 16));
+                        d.lhi[k] = fmaxf(d.lhi[k], __shfl_xor_sync(0xffffffffu, d.lhi[k], 16));
+                        d.rlo[k] = fminf(d.rlo[k], __shfl_xor_sync(0xffffffffu, d.rlo[k], 16));
+                        d.rhi[k] = fmaxf(d.rhi[k], __shfl_xor_sync(0xffffffffu, d.rhi[k], 16));
+                    }
+                    d.lc += __shfl_xor_sync(0xffffffffu, d.lc, 16);
+                    d.rc += __shfl_xor_sync(0xffffffffu, d.rc, 16);
+                    const bool priced = d.lc != 0u && d.rc != 0u && scale[2] != 0.0f;
+                    const float cost = area_of(d.llo, d.lhi) * (float)d.lc + area_of(d.rlo, d.rhi) * (float)d.rc;
+                    axes[2] = axis_best(priced, cost, 0u, lane);
+                }
+                const sah::Decision cut = sah::decide_from(axes, scale, bounds, n, leaf);
+                if (cut.cut == sah::CUT_HALF) m = n / 2u;
+                if (cut.cut == sah::CUT_PLANE) {
+                    uint32_t count = 0;
+#pragma unroll
+                    for (uint32_t q = 0; q < SUB_LANE; q++) {
+                        if (q * 32u >= n) break;
+                        const uint32_t word =
+                            __ballot_sync(0xffffffffu, held[q] && w.bin[cut.axis][mine[q]] <= cut.at);
+                        if (lane == 0) {
+                            w.lefts[q] = word;
+                            w.before[q] = count;
+                        }
+                        count += __popc(word);
+                    }
+                    __syncwarp();
+                    if (count == 0u || count == n) {
+                        m = n / 2u;  // no left slot or no right one: the swap loop moved nothing
+                    } else {
+                        m = count;
+                        uint8_t put[SUB_LANE];
+#pragma unroll
+                        for (uint32_t q = 0; q < SUB_LANE; q++) {
+                            // position x of the result: the x-th left slot, or (with
+                            // the log shifted by the first right slot) entry x,
+                            // chased to the slot it carries
+                            const uint32_t x = q * 32u + lane;
+                            put[q] = 0;
+                            if (q * 32u >= n) break;
+                            if (x >= n || x < m) continue;
+                            uint32_t j = x;
+                            while ((w.lefts[j >> 5] >> (j & 31u)) & 1u) j = lefts_before(w, j);
+                            put[q] = w.idx[s + j];
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (uint32_t q = 0; q < SUB_LANE; q++) {
+                            const uint32_t x = q * 32u + lane;
+                            if (q * 32u >= n) break;
+                            if (x < n && x >= m) w.idx[s + x] = put[q];
+                            if (held[q] && ((w.lefts[q] >> lane) & 1u)) w.idx[s + lefts_before(w, x)] = (uint8_t)mine[q];
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+        deepest = max(deepest, depth);
+        if (lane == 0)
+            out[nrec] = make_uint4(seed.start + s, seed.start + e, code, (m == sah::NONE ? SUB_LEAF : ninner) | depth << 8);
+        nrec++;
+        if (m != sah::NONE) {
+            if (lane == 0) {
+                w.stack[sp] = (s + m) | e << 8 | (depth + 1u) << 16;
+                w.rank_of[sp] = (uint8_t)ninner;
+            }
+            sp++;
+            code = ninner * 2u;
+            ninner++;
+            e = s + m;
+            depth++;
+            continue;
+        }
+        if (sp == 0u) break;
+        sp--;
+        __syncwarp();
+        const uint32_t top = w.stack[sp];
+        code = (uint32_t)w.rank_of[sp] * 2u + 1u;
+        s = top & 255u;
+        e = (top >> 8) & 255u;
+        depth = top >> 16;
+        __syncwarp();
+    }
+    for (uint32_t j = lane; j < total; j += 32u) order[seed.start + j] = w.slot[w.idx[j]];
+    if (lane == 0) {
+        loc_count[k0] = nrec;
+        inner[t] = ninner;
+        atomicMax(max_depth, deepest);
+    }
+}
+
+// The seeds' nodes at their final indices, with their bounds: leaves from
+// their primitives in slot order, inner nodes from their children, deepest
+// first (sah_core.cuh emit).
+__global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree_emit(
+    const uint32_t* __restrict__ seeds, uint32_t nseeds, const TNode* __restrict__ tn, const uint4* __restrict__ loc,
+    const uint32_t* __restrict__ loc_count, const uint32_t* __restrict__ rank, const uint32_t* __restrict__ final_index,
+    const float* __restrict__ prims, const uint32_t* __restrict__ order, sah::Box* boxes, float* nodes) {
+    __shared__ float s_box[SUB_WARPS][6][2 * SUB];  // 24 KB
+    __shared__ uint8_t s_child[SUB_WARPS][2 * SUB];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, k0 = blockIdx.x * SUB_WARPS + warp;
+    if (k0 >= nseeds) return;
+    float(*box)[2 * SUB] = s_box[warp];
+    uint8_t* child = s_child[warp];
+    const uint32_t t = seeds[k0], count = loc_count[k0], R = rank[t];
+    const uint4* rec = loc + 2 * (uint64_t)tn[t].start;
+    uint4 mine[2 * SUB_LANE];
+    uint32_t low = sah::MAX_DEPTH, high = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 2u * SUB_LANE; q++) {
+        const uint32_t k = q * 32u + lane;
+        if (k >= count) continue;
+        mine[q] = rec[k];
+        if (mine[q].z != sah::NONE) child[mine[q].z] = (uint8_t)k;
+        if ((mine[q].w & 255u) == SUB_LEAF) {
+            sah::Box b = sah::empty_box();
+            for (uint32_t j = mine[q].x; j < mine[q].y; j++) sah::grow(b, sah::prim_box(prims + 8 * (uint64_t)order[j]));
+            for (int f = 0; f < 3; f++) {
+                box[f][k] = b.lo[f];
+                box[3 + f][k] = b.hi[f];
+            }
+        } else {
+            low = min(low, mine[q].w >> 8);
+            high = max(high, mine[q].w >> 8);
+        }
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
+    __syncwarp();
+    for (uint32_t d = high; d + 1u > low; d--) {
+#pragma unroll
+        for (uint32_t q = 0; q < 2u * SUB_LANE; q++) {
+            const uint32_t k = q * 32u + lane;
+            if (k >= count || (mine[q].w & 255u) == SUB_LEAF || mine[q].w >> 8 != d) continue;
+            const uint32_t r = mine[q].w & 255u, l = child[2 * r], h = child[2 * r + 1];
+            for (int f = 0; f < 3; f++) {
+                box[f][k] = sah::rmin(box[f][l], box[f][h]);
+                box[3 + f][k] = sah::rmax(box[3 + f][l], box[3 + f][h]);
+            }
+        }
+        __syncwarp();
+        if (d == 0u) break;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 2u * SUB_LANE; q++) {
+        const uint32_t k = q * 32u + lane;
+        if (k >= count) continue;
+        const uint32_t code = mine[q].z, r = mine[q].w & 255u;
+        const uint32_t at = code == sah::NONE ? final_index[t] : 2u * (R + (code >> 1)) + 1u + (code & 1u);
+        const bool is_leaf = r == SUB_LEAF;
+        const uint32_t lo_i = is_leaf ? mine[q].x | sah::LEAF_BIT : 2u * (R + r) + 1u;
+        const uint32_t hi_i = is_leaf ? mine[q].y : 2u * (R + r) + 2u;
+        float4* o = (float4*)nodes + 2 * (uint64_t)at;
+        o[0] = make_float4(box[0][k], box[1][k], box[2][k], __uint_as_float(lo_i));
+        o[1] = make_float4(box[3][k], box[4][k], box[5][k], __uint_as_float(hi_i));
+        if (code == sah::NONE) {
+            sah::Box b;
+            for (int f = 0; f < 3; f++) {
+                b.lo[f] = box[f][k];
+                b.hi[f] = box[3 + f][k];
+            }
+            boxes[t] = b;
+        }
+    }
+}
+
+__global__ void k_big_setup(const uint32_t* __restrict__ big, uint32_t nb, const TNode* __restrict__ tn, BigNode* bn) {
     const uint32_t b = blockIdx.x;
     if (b >= nb) return;
     BigNode& B = bn[b];
     if (threadIdx.x == 0) {
         const TNode nd = tn[big[b]];
-        spans[b] = make_uint2(nd.start, nd.end);
         B.t = big[b];
         B.start = nd.start;
         B.end = nd.end;
@@ -382,10 +750,33 @@ __global__ void k_big_setup(const uint32_t* __restrict__ big, uint32_t nb, const
         B.bbox[i] = ord((i % 6) < 3 ? 3.402823466e38f : -3.402823466e38f);
 }
 
+// The level's chunk table, node after node, and its length (one block).
+__global__ void __launch_bounds__(CHUNK_THREADS) k_big_table(BigNode* bn, uint32_t nb, Chunk* __restrict__ chunks,
+                                                             uint32_t* nchunks, uint32_t* pending) {
+    uint32_t run = 0;
+    for (uint32_t b0 = 0; b0 < nb; b0 += CHUNK_THREADS) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint32_t start = b < nb ? bn[b].start : 0u, end = b < nb ? bn[b].end : 0u;
+        const uint32_t mine = (end - start + CHUNK - 1u) / CHUNK;
+        uint32_t total = 0;
+        const uint32_t at = run + block_sum_exclusive(mine, &total);
+        if (b < nb) {
+            bn[b].chunk0 = at;
+            bn[b].chunk1 = at + mine;
+            for (uint32_t k = 0; k < mine; k++)
+                chunks[at + k] = Chunk{b, start + k * CHUNK, min(start + (k + 1u) * CHUNK, end)};
+        }
+        run += total;
+    }
+    if (threadIdx.x == 0) *nchunks = run;
+    if (threadIdx.x <= JUMP_ROUNDS) pending[threadIdx.x] = 0u;
+}
+
 // Box of a big node's centres (sah.rs:121-123).
-__global__ void __launch_bounds__(CHUNK_THREADS) k_big_cbox(const Chunk* __restrict__ chunks, BigNode* bn,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_big_cbox(const Chunk* __restrict__ chunks, const uint32_t* nchunks, BigNode* bn,
                                                             const float* __restrict__ centres,
                                                             const uint32_t* __restrict__ order) {
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
     const Chunk ch = chunks[blockIdx.x];
     float lo[3] = {3.402823466e38f, 3.402823466e38f, 3.402823466e38f};
     float hi[3] = {-3.402823466e38f, -3.402823466e38f, -3.402823466e38f};
@@ -430,12 +821,13 @@ __global__ void k_big_grid(BigNode* bn, uint32_t nb, uint32_t leaf) {
 
 // The bins of a big node (sah.rs:128-140): per axis and bin, the slots and
 // the union of their boxes.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_big_bins(const Chunk* __restrict__ chunks, BigNode* bn,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_big_bins(const Chunk* __restrict__ chunks, const uint32_t* nchunks, BigNode* bn,
                                                             const float* __restrict__ prims,
                                                             const float* __restrict__ centres,
                                                             const uint32_t* __restrict__ order) {
     __shared__ uint32_t s_count[HBINS];
     __shared__ uint32_t s_box[HBINS * 6];
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
     const Chunk ch = chunks[blockIdx.x];
     BigNode& B = bn[ch.b];
     if (B.first_right == 0xFFFFFFFEu) return;  // decided on its grid
@@ -451,8 +843,8 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_big_bins(const Chunk* __restr
             const uint32_t at = k * sah::BINS + sah::bin_of(centres + 3 * (uint64_t)i, lo, scale, k);
             atomicAdd(&s_count[at], 1u);
             for (int e = 0; e < 3; e++) {  // a NaN bound loses, as in f32::min / max
-                if (p[e] == p[e]) atomicMin(&s_box[6 * at + e], ord(p[e]));
-                if (p[4 + e] == p[4 + e]) atomicMax(&s_box[6 * at + 3 + e], ord(p[4 + e]));
+                if (p[e] == p[e]) low_to(&s_box[6 * at + e], ord(p[e]));
+                if (p[4 + e] == p[4 + e]) high_to(&s_box[6 * at + 3 + e], ord(p[4 + e]));
             }
         }
     }
@@ -466,49 +858,86 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_big_bins(const Chunk* __restr
     }
 }
 
-// One thread a big node: the reference's decision from the bins, the left
-// count, and the children's entries (as sah_core.cuh process makes them).
-__global__ void k_big_choose(BigNode* bn, uint32_t nb, TNode* tn, uint32_t leaf, uint32_t* tcount, uint32_t* next,
-                             uint32_t* next_count) {
-    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    BigNode& B = bn[b];
+// A warp a big node: the reference's decision from the bins (a lane a plane,
+// each uniting the bins on its two sides), the left count, and the children's
+// entries (as sah_core.cuh process makes them).
+__global__ void __launch_bounds__(32) k_big_choose(BigNode* bn, TNode* tn, uint32_t leaf, uint32_t* tcount,
+                                                   uint32_t* next, uint32_t* next_count) {
+    __shared__ uint32_t s_count[HBINS], s_box[HBINS * 6];
+    BigNode& B = bn[blockIdx.x];
+    const uint32_t lane = threadIdx.x;
     const uint32_t count = B.end - B.start;
+    uint32_t cut = B.cut, m = B.m, axis = 0, at = 0;
     if (B.first_right != 0xFFFFFFFEu) {
-        uint32_t bcount[3][sah::BINS];
-        sah::Box bbox[3][sah::BINS];
-        for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (uint32_t i = 0; i < (HBINS * 6 + 31) / 32; i++)
+            if (i * 32u + lane < HBINS * 6) s_box[i * 32u + lane] = B.bbox[i * 32u + lane];
+        for (uint32_t i = lane; i < HBINS; i += 32u) s_count[i] = B.bcount[i];
+        __syncwarp();
+        const float scale[3] = {B.scale[0], B.scale[1], B.scale[2]};
+        sah::AxisBest axes[3];
+        sah::Box bounds = sah::empty_box();
+#pragma unroll 1
+        for (uint32_t pass = 0; pass < 2u; pass++) {
+            // axes 0 and 1 in lanes 0-14 and 15-29, then axis 2
+            const uint32_t k = pass ? 2u : (lane < 15u ? 0u : 1u);
+            const uint32_t plane = pass ? lane : lane - 15u * k;
+            sah::Box l = sah::empty_box(), r = sah::empty_box();
+            uint32_t lc = 0, rc = 0;
+#pragma unroll 4
             for (uint32_t a = 0; a < sah::BINS; a++) {
                 const uint32_t i = k * sah::BINS + a;
-                bcount[k][a] = B.bcount[i];
-                for (int e = 0; e < 3; e++) {
-                    bbox[k][a].lo[e] = unord(B.bbox[6 * i + e]);
-                    bbox[k][a].hi[e] = unord(B.bbox[6 * i + 3 + e]);
+                sah::Box b;
+                for (int f = 0; f < 3; f++) {
+                    b.lo[f] = unord(s_box[6 * i + f]);
+                    b.hi[f] = unord(s_box[6 * i + 3 + f]);
+                }
+                if (a <= plane) {
+                    sah::grow(l, b);
+                    lc += s_count[i];
+                } else {
+                    sah::grow(r, b);
+                    rc += s_count[i];
                 }
             }
-        const sah::Decision d = sah::decide(bcount, bbox, B.scale, count, leaf);
-        B.cut = d.cut;
-        B.axis = d.axis;
-        B.at = d.at;
-        if (d.cut == sah::CUT_HALF) B.m = count / 2;
-        if (d.cut == sah::CUT_PLANE) {
-            uint32_t m = 0;
-            for (uint32_t a = 0; a <= d.at; a++) m += bcount[d.axis][a];
+            const bool priced = lc != 0u && rc != 0u && (k == 0u ? scale[0] : (k == 1u ? scale[1] : scale[2])) != 0.0f;
+            const float cost = sah::area(l) * (float)lc + sah::area(r) * (float)rc;
+            if (pass == 0u) {
+                axes[0] = axis_best(priced, cost, 0u, lane);
+                axes[1] = axis_best(priced, cost, 15u, lane);
+                sah::grow(l, r);
+                bounds = l;
+            } else {
+                axes[2] = axis_best(priced, cost, 0u, lane);
+            }
+        }
+        // lane 0's sides of axis 0 make the node's bounds
+        const sah::Decision d = sah::decide_from(axes, scale, bounds, count, leaf);
+        cut = d.cut;
+        axis = d.axis;
+        at = d.at;
+        if (cut == sah::CUT_HALF) m = count / 2;
+        if (cut == sah::CUT_PLANE) {
+            m = __reduce_add_sync(0xffffffffu, lane <= at ? s_count[axis * sah::BINS + lane] : 0u);
             // no left slot or no right one: the swap loop moved nothing
             if (m == 0 || m == count) {
-                B.cut = sah::CUT_HALF;
+                cut = sah::CUT_HALF;
                 m = count / 2;
             }
-            B.m = m;
         }
     }
+    if (lane != 0) return;
+    B.cut = cut;
+    B.axis = axis;
+    B.at = at;
+    B.m = m;
     TNode nd = tn[B.t];
-    if (B.cut == sah::CUT_LEAF) {
+    if (cut == sah::CUT_LEAF) {
         nd.left = nd.right = sah::NONE;
     } else {
         const uint32_t c = atomicAdd(tcount, 2u);
-        tn[c] = TNode{nd.start, nd.start + B.m, nd.depth + 1, sah::NONE, sah::NONE};
-        tn[c + 1] = TNode{nd.start + B.m, nd.end, nd.depth + 1, sah::NONE, sah::NONE};
+        tn[c] = TNode{nd.start, nd.start + m, nd.depth + 1, sah::NONE, sah::NONE};
+        tn[c + 1] = TNode{nd.start + m, nd.end, nd.depth + 1, sah::NONE, sah::NONE};
         nd.left = c;
         nd.right = c + 1;
         const uint32_t p = atomicAdd(next_count, 2u);
@@ -524,10 +953,11 @@ __device__ __forceinline__ bool goes_left(const BigNode& B, const float* centres
 
 // Partition, step 1: each chunk's left slots ranked in the chunk, the
 // chunk's count of them, and the node's first right slot.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_part_flags(const Chunk* __restrict__ chunks, BigNode* bn,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_part_flags(const Chunk* __restrict__ chunks, const uint32_t* nchunks, BigNode* bn,
                                                               const float* __restrict__ centres,
                                                               const uint32_t* __restrict__ order,
                                                               uint32_t* __restrict__ rank, uint32_t* chunk_lefts) {
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
     const Chunk ch = chunks[blockIdx.x];
     BigNode& B = bn[ch.b];
     if (B.cut != sah::CUT_PLANE) return;
@@ -554,29 +984,33 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_part_flags(const Chunk* __res
     if ((threadIdx.x & 31u) == 0 && first != 0xFFFFFFFFu) atomicMin(&B.first_right, first);
 }
 
-// Partition, step 2 (a thread a chunk): the chunk's left count before it
-// within its node (the table lists a node's chunks in order, so they are the
-// chunks before it with the same node).
-__global__ void k_part_chunks(const Chunk* __restrict__ chunks, uint32_t nchunks, const uint32_t* __restrict__ lefts,
-                              uint32_t* offs) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    const uint32_t node = chunks[c].b;
+// Partition, step 2 (a block a node): the left count before each of the
+// node's chunks.
+__global__ void __launch_bounds__(CHUNK_THREADS) k_part_chunks(const BigNode* __restrict__ bn,
+                                                               const uint32_t* __restrict__ lefts, uint32_t* offs) {
+    const BigNode& B = bn[blockIdx.x];
+    if (B.cut != sah::CUT_PLANE) return;
     uint32_t run = 0;
-    for (uint32_t k = c; k-- > 0 && chunks[k].b == node;) run += lefts[k];
-    offs[c] = run;
+    for (uint32_t c0 = B.chunk0; c0 < B.chunk1; c0 += CHUNK_THREADS) {
+        const uint32_t c = c0 + threadIdx.x;
+        uint32_t total = 0;
+        const uint32_t before = block_sum_exclusive(c < B.chunk1 ? lefts[c] : 0u, &total);
+        if (c < B.chunk1) offs[c] = run + before;
+        run += total;
+    }
 }
 
 // Partition, step 3: left slots to their places; from the first right slot
 // on, every slot's log entry (a right slot carries itself; a left slot
 // links to the entry its rotation copies).
-__global__ void __launch_bounds__(CHUNK_THREADS) k_part_scatter(const Chunk* __restrict__ chunks,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_part_scatter(const Chunk* __restrict__ chunks, const uint32_t* nchunks,
                                                                 const BigNode* __restrict__ bn,
                                                                 const float* __restrict__ centres,
                                                                 const uint32_t* __restrict__ order,
                                                                 const uint32_t* __restrict__ rank,
                                                                 const uint32_t* __restrict__ offs, uint32_t* out,
                                                                 uint32_t* ptr, uint32_t* val) {
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
     const Chunk ch = chunks[blockIdx.x];
     const BigNode& B = bn[ch.b];
     if (B.cut != sah::CUT_PLANE) return;
@@ -599,22 +1033,41 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_part_scatter(const Chunk* __r
     }
 }
 
-// Partition, step 4: one round of pointer jumping over the log's links.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_part_jump(const Chunk* __restrict__ chunks,
-                                                             const BigNode* __restrict__ bn,
-                                                             const uint32_t* __restrict__ src, uint32_t* dst) {
+// Partition, step 4: the log's links followed to the slots they carry, up to
+// JUMPS hops a round and in place (a link only ever moves along its own
+// chain, so reading a neighbour's already moved link only shortens the
+// chase). A split near the middle has chains of about log2(n) links, which
+// round 0 follows to their end; a round that leaves some unfinished marks
+// pending[round + 1], and the next does nothing without that mark. Each round
+// multiplies the reach by JUMPS, so JUMP_ROUNDS of them reach 2^30.
+__global__ void __launch_bounds__(CHUNK_THREADS) k_part_jump(const Chunk* __restrict__ chunks, const uint32_t* nchunks,
+                                                             const BigNode* __restrict__ bn, uint32_t* ptr,
+                                                             uint32_t* pending, uint32_t round) {
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
+    if (round && pending[round] == 0u) return;
     const Chunk ch = chunks[blockIdx.x];
     const BigNode& B = bn[ch.b];
     if (B.cut != sah::CUT_PLANE) return;
     const uint32_t end = B.start + (B.end - B.first_right);  // the log's entries
-    for (uint32_t x = ch.lo + threadIdx.x; x < ch.hi && x < end; x += CHUNK_THREADS) dst[x] = src[src[x]];
+    for (uint32_t x = ch.lo + threadIdx.x; x < ch.hi && x < end; x += CHUNK_THREADS) {
+        uint32_t p = __ldcg(ptr + x), h = 1;
+#pragma unroll 1
+        for (; h < JUMPS; h++) {
+            const uint32_t q = __ldcg(ptr + p);
+            if (q == p) break;
+            p = q;
+        }
+        ptr[x] = p;
+        if (h == JUMPS) pending[round + 1] = 1u;
+    }
 }
 
 // Partition, step 5: the right block is the log's last (count - m) entries.
-__global__ void __launch_bounds__(CHUNK_THREADS) k_part_rights(const Chunk* __restrict__ chunks,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_part_rights(const Chunk* __restrict__ chunks, const uint32_t* nchunks,
                                                                const BigNode* __restrict__ bn,
                                                                const uint32_t* __restrict__ ptr,
                                                                const uint32_t* __restrict__ val, uint32_t* out) {
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
     const Chunk ch = chunks[blockIdx.x];
     const BigNode& B = bn[ch.b];
     if (B.cut != sah::CUT_PLANE) return;
@@ -627,9 +1080,10 @@ __global__ void __launch_bounds__(CHUNK_THREADS) k_part_rights(const Chunk* __re
     }
 }
 
-__global__ void __launch_bounds__(CHUNK_THREADS) k_part_copy(const Chunk* __restrict__ chunks,
+__global__ void __launch_bounds__(CHUNK_THREADS) k_part_copy(const Chunk* __restrict__ chunks, const uint32_t* nchunks,
                                                              const BigNode* __restrict__ bn,
                                                              const uint32_t* __restrict__ src, uint32_t* order) {
+    if (blockIdx.x >= *nchunks) return;  // the grid covers an upper bound
     const Chunk ch = chunks[blockIdx.x];
     if (bn[ch.b].cut != sah::CUT_PLANE) return;
     for (uint32_t x = ch.lo + threadIdx.x; x < ch.hi; x += CHUNK_THREADS) order[x] = src[x];
@@ -654,7 +1108,7 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     Ctx* c = &ctx->c;
     cudaStream_t s = c->stream;
     const uint32_t cap = 2 * n - 1;
-    DevMem centres, tn, lists, counters, inner, rank, final_index, boxes;
+    DevMem centres, tn, lists, counters, inner, rank, final_index, boxes, loc, loc_count;
     PHX_TRY(centres.reserve((size_t)n * 12));
     PHX_TRY(tn.reserve((size_t)cap * sizeof(TNode)));
     PHX_TRY(lists.reserve((size_t)cap * 4));
@@ -663,6 +1117,8 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     PHX_TRY(rank.reserve((size_t)cap * 4));
     PHX_TRY(final_index.reserve((size_t)cap * 4));
     PHX_TRY(boxes.reserve((size_t)cap * sizeof(sah::Box)));
+    PHX_TRY(loc.reserve((size_t)2 * n * sizeof(uint4)));
+    PHX_TRY(loc_count.reserve((size_t)cap * 4));
     const float* P = (const float*)prims;
     TNode* T = (TNode*)tn.ptr;
     uint32_t* L = (uint32_t*)lists.ptr;
@@ -680,14 +1136,13 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     // Big-node work arrays (sized for the widest level: at most n / BIG big
     // nodes, n / CHUNK + n / BIG chunks).
     const uint32_t max_big = n / BIG + 1, max_chunks = n / CHUNK + max_big + 1;
-    DevMem small_list, mid_list, large_list, big_list, lcounts, bnodes, spans, chunks, rank_w, lefts, offs, out_w,
-        ptr_a, ptr_b, val_w;
-    PHX_TRY(small_list.reserve((size_t)cap * 4));
-    PHX_TRY(mid_list.reserve((size_t)(n / MID + 1) * 4));
+    DevMem seeds, mid_list, large_list, big_list, lcounts, bnodes, chunks, rank_w, lefts, offs, out_w,
+        ptr_a, val_w;
+    PHX_TRY(seeds.reserve((size_t)cap * 4));
+    PHX_TRY(mid_list.reserve((size_t)(n / SUB + 1) * 4));
     PHX_TRY(large_list.reserve((size_t)(n / LARGE + 1) * 4));
-    PHX_TRY(lcounts.reserve(20));
+    PHX_TRY(lcounts.reserve(LC_WORDS * 4));
     if (n >= BIG) {
-        PHX_TRY(spans.reserve((size_t)max_big * 8));
         PHX_TRY(big_list.reserve((size_t)max_big * 4));
         PHX_TRY(bnodes.reserve((size_t)max_big * sizeof(BigNode)));
         PHX_TRY(chunks.reserve((size_t)max_chunks * sizeof(Chunk)));
@@ -696,78 +1151,61 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
         PHX_TRY(offs.reserve((size_t)max_chunks * 4));
         PHX_TRY(out_w.reserve((size_t)n * 4));
         PHX_TRY(ptr_a.reserve((size_t)n * 4));
-        PHX_TRY(ptr_b.reserve((size_t)n * 4));
         PHX_TRY(val_w.reserve((size_t)n * 4));
     }
     std::vector<uint32_t> off{0}, len{1};
-    std::vector<uint2> host_big;
-    std::vector<Chunk> host_chunks;
     // Level 0's classification; each level then classifies the next one
     // right behind its own kernels, and one wait a level reads both the
     // children opened and their classes.
-    PHX_CUDA(cudaMemsetAsync(lcounts.ptr, 0, 16, s));
-    k_sah_classify<<<1, 256, 0, s>>>(L, 1u, nullptr, T, (uint32_t*)small_list.ptr, (uint32_t*)big_list.ptr,
-                                     (uint32_t*)mid_list.ptr, (uint32_t*)large_list.ptr, (uint32_t*)lcounts.ptr);
+    uint32_t* LC = (uint32_t*)lcounts.ptr;
+    PHX_CUDA(cudaMemsetAsync(LC, 0, LC_WORDS * 4, s));
+    k_sah_classify<<<1, 256, 0, s>>>(L, 1u, nullptr, T, (uint32_t*)seeds.ptr, (uint32_t*)big_list.ptr,
+                                     (uint32_t*)mid_list.ptr, (uint32_t*)large_list.ptr, LC);
+    uint32_t nseeds = 0;
     for (uint32_t lv = 0; lv < sah::MAX_DEPTH; lv++) {
-        uint32_t lc[5] = {0, 0, 0, 0, 0};
-        PHX_CUDA(cudaMemcpyAsync(lc, lcounts.ptr, 20, cudaMemcpyDeviceToHost, s));
+        uint32_t lc[LC_WORDS] = {};
+        PHX_CUDA(cudaMemcpyAsync(lc, LC, LC_WORDS * 4, cudaMemcpyDeviceToHost, s));
         PHX_TRY(wait_stream(s, 0));
+        nseeds = lc[LC_SEEDS];
+        if (nseeds > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than 2n - 1");
         if (lv > 0) {
-            // lc[4]: the children the level before opened (this level's length)
-            if (lc[4] == 0) break;
+            // the children the level before opened (this level's length)
+            if (lc[LC_LEN] == 0) break;
             const uint32_t at = off[lv - 1] + len[lv - 1];
-            if (at + lc[4] > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than 2n - 1");
+            if (at + lc[LC_LEN] > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than 2n - 1");
             off.push_back(at);
-            len.push_back(lc[4]);
+            len.push_back(lc[LC_LEN]);
         }
         const uint32_t next = off[lv] + len[lv];
+        const uint32_t nb = lc[LC_BIG], nmid = lc[LC_MID], nlarge = lc[LC_LARGE];
+        if (nb + nmid + nlarge == 0) break;  // only seeds: no level follows
         PHX_CUDA(cudaMemsetAsync(cnt + 1, 0, 4, s));
-        const uint32_t* level = (const uint32_t*)small_list.ptr;
-        uint32_t nsmall = 0, nmid = 0, nlarge = 0;
         {
-            nsmall = lc[0];
-            nmid = lc[2];
-            nlarge = lc[3];
-            const uint32_t nb = lc[1];
             if (nb) {
                 BigNode* BN = (BigNode*)bnodes.ptr;
-                k_big_setup<<<nb, 256, 0, s>>>((const uint32_t*)big_list.ptr, nb, T, BN, (uint2*)spans.ptr);
-                host_big.resize(nb);
-                PHX_CUDA(cudaMemcpyAsync(host_big.data(), spans.ptr, (size_t)nb * 8, cudaMemcpyDeviceToHost, s));
-                PHX_TRY(wait_stream(s, 0));
-                host_chunks.clear();
-                uint32_t widest = 0;
-                for (uint32_t b = 0; b < nb; b++) {
-                    const uint32_t lo = host_big[b].x, hi = host_big[b].y;
-                    widest = std::max(widest, hi - lo);
-                    for (uint32_t j = lo; j < hi; j += CHUNK) host_chunks.push_back(Chunk{b, j, std::min(j + CHUNK, hi)});
-                }
-                const uint32_t nc = (uint32_t)host_chunks.size();
-                if (nc > max_chunks) return fail(PHX_ERR_DEVICE, "SAH build: chunk table overflow");
                 Chunk* CH = (Chunk*)chunks.ptr;
-                PHX_CUDA(cudaMemcpyAsync(CH, host_chunks.data(), nc * sizeof(Chunk), cudaMemcpyHostToDevice, s));
+                uint32_t* NC = LC + LC_CHUNKS;
+                // a chunk is full but for each node's last
+                const uint32_t nc = std::min(n / CHUNK + nb, max_chunks);
+                k_big_setup<<<nb, 256, 0, s>>>((const uint32_t*)big_list.ptr, nb, T, BN);
+                k_big_table<<<1, CHUNK_THREADS, 0, s>>>(BN, nb, CH, NC, LC + LC_PENDING);
                 const float* Cc = (const float*)centres.ptr;
-                k_big_cbox<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, Cc, order);
+                k_big_cbox<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, Cc, order);
                 k_big_grid<<<blocks_of(nb, 64), 64, 0, s>>>(BN, nb, leaf);
-                k_big_bins<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, P, Cc, order);
-                k_big_choose<<<blocks_of(nb, 64), 64, 0, s>>>(BN, nb, T, leaf, cnt, L + next, cnt + 1);
+                k_big_bins<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, P, Cc, order);
+                k_big_choose<<<nb, 32, 0, s>>>(BN, T, leaf, cnt, L + next, cnt + 1);
                 uint32_t* R = (uint32_t*)rank_w.ptr;
-                k_part_flags<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, Cc, order, R, (uint32_t*)lefts.ptr);
-                k_part_chunks<<<blocks_of(nc, 128), 128, 0, s>>>(CH, nc, (const uint32_t*)lefts.ptr,
-                                                                 (uint32_t*)offs.ptr);
+                k_part_flags<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, Cc, order, R, (uint32_t*)lefts.ptr);
+                k_part_chunks<<<nb, CHUNK_THREADS, 0, s>>>(BN, (const uint32_t*)lefts.ptr, (uint32_t*)offs.ptr);
                 uint32_t* pa = (uint32_t*)ptr_a.ptr;
-                uint32_t* pb = (uint32_t*)ptr_b.ptr;
-                k_part_scatter<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, Cc, order, R, (const uint32_t*)offs.ptr,
+                k_part_scatter<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, Cc, order, R, (const uint32_t*)offs.ptr,
                                                             (uint32_t*)out_w.ptr, pa, (uint32_t*)val_w.ptr);
-                uint32_t rounds = 1;
-                while ((1u << rounds) < widest) rounds++;
-                for (uint32_t r = 0; r <= rounds; r++) {
-                    k_part_jump<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, pa, pb);
-                    std::swap(pa, pb);
-                }
-                k_part_rights<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, pa, (const uint32_t*)val_w.ptr,
+                uint64_t reach = 1;
+                for (uint32_t r = 0; r < JUMP_ROUNDS && reach < n; r++, reach *= JUMPS)
+                    k_part_jump<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, pa, LC + LC_PENDING, r);
+                k_part_rights<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, pa, (const uint32_t*)val_w.ptr,
                                                            (uint32_t*)out_w.ptr);
-                k_part_copy<<<nc, CHUNK_THREADS, 0, s>>>(CH, BN, (const uint32_t*)out_w.ptr, order);
+                k_part_copy<<<nc, CHUNK_THREADS, 0, s>>>(CH, NC, BN, (const uint32_t*)out_w.ptr, order);
                 PHX_CUDA(cudaGetLastError());
             }
         }
@@ -777,33 +1215,40 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
         if (nmid)
             k_sah_block<64><<<nmid, 64, 0, s>>>((const uint32_t*)mid_list.ptr, T, P, (const float*)centres.ptr, order,
                                                 leaf, cnt, L + next, cnt + 1);
-        if (nsmall)
-            k_sah_thread<<<blocks_of(nsmall, 64), 64, 0, s>>>(level, nsmall, T, P, (const float*)centres.ptr, order,
-                                                              leaf, cnt, L + next, cnt + 1);
         PHX_CUDA(cudaGetLastError());
         // the next level: its length is the children just opened (cnt[1]);
         // at most two a node of this level
-        PHX_CUDA(cudaMemsetAsync(lcounts.ptr, 0, 16, s));
+        PHX_CUDA(cudaMemsetAsync(LC, 0, LC_SEEDS * 4, s));
         k_sah_classify<<<blocks_of(2 * len[lv], 256), 256, 0, s>>>(
-            L + next, 0u, cnt + 1, T, (uint32_t*)small_list.ptr, (uint32_t*)big_list.ptr, (uint32_t*)mid_list.ptr,
-            (uint32_t*)large_list.ptr, (uint32_t*)lcounts.ptr);
+            L + next, 0u, cnt + 1, T, (uint32_t*)seeds.ptr, (uint32_t*)big_list.ptr, (uint32_t*)mid_list.ptr,
+            (uint32_t*)large_list.ptr, LC);
         PHX_CUDA(cudaGetLastError());
     }
     const uint32_t levels = (uint32_t)len.size();
+    const uint32_t *SD = (const uint32_t*)seeds.ptr, sub_blocks = blocks_of(nseeds, SUB_WARPS);
+    if (nseeds)
+        k_sah_subtree<<<sub_blocks, 32 * SUB_WARPS, 0, s>>>(SD, nseeds, T, P, (const float*)centres.ptr, order, leaf,
+                                                            (uint4*)loc.ptr, (uint32_t*)loc_count.ptr,
+                                                            (uint32_t*)inner.ptr, LC + LC_DEPTH);
     for (uint32_t lv = levels; lv-- > 0;)
         k_sah_count<<<blocks_of(len[lv], 256), 256, 0, s>>>(L + off[lv], len[lv], T, (uint32_t*)inner.ptr);
     for (uint32_t lv = 0; lv < levels; lv++)
         k_sah_place<<<blocks_of(len[lv], 256), 256, 0, s>>>(L + off[lv], len[lv], T, (const uint32_t*)inner.ptr,
                                                             (uint32_t*)rank.ptr, (uint32_t*)final_index.ptr);
+    if (nseeds)
+        k_sah_subtree_emit<<<sub_blocks, 32 * SUB_WARPS, 0, s>>>(
+            SD, nseeds, T, (const uint4*)loc.ptr, (const uint32_t*)loc_count.ptr, (const uint32_t*)rank.ptr,
+            (const uint32_t*)final_index.ptr, P, order, (sah::Box*)boxes.ptr, (float*)nodes);
     for (uint32_t lv = levels; lv-- > 0;)
         k_sah_emit<<<blocks_of(len[lv], 256), 256, 0, s>>>(L + off[lv], len[lv], T, (const uint32_t*)final_index.ptr, P,
                                                            order, (sah::Box*)boxes.ptr, (float*)nodes);
     PHX_CUDA(cudaGetLastError());
-    uint32_t total = 0;
-    PHX_CUDA(cudaMemcpyAsync(&total, cnt, 4, cudaMemcpyDeviceToHost, s));
+    uint32_t inners = 0, deepest = 0;
+    PHX_CUDA(cudaMemcpyAsync(&inners, inner.ptr, 4, cudaMemcpyDeviceToHost, s));
+    PHX_CUDA(cudaMemcpyAsync(&deepest, LC + LC_DEPTH, 4, cudaMemcpyDeviceToHost, s));
     PHX_TRY(wait_stream(s, 0));
-    *node_count = total;
-    *depth = levels - 1;
+    *node_count = 2 * inners + 1;
+    *depth = std::max(levels - 1, deepest);  // (a leaf that is no seed sits on a level of its own)
     return read_status(c);
 }
 
