@@ -86,6 +86,29 @@ int32_t launch_refit_step(cudaStream_t s, const void* params, void* const* bufs,
 // Face boxes (Aabb::of_tri) of vec4 vertices over uvec4 faces (skin.cu).
 int32_t launch_face_boxes(cudaStream_t s, const float* verts, const uint32_t* faces, uint32_t nfaces, phx_aabb* boxes);
 
+// The weight and bias gradients of one 3x3 convolution, added to dWt
+// ([9 cin][cout]) and db ([cout]) (nn.cu).
+int32_t nn_conv_grads(Ctx* c, const void* X, int xs, int xo, int cin, const void* dY, int dys, int dyo, int cout,
+                      float* dWt, float* db, int B, int H, int W);
+
+// One layer of an Adam step over a whole network (nn.cu k_adam_net): weights
+// [rows][Kp] with their moments, gradient [Kp][rows], bf16 copy and flipped
+// copy (null: none), and the bias. rows and Kp are multiples of 32.
+struct AdamLayer {
+    float *w, *m, *v;
+    const float* g;
+    void *wb, *w2;
+    float *b, *mb, *vb;
+    const float* gb;
+    int rows, Kp, K, cin, Kp2, block0;
+};
+struct AdamNet {
+    AdamLayer l[20];
+    int layers;
+    float lr, b1, b2, eps, c1, c2;
+};
+int32_t nn_adam_net(Ctx* c, AdamNet& net);
+
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 }  // namespace phx

@@ -139,28 +139,6 @@ struct Geo {
     int K, Kp;         // 9 cin, padded to a multiple of 64
 };
 
-// A row of the im2col matrix: the pixel's image, y, x (or -1: past the end).
-struct PixRow {
-    int b, y, x;
-};
-
-__device__ __forceinline__ PixRow pix_row(int p, const Geo& g) {
-    const int P = g.B * g.H * g.W;
-    if (p >= P) return PixRow{-1, 0, 0};
-    const int hw = g.H * g.W;
-    const int b = p / hw, rem = p - b * hw;
-    return PixRow{b, rem / g.W, rem - (rem / g.W) * g.W};
-}
-
-// 8 consecutive k (one tap, 8 channels) of im2col row `pr`, 16 bytes.
-__device__ __forceinline__ uint4 im2col_vec(const bf16* __restrict__ X, const PixRow& pr, int k, const Geo& g) {
-    if (pr.b < 0 || k >= g.K) return make_uint4(0, 0, 0, 0);
-    const int tap = k / g.cin, ci = k - tap * g.cin;
-    const int y = pr.y + tap / 3 - 1, x = pr.x + tap % 3 - 1;
-    if (y < 0 || y >= g.H || x < 0 || x >= g.W) return make_uint4(0, 0, 0, 0);
-    return __ldg((const uint4*)(X + ((size_t)(pr.b * g.H + y) * g.W + x) * g.xs + g.xo + ci));
-}
-
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *(const uint32_t*)&v;
@@ -566,89 +544,184 @@ __global__ void __launch_bounds__(128) k_conv_ws(const bf16* __restrict__ X, con
     if (warp == 0) tc::tmem_free(tm, COLS);
 }
 
-// Weight gradient: dWt[k][co] += sum over pixels p of im2col(X)[p][k] dY[p][co].
-// GEMM rows = k (a 128-row block per CTA), N = cout, the reduction over the
-// pixel range of this CTA's split, 64 pixels a chunk; the tiles are written
-// transposed from the NHWC vectors. The split partial sums meet in dWt by
-// fp32 atomics. dY has pitch `dys` (cout channels at offset 0).
-template <int N>
+// ---- weight gradient: dWt[tap cin + ci][co] += sum over pixels p of
+// X[p + tap][ci] dY[p][co] ----
+//
+// The pixels are the reduction (K), and NHWC keeps the channels of a pixel
+// together, so both operands are read MN-major from the tiles the forward
+// convolution stages: 16-byte vectors of 8 channels, pixel after pixel. (The
+// form before gathered each tap's vectors and wrote them transposed, two bytes
+// a store, and waited for every 64 pixels' MMAs: 2.7 ms of a 4.6 ms training
+// step on 12 x 128^2.) A block walks tiles of 16 x 8 pixels with up to six in
+// flight; per tile, A is dY (M = 128 output channels; the rows past the
+// layer's channels multiply whatever lies there and are not read back), B the
+// input patch at a tap's shift (N = its channels, at most 128), and an MMA
+// takes two image rows of 8 pixels (K = 16). TMEM holds an accumulator a tap:
+// all nine where a tap's has at most 32 columns, else the three of one row of
+// taps, a block each. The bias gradient is one more MMA with a B of ones. The
+// blocks' partial sums meet in dWt by fp32 atomics, consecutive lanes at
+// consecutive output channels.
+struct WgradPlan {
+    int n;             // input channels a block (the last chunk may hold fewer)
+    int taps;          // 9 or 3
+    uint32_t acc;      // TMEM columns of a tap's accumulator
+    uint32_t cols;     // TMEM columns in all
+    int rows;          // patch rows staged
+    int a_bytes, stage, stages, smem;
+};
+
+constexpr int WG_AREA = 16 * 128;  // bytes of dY's 16 x 8 pixels of one 8-channel group
+constexpr int WG_ONES = 512;       // the bias MMA's B: 16 x 16 ones
+
+WgradPlan wgrad_plan(int cin, int cout) {
+    WgradPlan p;
+    const int chunks = (cin + 127) / 128;
+    p.n = ((cin / 16 + chunks - 1) / chunks) * 16;
+    p.acc = tc::tmem_cols(p.n);
+    p.taps = p.acc <= 32u ? 9 : 3;
+    p.cols = tc::tmem_cols((int)(p.taps * p.acc + 16));
+    if (p.taps * p.acc + 16 > 256) p.cols = 512;
+    p.rows = p.taps == 9 ? PY : TY;
+    p.a_bytes = std::min(cout, 128) / 8 * WG_AREA;
+    p.stage = p.a_bytes + p.n / 8 * p.rows * ROWB;
+    p.stages = std::max(2, std::min(6, (int)(180 * 1024 / p.stage)));
+    // A's descriptor always spans 16 channel groups from its stage's start
+    p.smem = WG_ONES + std::max(p.stages * p.stage, (p.stages - 1) * p.stage + 16 * WG_AREA);
+    return p;
+}
+
+__host__ __device__ constexpr uint32_t instr_desc_mn(int N) {
+    return tc::instr_desc_bf16(tc::BM, N) | (1u << 15) | (1u << 16);  // A and B MN-major
+}
+
 __global__ void __launch_bounds__(128) k_conv_wgrad(const bf16* __restrict__ X, const bf16* __restrict__ dY, int dys,
-                                                    int dyo, float* __restrict__ dWt, Geo g, int chunk_px,
-                                                    uint32_t* status) {
+                                                    int dyo, float* __restrict__ dWt, float* __restrict__ db, Geo g,
+                                                    WgradPlan pl, uint32_t* status) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[6];
     __shared__ uint32_t tmem_base;
-    using P = Plan<N>;
-    uint8_t* a_tile = smem + P::A_OFF;
-    uint8_t* b_tile = smem + P::B_OFF;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == 0) tc::tmem_alloc(&tmem_base, tc::tmem_cols(N));
+    if (warp == 0) tc::tmem_alloc(&tmem_base, pl.cols);
     if (tid == 0) {
-        tc::mbar_init(&bar, 1);
+        for (int i = 0; i < pl.stages; i++) tc::mbar_init(&bar[i], 1);
         fence_barrier_init();
     }
+    for (int i = tid; i < WG_ONES / 4; i += 128) ((uint32_t*)smem)[i] = 0x3F803F80u;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tm = tmem_base;
-    const int k0 = blockIdx.x * tc::BM;
-    const int P0 = blockIdx.y * chunk_px;
-    const int Ptot = g.B * g.H * g.W;
-    const int P1 = min(P0 + chunk_px, Ptot);
-    // A: this thread stages k-vector rv = tid % 16 (rows rv*8..rv*8+7) at
-    // pixel columns tid / 16 + 8 j.
-    const int rv = tid & 15;
-    const int kv = k0 + rv * 8;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int pb = P0; pb < P1 && ok; pb += tc::BK) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int col = (tid >> 4) + 8 * j;
-            const PixRow pr = pix_row(pb + col < P1 ? pb + col : Ptot, g);
-            const uint4 val = im2col_vec(X, pr, kv, g);
-            const bf16* e = (const bf16*)&val;
-#pragma unroll
-            for (int q = 0; q < 8; q++) *(bf16*)(a_tile + tc::tile_off(rv * 8 + q, col, tc::BM)) = e[q];
+    const int groups = 9 / pl.taps, tap0 = (blockIdx.y % groups) * pl.taps;
+    const int c0 = (blockIdx.y / groups) * pl.n, n = min(pl.n, g.cin - c0);
+    const int m0 = blockIdx.z * 128, cm = min(128, g.cout - m0);
+    const bool bias = db != nullptr && blockIdx.y == 0;
+    const int row0 = pl.taps == 9 ? -1 : tap0 / 3 - 1;  // image row of the patch's first, against the tile's
+    const int tiles_x = (g.W + TX - 1) / TX, tiles_y = (g.H + TY - 1) / TY;
+    const int ntiles = g.B * tiles_x * tiles_y;
+    const int patch_group = pl.rows * ROWB;  // bytes between channel groups of the patch
+
+    auto issue = [&](int tile, int stage) {
+        const int bx = tile % tiles_x, by = (tile / tiles_x) % tiles_y, img = tile / (tiles_x * tiles_y);
+        const int y0 = by * TY, x0 = bx * TX;
+        uint8_t* a = smem + WG_ONES + stage * pl.stage;
+        uint8_t* patch = a + pl.a_bytes;
+        const int ga = cm / 8, gb = n / 8;
+        for (int v = tid; v < TY * TX * ga; v += 128) {
+            const int kg = v % ga, q = v / ga;
+            const int y = y0 + q / TX, x = x0 + q % TX;
+            const bool ok = y < g.H && x < g.W;
+            const bf16* src = ok ? dY + ((size_t)(img * g.H + y) * g.W + x) * dys + dyo + m0 + kg * 8 : dY;
+            cp_async_ca16(a + kg * WG_AREA + q * 16, src, ok ? 16u : 0u);
         }
-        for (int v = tid; v < N * 8; v += 128) {
-            const int bv = v % (N / 8), col = v / (N / 8);
-            const int p = pb + col;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (p < P1) val = __ldg((const uint4*)(dY + (size_t)p * dys + dyo + bv * 8));
-            const bf16* e = (const bf16*)&val;
-#pragma unroll
-            for (int q = 0; q < 8; q++) *(bf16*)(b_tile + tc::tile_off(bv * 8 + q, col, N)) = e[q];
+        for (int v = tid; v < pl.rows * PX * gb; v += 128) {
+            const int kg = v % gb, q = v / gb;
+            const int py = q / PX, px = q - py * PX;
+            const int y = y0 + row0 + py, x = x0 + px - 1;
+            const bool ok = y >= 0 && y < g.H && x >= 0 && x < g.W;
+            const bf16* src = ok ? X + ((size_t)(img * g.H + y) * g.W + x) * g.xs + g.xo + c0 + kg * 8 : X;
+            cp_async_ca16(patch + kg * patch_group + py * ROWB + px * 16, src, ok ? 16u : 0u);
+        }
+    };
+
+    const int first = blockIdx.x, step = gridDim.x;  // (gridDim.x <= ntiles: every block has a tile)
+    const int mine = (ntiles - first + step - 1) / step;
+    for (int k = 0; k < pl.stages - 1; k++) {
+        if (k < mine) issue(first + k * step, k);
+        cp_async_commit();
+    }
+    const uint32_t idesc = instr_desc_mn(n), idesc_bias = instr_desc_mn(16);
+    bool ok = true;
+    for (int i = 0; i < mine; i++) {
+        // this thread's copies of tile i have landed: one commit group a tile,
+        // those of the stages - 2 tiles after it may be in flight
+        switch (pl.stages) {
+            case 2: cp_async_wait<0>(); break;
+            case 3: cp_async_wait<1>(); break;
+            case 4: cp_async_wait<2>(); break;
+            case 5: cp_async_wait<3>(); break;
+            default: cp_async_wait<4>(); break;
         }
         tc::fence_async_smem();
         __syncthreads();
         if (tid == 0) {
             tc::fence_after_sync();
-            tc::mma_chunk<N>(tm, a_tile, b_tile, pb == P0);
-            tc::mma_commit(&bar);
-        }
-        ok = tc::mbar_wait(&bar, phase);
-        phase ^= 1u;
-        ok = __syncthreads_and(ok);
-    }
-    tc::fence_after_sync();
-    if (ok && P0 < P1) {
-        const int k = k0 + warp * 32 + lane;
-#pragma unroll 1
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (k < g.Kp) {
+            const uint32_t a = tc::smem_addr(smem + WG_ONES + (i % pl.stages) * pl.stage);
+            // MN-major: LBO between the two rows of 8 pixels, SBO between channel groups
+            const uint64_t da0 = tc::smem_desc(a, 128, WG_AREA);
+            const uint64_t db0 = tc::smem_desc(a + pl.a_bytes, ROWB, patch_group);
+            const uint64_t ones = tc::smem_desc(tc::smem_addr(smem), 128, 256);
+            for (int t = 0; t < pl.taps; t++) {
+                const int tap = tap0 + t;
+                const int dy = pl.taps == 9 ? tap / 3 : 0, dx = tap % 3;
+                const uint64_t shift = (uint64_t)((dy * ROWB + dx * 16) >> 4);
 #pragma unroll
-                for (int j = 0; j < 16; j++) atomicAdd(dWt + (size_t)k * N + c0 + j, v[j]);
+                for (int r = 0; r < TY / 2; r++)
+                    tc::mma_bf16(tm + (uint32_t)t * pl.acc, da0 + (uint64_t)(r * 256 >> 4),
+                                 db0 + shift + (uint64_t)(r * 2 * ROWB >> 4), idesc, (i | r) ? 1u : 0u);
+            }
+            if (bias)
+                for (int r = 0; r < TY / 2; r++)
+                    tc::mma_bf16(tm + (uint32_t)pl.taps * pl.acc, da0 + (uint64_t)(r * 256 >> 4), ones, idesc_bias,
+                                 (i | r) ? 1u : 0u);
+            tc::mma_commit(&bar[i % pl.stages]);
+        }
+        const int next = i + pl.stages - 1;
+        if (next < mine) {
+            if (i >= 1) ok = tc::mbar_wait(&bar[(i - 1) % pl.stages], ((i - 1) / pl.stages) & 1) && ok;
+            issue(first + next * step, next % pl.stages);
+        }
+        cp_async_commit();
+    }
+    ok = tc::mbar_wait(&bar[(mine - 1) % pl.stages], ((mine - 1) / pl.stages) & 1) && ok;
+    ok = __syncthreads_and(ok);
+    tc::fence_after_sync();
+    if (ok) {
+        const int co = warp * 32 + lane;
+        const uint32_t row = tm + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+        for (int t = 0; t < pl.taps; t++) {
+#pragma unroll 1
+            for (int c = 0; c < n; c += 16) {
+                float v[16];
+                tc::tmem_ld16(row + (uint32_t)t * pl.acc + (uint32_t)c, v);
+                float* o = dWt + (size_t)((tap0 + t) * g.cin + c0 + c) * g.cout + m0 + co;
+                if (co < cm) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) atomicAdd(o + (size_t)j * g.cout, v[j]);
+                }
             }
         }
-    } else if (!ok && tid == 0) {
+        if (bias) {
+            float v[16];
+            tc::tmem_ld16(row + (uint32_t)pl.taps * pl.acc, v);
+            if (co < cm) atomicAdd(db + m0 + co, v[0]);
+        }
+    } else if (tid == 0) {
         atomicOr(status, STATUS_SPIN_LIMIT);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_free(tm, tc::tmem_cols(N));
+    if (warp == 0) tc::tmem_free(tm, pl.cols);
 }
 
 // ---- the network's other layers (elementwise, fp32 math on bf16 data) ----
@@ -931,6 +1004,58 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
     if (wb) wb[i] = __float2bfloat16(nw);
 }
 
+// Adam on every layer of a network in one launch, with the bf16 copies the
+// next forward and data-gradient convolutions read. One 32 x 32 tile of a
+// layer's [rows][Kp] weights a block, through shared memory, so that the
+// weights, moments and bf16 copy (k fastest) and the gradient and the flipped
+// copy (row fastest) are all read and written in whole lines; one more block
+// a layer for its bias. A launch a tensor and a flip a layer (56 of them) took
+// 165 of a training step's 1,860 us. The arithmetic is k_adam's.
+__global__ void __launch_bounds__(256) k_adam_net(const __grid_constant__ AdamNet net) {
+    __shared__ float s_g[32][33];
+    __shared__ bf16 s_w[32][33];
+    int l = 0;
+    while (l + 1 < net.layers && (int)blockIdx.x >= net.l[l + 1].block0) l++;
+    const AdamLayer& L = net.l[l];
+    const int t = (int)blockIdx.x - L.block0, ktiles = L.Kp / 32;
+    auto update = [&](float* w, float* m, float* v, size_t i, float gr) {
+        const float mm = net.b1 * m[i] + (1.0f - net.b1) * gr;
+        const float vv = net.b2 * v[i] + (1.0f - net.b2) * gr * gr;
+        m[i] = mm;
+        v[i] = vv;
+        const float upd = net.lr * (mm / net.c1) / (sqrtf(vv / net.c2) + net.eps);
+        const float nw = w[i] - upd;
+        w[i] = nw;
+        return nw;
+    };
+    if (t == ktiles * (L.rows / 32)) {
+        for (int i = threadIdx.x; i < L.rows; i += 256) update(L.b, L.mb, L.vb, i, L.gb[i]);
+        return;
+    }
+    const int k0 = (t % ktiles) * 32, r0 = (t / ktiles) * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = ty; j < 32; j += 8) s_g[j][tx] = L.g[(size_t)(k0 + j) * L.rows + r0 + tx];
+    __syncthreads();
+#pragma unroll
+    for (int j = ty; j < 32; j += 8) {
+        const int k = k0 + tx;
+        const size_t i = (size_t)(r0 + j) * L.Kp + k;
+        const bf16 b = k < L.K ? __float2bfloat16(update(L.w, L.m, L.v, i, s_g[tx][j])) : __float2bfloat16(0.0f);
+        ((bf16*)L.wb)[i] = b;
+        s_w[tx][j] = b;
+    }
+    if (!L.w2) return;
+    __syncthreads();
+#pragma unroll
+    for (int j = ty; j < 32; j += 8) {  // W2[ci][(8 - tap) cout + co] (k_flip)
+        const int k = k0 + j;
+        if (k >= L.K) continue;
+        const int tap = k / L.cin, ci = k - tap * L.cin;
+        ((bf16*)L.w2)[(size_t)ci * L.Kp2 + (8 - tap) * L.rows + r0 + tx] = s_w[j][tx];
+    }
+}
+
 __device__ __forceinline__ float finite_or_zero(float v) { return isfinite(v) ? v : 0.0f; }
 
 // Network inputs from a traced image (px planes, src/trace/read.rs:37-56).
@@ -1181,19 +1306,17 @@ int32_t conv_fwd_any(Ctx* c, const bf16* X, const bf16* W, const float* bias, vo
     return fail(PHX_ERR_INVALID, "conv: output tile of %d channels (32, 64, 96, 128 or 160)", g.cout);
 }
 
-template <int N>
-int32_t wgrad_n(Ctx* c, const bf16* X, const bf16* dY, int dys, int dyo, float* dWt, const Geo& g) {
-    const int smem = Plan<N>::TOTAL;
+// dWt (and db, unless null) += the gradients of one convolution.
+int32_t conv_wgrad(Ctx* c, const bf16* X, const bf16* dY, int dys, int dyo, float* dWt, float* db, const Geo& g) {
+    const WgradPlan p = wgrad_plan(g.cin, g.cout);
     static std::atomic<uint64_t> done{0};
-    PHX_TRY(smem_limit(k_conv_wgrad<N>, smem, c->device, done));
-    const int P = g.B * g.H * g.W;
-    // Split the pixel reduction so the grid covers the SMs a few times.
-    const int kblocks = (g.Kp + tc::BM - 1) / tc::BM;
-    int splits = (c->sms * 2 + kblocks - 1) / kblocks;
-    int chunk = (P + splits - 1) / splits;
-    chunk = (chunk + tc::BK - 1) / tc::BK * tc::BK;
-    splits = (P + chunk - 1) / chunk;
-    k_conv_wgrad<N><<<dim3(kblocks, splits), 128, smem, c->stream>>>(X, dY, dys, dyo, dWt, g, chunk, c->status);
+    PHX_TRY(smem_limit(k_conv_wgrad, 224 * 1024, c->device, done));
+    const int ntiles = g.B * ((g.H + TY - 1) / TY) * ((g.W + TX - 1) / TX);
+    const int gy = 9 / p.taps * ((g.cin + p.n - 1) / p.n), gz = (g.cout + 127) / 128;
+    // the tiles are split so that the blocks fill the SMs once (a block's
+    // accumulators take most of an SM's TMEM)
+    const int splits = std::max(1, std::min(ntiles, c->sms / (gy * gz)));
+    k_conv_wgrad<<<dim3(splits, gy, gz), 128, p.smem, c->stream>>>(X, dY, dys, dyo, dWt, db, g, p, c->status);
     return cuda_check(cudaGetLastError(), "conv wgrad");
 }
 
@@ -1210,6 +1333,23 @@ int32_t check_geo(const Geo& g) {
 uint32_t blocks_for(size_t n) { return (uint32_t)((n + 255) / 256); }
 
 }  // namespace
+
+int32_t nn_adam_net(Ctx* c, AdamNet& net) {
+    int blocks = 0;
+    for (int i = 0; i < net.layers; i++) {
+        net.l[i].block0 = blocks;
+        blocks += net.l[i].Kp / 32 * (net.l[i].rows / 32) + 1;
+    }
+    k_adam_net<<<blocks, 256, 0, c->stream>>>(net);
+    return cuda_check(cudaGetLastError(), "adam");
+}
+
+int32_t nn_conv_grads(Ctx* c, const void* X, int xs, int xo, int cin, const void* dY, int dys, int dyo, int cout,
+                      float* dWt, float* db, int B, int H, int W) {
+    const Geo g{B, H, W, cin, xs, xo, cout, cout, 0, 9 * cin, (9 * cin + 63) / 64 * 64};
+    return conv_wgrad(c, (const bf16*)X, (const bf16*)dY, dys, dyo, dWt, db, g);
+}
+
 }  // namespace phx
 
 using namespace phx;
@@ -1250,16 +1390,9 @@ int32_t phx_nn_conv_wgrad(phx_ctx ctx, const void* X, int32_t xs, int32_t xo, in
     if (dys % 8 || dyo % 8 || dyo < 0 || dyo + cout > dys)
         return fail(PHX_ERR_INVALID, "wgrad: dY pitch/offset must be multiples of 8 holding cout channels");
     PHX_TRY(use(&ctx->c));
-    const bf16* x = (const bf16*)X;
-    const bf16* d = (const bf16*)dY;
-    switch (cout) {
-        case 32: return wgrad_n<32>(&ctx->c, x, d, dys, dyo, dWt, g);
-        case 64: return wgrad_n<64>(&ctx->c, x, d, dys, dyo, dWt, g);
-        case 96: return wgrad_n<96>(&ctx->c, x, d, dys, dyo, dWt, g);
-        case 128: return wgrad_n<128>(&ctx->c, x, d, dys, dyo, dWt, g);
-        case 160: return wgrad_n<160>(&ctx->c, x, d, dys, dyo, dWt, g);
-    }
-    return fail(PHX_ERR_INVALID, "wgrad: %d output channels (32, 64, 96, 128 or 160)", cout);
+    if (cout != 32 && cout != 64 && cout != 96 && cout != 128 && cout != 160)
+        return fail(PHX_ERR_INVALID, "wgrad: %d output channels (32, 64, 96, 128 or 160)", cout);
+    return conv_wgrad(&ctx->c, (const bf16*)X, (const bf16*)dY, dys, dyo, dWt, nullptr, g);
 }
 
 int32_t phx_nn_bias_grad(phx_ctx ctx, const void* dY, int32_t dys, int32_t dyo, int32_t C, int32_t P, float* db) {

@@ -164,9 +164,7 @@ int32_t layer_fwd(phx_unet_s* n, int i, View in, View out, const Shape& s, int l
 int32_t layer_bwd(phx_unet_s* n, int i, View x, View dy, View* dx, const Shape& s, int level) {
     Conv& c = n->L[i];
     const int H = s.H >> level, W = s.W >> level;
-    PHX_TRY(phx_nn_conv_wgrad(n->handle, x.p, x.pitch, x.off, c.cin, dy.p, dy.pitch, dy.off, c.cout,
-                              c.gw, c.Kp, s.B, H, W));
-    PHX_TRY(phx_nn_bias_grad(n->handle, dy.p, dy.pitch, dy.off, c.cout, s.B * H * W, c.gb));
+    PHX_TRY(nn_conv_grads(n->ctx, x.p, x.pitch, x.off, c.cin, dy.p, dy.pitch, dy.off, c.cout, c.gw, c.gb, s.B, H, W));
     if (dx)
         PHX_TRY(conv(n, dy, c.cout, c.w2.ptr, c.Kp2, (const float*)n->zero_bias.ptr, *dx, c.cin, s, level, false,
                      false));
@@ -511,14 +509,22 @@ int32_t phx_unet_adam(phx_unet net, float lr) {
     if (!net) return fail(PHX_ERR_INVALID, "null argument");
     PHX_TRY(use(net->ctx));
     const int t = ++net->step;
+    AdamNet a;
+    a.layers = NL;
+    a.lr = lr;
+    a.b1 = net->b1;
+    a.b2 = net->b2;
+    a.eps = net->eps;
+    a.c1 = 1.0f - powf(net->b1, (float)t);
+    a.c2 = 1.0f - powf(net->b2, (float)t);
+    static_assert(NL <= 20, "the layers fit the table");
     for (int i = 0; i < NL; i++) {
         Conv& c = net->L[i];
-        PHX_TRY(phx_nn_adam(net->handle, (float*)c.w32.ptr, c.gw, (float*)c.mw.ptr,
-                            (float*)c.vw.ptr, c.wb.ptr, c.cout, c.Kp, c.K, 1, lr, net->b1, net->b2, net->eps, t));
-        PHX_TRY(phx_nn_adam(net->handle, (float*)c.b32.ptr, c.gb, (float*)c.mb.ptr,
-                            (float*)c.vb.ptr, nullptr, 1, c.cout, c.cout, 0, lr, net->b1, net->b2, net->eps, t));
+        a.l[i] = AdamLayer{(float*)c.w32.ptr, (float*)c.mw.ptr, (float*)c.vw.ptr, c.gw, c.wb.ptr,
+                           i ? c.w2.ptr : nullptr, (float*)c.b32.ptr, (float*)c.mb.ptr, (float*)c.vb.ptr, c.gb,
+                           c.cout, c.Kp, c.K, c.cin, c.Kp2, 0};
     }
-    return flip_all(net);
+    return nn_adam_net(net->ctx, a);
 }
 
 int32_t phx_unet_train_step(phx_unet net, const void* feat, const float* irr, const float* alb, const float* ref,
