@@ -86,6 +86,12 @@ int32_t launch_refit_step(cudaStream_t s, const void* params, void* const* bufs,
 // Face boxes (Aabb::of_tri) of vec4 vertices over uvec4 faces (skin.cu).
 int32_t launch_face_boxes(cudaStream_t s, const float* verts, const uint32_t* faces, uint32_t nfaces, phx_aabb* boxes);
 
+// Y = relu(conv3x3(X, W) + bias) (phx_nn_conv_fwd's arguments); with `below`,
+// the input's first `up` channels are the nearest upsampling of that half-size
+// tensor and X holds the others from xo on; with `pool`, the output's 2 x 2
+// average goes there too (nn.cu).
+int32_t nn_conv_relu(Ctx* c, const void* X, int xs, int xo, int cin, const void* W, int Kp, const float* bias, void* Y,
+                     int ys, int yo, int cout, int B, int H, int Wd, const void* below, int up, void* pool);
 // The weight and bias gradients of one 3x3 convolution, added to dWt
 // ([9 cin][cout]) and db ([cout]) (nn.cu).
 int32_t nn_conv_grads(Ctx* c, const void* X, int xs, int xo, int cin, const void* dY, int dys, int dyo, int cout,

@@ -139,9 +139,24 @@ struct Geo {
     int K, Kp;         // 9 cin, padded to a multiple of 64
 };
 
+// What a forward convolution may do beside itself, each part null or 0 when
+// it does not: take its first `up` input channels from a half-size tensor
+// (H/2 x W/2, `up` channels contiguous), each pixel standing for 2 x 2 (the
+// nearest upsampling k_up_fwd writes out), and write the 2 x 2 average of its
+// bf16 output (H/2 x W/2, cout channels contiguous; k_pool_fwd's).
+struct ConvMore {
+    const bf16* below = nullptr;
+    int up = 0;
+    bf16* pool = nullptr;
+};
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *(const uint32_t*)&v;
+}
+
+__device__ __forceinline__ float2 unpack_bf16x2(uint32_t w) {
+    return __bfloat1622float2(*(const __nv_bfloat162*)&w);
 }
 
 // Asynchronous 16-byte global -> shared copy; src_bytes 0 fills zeros (the
@@ -153,10 +168,72 @@ __device__ __forceinline__ void cp_async_ca16(void* dst, const void* src, uint32
 __device__ __forceinline__ void cp_async_cg16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_addr(dst)), "l"(src) : "memory");
 }
+// The same to a shared-memory address.
+__device__ __forceinline__ void cp_async_ca16_at(uint32_t dst, const void* src, uint32_t src_bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_cg16_at(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// 16 output channels of one pixel: bias, ReLU, the store, and (pool) the 2 x 2
+// average. Lane m of the tile's rows is pixel (m / 8, m % 8), so a pixel's
+// right, lower and diagonal neighbours are lanes + 1, + 8 and + 9; every lane
+// of the warp calls. `live`: the pixel lies in the image.
+template <bool RELU, bool OUT_F32>
+__device__ __forceinline__ void conv_store16(float* v, const float* s_bias, void* Y, size_t p, const Geo& g, int c0,
+                                             bool live, bf16* pool, int img, int y, int x) {
+    const float4* b = (const float4*)(s_bias + c0);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const float4 bv = b[q];
+        v[4 * q] += bv.x;
+        v[4 * q + 1] += bv.y;
+        v[4 * q + 2] += bv.z;
+        v[4 * q + 3] += bv.w;
+    }
+    if (RELU) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.0f);
+    }
+    if constexpr (OUT_F32) {
+        if (!live) return;
+        float4* o = (float4*)((float*)Y + p * g.ys + g.yo + c0);
+#pragma unroll
+        for (int q = 0; q < 4; q++) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+        uint32_t w[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) w[q] = pack_bf16x2(v[2 * q], v[2 * q + 1]);
+        if (live) {
+            uint4* o = (uint4*)((bf16*)Y + p * g.ys + g.yo + c0);
+            o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+        if (!pool) return;
+        uint32_t r[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            float2 s = unpack_bf16x2(w[q]);
+            const float2 a = unpack_bf16x2(__shfl_xor_sync(0xffffffffu, w[q], 1));
+            const float2 c = unpack_bf16x2(__shfl_xor_sync(0xffffffffu, w[q], 8));
+            const float2 d = unpack_bf16x2(__shfl_xor_sync(0xffffffffu, w[q], 9));
+            // k_pool_fwd's order
+            s.x = 0.25f * (((s.x + a.x) + c.x) + d.x);
+            s.y = 0.25f * (((s.y + a.y) + c.y) + d.y);
+            r[q] = pack_bf16x2(s.x, s.y);
+        }
+        if (live && !((y | x) & 1)) {
+            uint4* o = (uint4*)(pool + (((size_t)img * (g.H / 2) + y / 2) * (g.W / 2) + x / 2) * g.cout + c0);
+            o[0] = make_uint4(r[0], r[1], r[2], r[3]);
+            o[1] = make_uint4(r[4], r[5], r[6], r[7]);
+        }
+    }
 }
 
 // ---- the convolution forward: shifted descriptors over a staged patch ----
@@ -198,22 +275,41 @@ struct Conv {
     static constexpr uint32_t COLS = tc::tmem_cols(T * ACC);
 };
 
+// Threads a block: two blocks an SM fit the shared memory whatever the count. At
+// 96 channels 256 threads share the copies and the epilogue's six channel runs
+// evenly (1080p layers of the U-Net 69 / 138 / 64 us against 76 / 141 / 69 with
+// 128); elsewhere 128 do as well or better (N = 64: 119 / 180 / 102 us against
+// 118 / 185 / 106; N = 32 with upsampling: 276 against 284).
+__host__ __device__ constexpr int fwd_threads(int n) { return n == 96 ? 256 : 128; }
+
 // Y = act(conv3x3(X, W) + bias). OUT_F32: fp32 output (the network's head).
-template <int N, int CC, int T, bool RELU, bool OUT_F32>
-__global__ void __launch_bounds__(128) k_conv_fwd(const bf16* __restrict__ X, const bf16* __restrict__ Wt,
+// UP: the first `more.up` input channels come from the half-size tensor.
+// Bound by latency: two blocks an SM, the tensor cores 16 % and the issue slots
+// 24 % busy at N = 64; a chunk waits for its copies, its MMAs and the next
+// chunk's issue in turn. The network's forward pass at 1920 x 1080 took 2.41 ms
+// on the device with the pooling, the upsampling and the copies' addresses
+// worked out each chunk as they were, 1.85 ms now.
+// What a thread copies each chunk is at the same places of its tile, so those
+// are worked out once a block (their index arithmetic, some forty instructions
+// a copy in every chunk, took more issue slots than all else together).
+template <int N, int CC, int T, bool RELU, bool OUT_F32, bool UP>
+__global__ void __launch_bounds__(fwd_threads(N), fwd_threads(N) == 256 ? 2 : 3) k_conv_fwd(const bf16* __restrict__ X, const bf16* __restrict__ Wt,
                                                   const float* __restrict__ bias, void* __restrict__ Y, Geo g,
-                                                  uint32_t* status) {
+                                                  ConvMore more, uint32_t* status) {
     using C = Conv<N, CC, T>;
-    constexpr int STAGES = C::STAGES;
+    constexpr int STAGES = C::STAGES, THREADS = fwd_threads(N);
+    static_assert(C::KG == 2, "two 8-channel groups a chunk");
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t bar[STAGES];
     __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float s_bias[N];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) tc::tmem_alloc(&tmem_base, C::COLS);
     if (tid == 0) {
         for (int i = 0; i < STAGES; i++) tc::mbar_init(&bar[i], 1);
         fence_barrier_init();
     }
+    for (int k = tid; k < N; k += THREADS) s_bias[k] = __ldg(bias + k);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -223,23 +319,50 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const bf16* __restrict__ X, co
     const int y0 = by * TY, x0 = bx * TX * T;
     const int nk = g.cin / CC;
 
+    // this thread's patch vectors: pixel q = tid / 2 + STEP j of the patch, 8-channel
+    // group tid & 1; -1 outside the image. Their places in shared memory are
+    // affine: a patch row is PXT pixels of 16 bytes.
+    constexpr int STEP = THREADS / 2;
+    constexpr int NV = (PY * C::PXT + STEP - 1) / STEP;
+    int pix[NV], half[UP ? NV : 1];
+#pragma unroll
+    for (int j = 0; j < NV; j++) {
+        const int q = (tid >> 1) + STEP * j;
+        const int py = q / C::PXT, px = q - py * C::PXT;
+        const int y = y0 + py - 1, x = x0 + px - 1;
+        const bool ok = y >= 0 && y < g.H && x >= 0 && x < g.W;
+        pix[j] = ok ? (img * g.H + y) * g.W + x : -1;
+        if (UP) half[j] = (img * (g.H / 2) + (y >> 1)) * (g.W / 2) + (x >> 1);
+    }
+    const uint32_t a_at = tc::smem_addr(smem) + (uint32_t)((tid & 1) * C::LBO_A + (tid >> 1) * 16);
     auto issue = [&](int chunk) {
-        uint8_t* patch = smem + (chunk % STAGES) * C::STAGE;
-        uint8_t* wb = patch + C::PATCH;
-        const int c0 = chunk * CC;
-        for (int v = tid; v < PY * C::PXT * C::KG; v += 128) {
-            const int kg = v % C::KG, q = v / C::KG;
-            const int py = q / C::PXT, px = q - py * C::PXT;
-            const int y = y0 + py - 1, x = x0 + px - 1;
-            const bool ok = y >= 0 && y < g.H && x >= 0 && x < g.W;
-            const bf16* src = ok ? X + ((size_t)(img * g.H + y) * g.W + x) * g.xs + g.xo + c0 + kg * 8 : X;
-            cp_async_ca16(patch + kg * C::LBO_A + py * C::ROWT + px * 16, src, ok ? 16u : 0u);
+        const uint32_t stage = (uint32_t)((chunk % STAGES) * C::STAGE);
+        const int c0 = chunk * CC + (tid & 1) * 8;
+        const bool below = UP && chunk * CC < more.up;
+        const bf16* src = below ? more.below + c0 : X + g.xo + (c0 - (UP ? more.up : 0));
+        const size_t pitch = below ? (size_t)more.up : (size_t)g.xs;
+#pragma unroll
+        for (int j = 0; j < NV; j++) {
+            if ((tid >> 1) + STEP * j >= PY * C::PXT) break;
+            const int at = (UP && below) ? half[UP ? j : 0] : pix[j];
+            const bool ok = pix[j] >= 0;
+            cp_async_ca16_at(a_at + stage + (uint32_t)(j * STEP * 16), ok ? src + (size_t)at * pitch : X, ok ? 16u : 0u);
         }
-        for (int v = tid; v < 9 * N * C::KG; v += 128) {
-            const int kg = v % C::KG, q = v / C::KG;
-            const int r = q % N, tap = q / N;
-            cp_async_cg16(wb + tap * C::BTAP + tc::tile_off(r, kg * 8, N),
-                          Wt + (size_t)r * g.Kp + tap * g.cin + c0 + kg * 8);
+        // the weights: row r and 8-channel group of all nine taps a thread
+        const uint32_t wb = tc::smem_addr(smem) + stage + (uint32_t)C::PATCH;
+        constexpr int SPLIT = THREADS / (N * 2) > 0 ? THREADS / (N * 2) : 1;  // threads that share a row's taps
+        constexpr int ROWS = SPLIT > 1 ? N * 2 : THREADS;
+#pragma unroll
+        for (int i = 0; i < (N * 2 + ROWS - 1) / ROWS; i++) {
+            const int k = tid % ROWS + ROWS * i;
+            if (k >= N * 2 || (SPLIT > 1 && tid / ROWS >= SPLIT)) break;
+            const int r = k >> 1, kg = k & 1;
+            const bf16* w = Wt + (size_t)r * g.Kp + chunk * CC + kg * 8;
+            const uint32_t to = wb + tc::tile_off(r, kg * 8, N);
+#pragma unroll
+            for (int tap = 0; tap < 9; tap++)
+                if (SPLIT == 1 || tap % SPLIT == tid / ROWS)
+                    cp_async_cg16_at(to + (uint32_t)(tap * C::BTAP), w + tap * g.cin);
         }
     };
 
@@ -287,34 +410,18 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const bf16* __restrict__ X, co
     ok = __syncthreads_and(ok);
     tc::fence_after_sync();
     if (ok) {
-        const int m = warp * 32 + lane;
+        // a warp reads the 32 TMEM lanes of its place among four; the groups
+        // of four warps take the tiles' runs of 16 channels in turn
+        const int m = (warp & 3) * 32 + lane;
 #pragma unroll 1
-        for (int t = 0; t < T; t++) {
+        for (int u = warp >> 2; u < T * (N / 16); u += THREADS / 128) {
+            const int t = u / (N / 16), c0 = (u - t * (N / 16)) * 16;
             const int y = y0 + m / TX, x = x0 + TX * t + m % TX;
             const bool live = y < g.H && x < g.W;
             const size_t p = ((size_t)img * g.H + y) * g.W + x;
-#pragma unroll 1
-            for (int c0 = 0; c0 < N; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)t * C::ACC + (uint32_t)c0, v);
-                if (!live) continue;
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    v[j] += __ldg(bias + c0 + j);
-                    if (RELU) v[j] = fmaxf(v[j], 0.0f);
-                }
-                if (OUT_F32) {
-                    float4* o = (float4*)((float*)Y + p * g.ys + g.yo + c0);
-#pragma unroll
-                    for (int q = 0; q < 4; q++) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                } else {
-                    uint4* o = (uint4*)((bf16*)Y + p * g.ys + g.yo + c0);
-                    o[0] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
-                                      pack_bf16x2(v[6], v[7]));
-                    o[1] = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
-                                      pack_bf16x2(v[14], v[15]));
-                }
-            }
+            float v[16];
+            tc::tmem_ld16(tm + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)t * C::ACC + (uint32_t)c0, v);
+            conv_store16<RELU, OUT_F32>(v, s_bias, Y, p, g, c0, live, more.pool, img, y, x);
         }
     } else if (tid == 0) {
         atomicOr(status, STATUS_SPIN_LIMIT);
@@ -328,7 +435,7 @@ __global__ void __launch_bounds__(128) k_conv_fwd(const bf16* __restrict__ X, co
 //
 // Used when the layer's weights (9 taps x N x cin bf16) and two input
 // patches fit in shared memory. Each CTA loads the weights once and walks
-// the output tiles blockIdx.x, + gridDim.x, ...; the tensor memory holds two
+// its share of the output tiles; the tensor memory holds two
 // accumulators of N columns (at column 0 and at the power of two >= N). Iteration i: thread 0 issues tile i's MMAs
 // (9 taps x cin / 16, shifted descriptors over patch buffer i & 1) into
 // accumulator i & 1 and commits them to mbarrier i & 1; meanwhile every
@@ -355,8 +462,12 @@ struct KpnOut {
     int h, w;  // the valid corner of the padded H x W images
 };
 
-__device__ __forceinline__ void kpn_pixel(const float* lg, const KpnOut& k, int img, int y, int x, int Hp, int Wp,
-                                          size_t p) {
+// A tile's irradiance with a border of 2, clamped to the valid image, in
+// shared memory (the kernels of its 128 pixels read it 25 times a pixel).
+constexpr int KPN_Y = TY + 4, KPN_X = TX + 4;
+
+__device__ __forceinline__ void kpn_pixel(const float* lg, const KpnOut& k, const float (*tile)[3], int ty, int tx,
+                                          int y, int x, size_t p) {
     if (!(y < k.h && x < k.w)) {
         for (int c = 0; c < 3; c++) k.out[p * 3 + c] = 0.0f;
         k.err[p] = 0.0f;
@@ -378,11 +489,10 @@ __device__ __forceinline__ void kpn_pixel(const float* lg, const KpnOut& k, int 
     float sm[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int t = 0; t < 25; t++) {
-        const int yy = min(max(y + t / 5 - 2, 0), k.h - 1), xx = min(max(x + t % 5 - 2, 0), k.w - 1);
-        const float* q = k.irr + ((size_t)(img * Hp + yy) * Wp + xx) * 3;
+        const float* q = tile[(ty + t / 5) * KPN_X + tx + t % 5];
         const float wv = wt[t] * iz;
 #pragma unroll
-        for (int c = 0; c < 3; c++) sm[c] += wv * __ldg(q + c);
+        for (int c = 0; c < 3; c++) sm[c] += wv * q[c];
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) k.out[p * 3 + c] = __ldg(k.alb + p * 3 + c) * sm[c];
@@ -390,12 +500,14 @@ __device__ __forceinline__ void kpn_pixel(const float* lg, const KpnOut& k, int 
 }
 
 template <int N, bool RELU, bool OUT_F32, bool KPN = false>
-__global__ void __launch_bounds__(128) k_conv_ws(const bf16* __restrict__ X, const bf16* __restrict__ Wt,
+__global__ void __launch_bounds__(128, 4) k_conv_ws(const bf16* __restrict__ X, const bf16* __restrict__ Wt,
                                                  const float* __restrict__ bias, void* __restrict__ Y, Geo g,
-                                                 uint32_t* status, KpnOut kp = KpnOut{}) {
+                                                 ConvMore more, uint32_t* status, KpnOut kp = KpnOut{}) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t bar[2];
     __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float s_bias[N];
+    __shared__ float s_irr[KPN ? KPN_Y * KPN_X : 1][3];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // accumulator b at column b * ACC (a power of two: aligned like a whole allocation)
     constexpr uint32_t ACC = tc::tmem_cols(N);
@@ -406,6 +518,7 @@ __global__ void __launch_bounds__(128) k_conv_ws(const bf16* __restrict__ X, con
         tc::mbar_init(&bar[1], 1);
         fence_barrier_init();
     }
+    for (int k = tid; k < N; k += 128) s_bias[k] = (!KPN || k < 26) ? __ldg(bias + k) : 0.0f;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -426,58 +539,96 @@ __global__ void __launch_bounds__(128) k_conv_ws(const bf16* __restrict__ X, con
         cp_async_cg16(wsm + tap * BTAP + tc::tile_off(r, kg * 8, N), Wt + (size_t)r * g.Kp + tap * g.cin + kg * 8);
     }
     cp_async_commit();
-    auto issue_patch = [&](int tile, int buf) {
-        const int bx = tile % tiles_x, by = (tile / tiles_x) % tiles_y, img = tile / (tiles_x * tiles_y);
-        const int y0 = by * TY, x0 = bx * TX;
-        uint8_t* patch = patch0 + buf * PATCH;
-        for (int v = tid; v < PY * PX * KG; v += 128) {
-            const int kg = v % KG, q = v / KG;
-            const int py = q / PX, px = q - py * PX;
-            const int y = y0 + py - 1, x = x0 + px - 1;
-            const bool ok = y >= 0 && y < g.H && x >= 0 && x < g.W;
-            const bf16* src = ok ? X + ((size_t)(img * g.H + y) * g.W + x) * g.xs + g.xo + kg * 8 : X;
-            cp_async_ca16(patch + kg * LBO_A + py * ROWB + px * 16, src, ok ? 16u : 0u);
+    // This thread's vectors of every patch, worked out once: the patch pixel
+    // (row py, column px), its offset in the image's pixels from the patch's
+    // first, and its places in shared memory and among the channels.
+    constexpr int NV = 12;  // 18 x 10 pixels of 8 groups (64 channels) over 128 threads
+    int rel[NV], at[NV];    // rel: pixel offset; at: shared offset | py << 20 | px << 26
+    const int nv = PY * PX * KG;
+#pragma unroll
+    for (int j = 0; j < NV; j++) {
+        const int v = tid + 128 * j;
+        const int kg = v % KG, q = v / KG, py = q / PX, px = q - py * PX;
+        rel[j] = (py * g.W + px) * 8 + kg;  // the group beside it (at most 8 of them)
+        at[j] = (kg * LBO_A + q * 16) | py << 20 | px << 26;
+    }
+    // A block's tiles are consecutive, so that a tile's place is one step from
+    // the last one's (two divisions a tile and use cost a third of the loop: the
+    // 1080p layers of 32 channels 95 / 147 / 115 us so, 85 / 144 / 109 with
+    // steps). The kernel-prediction head, whose epilogue outweighs the loop,
+    // takes every gridDim.x-th tile: neighbouring blocks then read the same
+    // rows of irradiance and albedo at the same time (251 us against 260).
+    struct Place {
+        int bx, by, img, tile;
+    };
+    const int tile0 = KPN ? (int)blockIdx.x : (int)((long long)blockIdx.x * ntiles / gridDim.x);
+    const int mine = KPN ? (ntiles - tile0 + (int)gridDim.x - 1) / (int)gridDim.x
+                         : (int)((long long)(blockIdx.x + 1) * ntiles / gridDim.x) - tile0;
+    auto place = [&](int t) { return Place{t % tiles_x, (t / tiles_x) % tiles_y, t / (tiles_x * tiles_y), t}; };
+    auto step = [&](Place& q) {
+        if (KPN) {
+            q = place(q.tile + (int)gridDim.x);
+            return;
+        }
+        if (++q.bx < tiles_x) return;
+        q.bx = 0;
+        if (++q.by < tiles_y) return;
+        q.by = 0;
+        q.img++;
+    };
+    Place ahead = place(tile0);
+    Place done = ahead;  // of the next epilogue
+    auto issue_patch = [&](int buf) {
+        const int img = ahead.img, y0 = ahead.by * TY - 1, x0 = ahead.bx * TX - 1;
+        step(ahead);
+        const uint32_t patch = tc::smem_addr(patch0 + buf * PATCH);
+        const bool inside = y0 >= 0 && x0 >= 0 && y0 + PY <= g.H && x0 + PX <= g.W;
+        const bf16* base = X + g.xo + ((ptrdiff_t)(img * g.H + y0) * g.W + x0) * g.xs;
+#pragma unroll
+        for (int j = 0; j < NV; j++) {
+            if (128 * j >= nv) break;
+            if (tid + 128 * j >= nv) continue;
+            bool ok = true;
+            if (!inside) {
+                const int y = y0 + ((at[j] >> 20) & 31), x = x0 + (at[j] >> 26);
+                ok = y >= 0 && y < g.H && x >= 0 && x < g.W;
+            }
+            const bf16* src = ok ? base + (size_t)(rel[j] >> 3) * g.xs + (rel[j] & 7) * 8 : X;
+            cp_async_ca16_at(patch + (uint32_t)(at[j] & 0xFFFFF), src, ok ? 16u : 0u);
         }
         cp_async_commit();
     };
-    auto epilogue = [&](int tile, int buf) {
-        const int bx = tile % tiles_x, by = (tile / tiles_x) % tiles_y, img = tile / (tiles_x * tiles_y);
+    auto epilogue = [&](int buf) {
+        const int bx = done.bx, by = done.by, img = done.img;
+        step(done);
         const int m = warp * 32 + lane;
         const int y = by * TY + m / TX, x = bx * TX + m % TX;
         const bool live = y < g.H && x < g.W;
         const size_t p = ((size_t)img * g.H + y) * g.W + x;
-        if (KPN) {
+        if constexpr (KPN) {
+            __syncthreads();  // the last tile's irradiance is read
+            for (int k = tid; k < KPN_Y * KPN_X; k += 128) {
+                const int ly = k / KPN_X, lx = k - ly * KPN_X;
+                const int yy = min(max(by * TY + ly - 2, 0), kp.h - 1), xx = min(max(bx * TX + lx - 2, 0), kp.w - 1);
+                const float* q = kp.irr + ((size_t)(img * g.H + yy) * g.W + xx) * 3;
+#pragma unroll
+                for (int c = 0; c < 3; c++) s_irr[k][c] = __ldg(q + c);
+            }
+            __syncthreads();
             float lg[32];
             tc::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * ACC, lg);
             tc::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * ACC + 16u, lg + 16);
             if (live) {
 #pragma unroll
-                for (int j = 0; j < 26; j++) lg[j] += __ldg(bias + j);
-                kpn_pixel(lg, kp, img, y, x, g.H, g.W, p);
+                for (int j = 0; j < 26; j++) lg[j] += s_bias[j];
+                kpn_pixel(lg, kp, s_irr, m / TX, m % TX, y, x, p);
             }
-            tc::fence_before_sync();
-            return;
-        }
+        } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * ACC + (uint32_t)c0, v);
-            if (!live) continue;
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                v[j] += __ldg(bias + c0 + j);
-                if (RELU) v[j] = fmaxf(v[j], 0.0f);
-            }
-            if (OUT_F32) {
-                float4* o = (float4*)((float*)Y + p * g.ys + g.yo + c0);
-#pragma unroll
-                for (int q = 0; q < 4; q++) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            } else {
-                uint4* o = (uint4*)((bf16*)Y + p * g.ys + g.yo + c0);
-                o[0] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
-                                  pack_bf16x2(v[6], v[7]));
-                o[1] = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
-                                  pack_bf16x2(v[14], v[15]));
+            for (int c0 = 0; c0 < N; c0 += 16) {
+                float v[16];
+                tc::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * ACC + (uint32_t)c0, v);
+                conv_store16<RELU, OUT_F32>(v, s_bias, Y, p, g, c0, live, more.pool, img, y, x);
             }
         }
         tc::fence_before_sync();
@@ -487,15 +638,14 @@ __global__ void __launch_bounds__(128) k_conv_ws(const bf16* __restrict__ X, con
     constexpr uint32_t b_lbo = (N / 8) * 128;
     constexpr int NP = ConvWS<N>::PATCHES;
     bool ok = true;
-    int i = 0, prev = -1;
     // Prologue: tiles 0 and 1 of this block in flight (commit groups 1, 2 after
     // the weights' group 0; an empty group stands in for a missing tile).
     for (int k = 0; k < NP - 1; k++) {
-        const int t = blockIdx.x + k * gridDim.x;
-        if (t < ntiles) issue_patch(t, k);
+        if (k < mine) issue_patch(k);
         else cp_async_commit();
     }
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, i++) {
+    int i = 0;
+    for (; i < mine; i++) {
         const int b = i & 1;
         cp_async_wait<NP - 2>();  // this thread's copies of tile i (and the weights) landed
         tc::fence_async_smem();
@@ -523,19 +673,17 @@ __global__ void __launch_bounds__(128) k_conv_ws(const bf16* __restrict__ X, con
         }
         if (i >= 1) ok = tc::mbar_wait(&bar[b ^ 1], ((i - 1) >> 1) & 1) && ok;  // tile i - 1's MMAs done
         // tile i + 2 into the patch buffer tile i - 1 used
-        const int ahead = tile + (NP - 1) * gridDim.x;
-        if (ahead < ntiles) issue_patch(ahead, (i + NP - 1) % NP);
+        if (i + NP - 1 < mine) issue_patch((i + NP - 1) % NP);
         else cp_async_commit();
         if (i >= 1) {
             tc::fence_after_sync();
-            epilogue(prev, b ^ 1);
+            epilogue(b ^ 1);
         }
-        prev = tile;
     }
     if (i >= 1) {
         ok = tc::mbar_wait(&bar[(i - 1) & 1], ((i - 1) >> 1) & 1) && ok;
         tc::fence_after_sync();
-        epilogue(prev, (i - 1) & 1);
+        epilogue((i - 1) & 1);
     }
     ok = __syncthreads_and(ok);
     if (!ok && tid == 0) atomicOr(status, STATUS_SPIN_LIMIT);
@@ -1241,32 +1389,36 @@ __global__ void k_compose(const float* __restrict__ out, const float* __restrict
     px[i] = pack_rgba(shown, __uint_as_float(px[24 * n + i]) * k);
 }
 
-template <int N, int CC, int T, bool RELU, bool F32>
-int32_t conv_fwd_n(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g) {
+template <int N, int CC, int T, bool RELU, bool F32, bool UP>
+int32_t conv_fwd_n(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g, const ConvMore& more) {
     const int smem = Conv<N, CC, T>::TOTAL;
     static std::atomic<uint64_t> done{0};
-    PHX_TRY(smem_limit(k_conv_fwd<N, CC, T, RELU, F32>, smem, c->device, done));
+    PHX_TRY(smem_limit(k_conv_fwd<N, CC, T, RELU, F32, UP>, smem, c->device, done));
     const uint32_t blocks = (uint32_t)g.B * ((g.H + TY - 1) / TY) * ((g.W + TX * T - 1) / (TX * T));
-    k_conv_fwd<N, CC, T, RELU, F32><<<blocks, 128, smem, c->stream>>>(X, W, bias, Y, g, c->status);
+    k_conv_fwd<N, CC, T, RELU, F32, UP><<<blocks, fwd_threads(N), smem, c->stream>>>(X, W, bias, Y, g, more, c->status);
     return cuda_check(cudaGetLastError(), "conv fwd");
 }
 
 constexpr size_t WS_MAX_SMEM = 110 * 1024;
+constexpr int WS_MAX_CIN = 64;  // k_conv_ws's copies a thread
+
+// Blocks per SM of k_conv_ws: by shared memory (the SM's 228 KB less 1 KB per
+// block, this kernel's static data), by the 512 TMEM columns (two
+// accumulators a block) and by threads; its grid.
+int ws_grid(Ctx* c, const Geo& g, int smem, int fixed, uint32_t acc) {
+    const int by_smem = (228 * 1024) / (smem + 1024 + fixed);
+    const int per_sm = std::max(1, std::min(std::min(by_smem, (int)(512 / (2 * acc))), 16));
+    const int ntiles = g.B * ((g.H + TY - 1) / TY) * ((g.W + TX - 1) / TX);
+    return std::min(ntiles, per_sm * c->sms);
+}
 
 template <int N, bool RELU, bool F32>
-int32_t conv_ws_n(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g) {
+int32_t conv_ws_n(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g, const ConvMore& more) {
     const int smem = (int)ConvWS<N>::bytes(g.cin);
     static std::atomic<uint64_t> done{0};
     PHX_TRY(smem_limit(k_conv_ws<N, RELU, F32>, (int)WS_MAX_SMEM, c->device, done));
-    // Blocks per SM: by shared memory (the SM's 228 KB less 1 KB per block,
-    // this kernel's 1 KB of static data), by the 512 TMEM columns (two
-    // accumulators a block) and by threads.
-    const int by_smem = (228 * 1024) / (smem + 2 * 1024);
-    const int by_tmem = (int)(512 / (2 * tc::tmem_cols(N)));
-    const int per_sm = std::max(1, std::min(std::min(by_smem, by_tmem), 16));
-    const int ntiles = g.B * ((g.H + TY - 1) / TY) * ((g.W + TX - 1) / TX);
-    const int grid = std::min(ntiles, per_sm * c->sms);
-    k_conv_ws<N, RELU, F32><<<grid, 128, smem, c->stream>>>(X, W, bias, Y, g, c->status);
+    const int grid = ws_grid(c, g, smem, 1024, tc::tmem_cols(N));
+    k_conv_ws<N, RELU, F32><<<grid, 128, smem, c->stream>>>(X, W, bias, Y, g, more, c->status);
     return cuda_check(cudaGetLastError(), "conv fwd (weight-stationary)");
 }
 
@@ -1276,32 +1428,35 @@ int32_t conv_kpn(Ctx* c, const bf16* X, const bf16* W, const float* bias, const 
     if ((size_t)smem > WS_MAX_SMEM) return fail(PHX_ERR_INVALID, "conv+kpn: %d input channels do not fit", g.cin);
     static std::atomic<uint64_t> done{0};
     PHX_TRY(smem_limit(k_conv_ws<32, false, true, true>, (int)WS_MAX_SMEM, c->device, done));
-    const int by_smem = (228 * 1024) / (smem + 2 * 1024);
-    const int per_sm = std::max(1, std::min(std::min(by_smem, (int)(512 / (2 * tc::tmem_cols(32)))), 16));
-    const int ntiles = g.B * ((g.H + TY - 1) / TY) * ((g.W + TX - 1) / TX);
-    const int grid = std::min(ntiles, per_sm * c->sms);
-    k_conv_ws<32, false, true, true><<<grid, 128, smem, c->stream>>>(X, W, bias, nullptr, g, c->status, kp);
+    const int grid = ws_grid(c, g, smem, 4096, tc::tmem_cols(32));
+    k_conv_ws<32, false, true, true><<<grid, 128, smem, c->stream>>>(X, W, bias, nullptr, g, ConvMore{}, c->status, kp);
     return cuda_check(cudaGetLastError(), "conv + kpn");
 }
 
 // The weight-stationary form where two of its blocks fit an SM, else the
-// chunked form over 16 channels a chunk.
+// chunked form over 16 channels a chunk (always where the first channels come
+// from a half-size tensor).
 template <int N, bool RELU, bool F32>
-int32_t conv_fwd_cc(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g) {
-    if (N <= 128 && ConvWS<N>::bytes(g.cin) <= WS_MAX_SMEM) return conv_ws_n<N, RELU, F32>(c, X, W, bias, Y, g);
+int32_t conv_fwd_cc(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g, const ConvMore& more) {
     // chunked: several tiles a block where N is small (their weights read once)
     constexpr int T = N <= 32 ? 4 : (N <= 64 ? 2 : 1);
-    return conv_fwd_n<N, 16, T, RELU, F32>(c, X, W, bias, Y, g);
+    if constexpr (RELU && !F32 && N <= 128)
+        if (more.below) return conv_fwd_n<N, 16, T, RELU, F32, true>(c, X, W, bias, Y, g, more);
+    if (more.below) return fail(PHX_ERR_INVALID, "conv: no such form over a half-size input");
+    if (N <= 128 && g.cin <= WS_MAX_CIN && ConvWS<N>::bytes(g.cin) <= WS_MAX_SMEM)
+        return conv_ws_n<N, RELU, F32>(c, X, W, bias, Y, g, more);
+    return conv_fwd_n<N, 16, T, RELU, F32, false>(c, X, W, bias, Y, g, more);
 }
 
 template <bool RELU, bool F32>
-int32_t conv_fwd_any(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g) {
+int32_t conv_fwd_any(Ctx* c, const bf16* X, const bf16* W, const float* bias, void* Y, const Geo& g,
+                     const ConvMore& more = ConvMore{}) {
     switch (g.cout) {
-        case 32: return conv_fwd_cc<32, RELU, F32>(c, X, W, bias, Y, g);
-        case 64: return conv_fwd_cc<64, RELU, F32>(c, X, W, bias, Y, g);
-        case 96: return conv_fwd_cc<96, RELU, F32>(c, X, W, bias, Y, g);
-        case 128: return conv_fwd_cc<128, RELU, F32>(c, X, W, bias, Y, g);
-        case 160: return conv_fwd_cc<160, RELU, F32>(c, X, W, bias, Y, g);
+        case 32: return conv_fwd_cc<32, RELU, F32>(c, X, W, bias, Y, g, more);
+        case 64: return conv_fwd_cc<64, RELU, F32>(c, X, W, bias, Y, g, more);
+        case 96: return conv_fwd_cc<96, RELU, F32>(c, X, W, bias, Y, g, more);
+        case 128: return conv_fwd_cc<128, RELU, F32>(c, X, W, bias, Y, g, more);
+        case 160: return conv_fwd_cc<160, RELU, F32>(c, X, W, bias, Y, g, more);
     }
     return fail(PHX_ERR_INVALID, "conv: output tile of %d channels (32, 64, 96, 128 or 160)", g.cout);
 }
@@ -1342,6 +1497,16 @@ int32_t nn_adam_net(Ctx* c, AdamNet& net) {
     }
     k_adam_net<<<blocks, 256, 0, c->stream>>>(net);
     return cuda_check(cudaGetLastError(), "adam");
+}
+
+int32_t nn_conv_relu(Ctx* c, const void* X, int xs, int xo, int cin, const void* W, int Kp, const float* bias, void* Y,
+                     int ys, int yo, int cout, int B, int H, int Wd, const void* below, int up, void* pool) {
+    const Geo g{B, H, Wd, cin, xs, xo, cout, ys, yo, 9 * cin, Kp};
+    ConvMore more;
+    more.below = (const bf16*)below;
+    more.up = up;
+    more.pool = (bf16*)pool;
+    return conv_fwd_any<true, false>(c, (const bf16*)X, (const bf16*)W, bias, Y, g, more);
 }
 
 int32_t nn_conv_grads(Ctx* c, const void* X, int xs, int xo, int cin, const void* dY, int dys, int dyo, int cout,

@@ -177,14 +177,23 @@ int32_t relu_bwd(phx_unet_s* n, View y, View dy, int C, const Shape& s, int leve
 
 View v(DevMem& m, int pitch, int off = 0) { return View{m.ptr, pitch, off}; }
 
-// Every layer up to the head's input (Db[0]); with_head: the head too (fp32 logits).
+// Layer i with its ReLU, and beside it the pooling of its output, or its
+// first input channels taken from the level below (upsampled as read).
+int32_t layer_fwd_more(phx_unet_s* n, int i, View in, View out, const Shape& s, int level, const void* below, int up,
+                       void* pool) {
+    Conv& c = n->L[i];
+    return nn_conv_relu(n->ctx, in.p, in.pitch, in.off, c.cin, c.wb.ptr, c.Kp, (const float*)c.b32.ptr, out.p,
+                        out.pitch, out.off, c.cout, s.B, s.H >> level, s.W >> level, below, up, pool);
+}
+
+// Every layer up to the head's input (Db[0]); with_head: the head too (fp32
+// logits), as training does, whose backward pass reads the upsampled channels.
 int32_t forward(phx_unet_s* n, const void* feat, const Shape& s, bool with_head = true) {
     View x{(void*)feat, FEAT, 0};
     for (int l = 0; l < 4; l++) {
         PHX_TRY(layer_fwd(n, 2 * l, x, v(n->A[l], LEVEL_CH[l]), s, l));
-        PHX_TRY(layer_fwd(n, 2 * l + 1, v(n->A[l], LEVEL_CH[l]), v(n->cat[l], CAT_CH[l], UP_CH[l]), s, l));
-        PHX_TRY(phx_nn_pool_fwd(n->handle, n->cat[l].ptr, CAT_CH[l], UP_CH[l], LEVEL_CH[l], s.B, s.H >> l, s.W >> l,
-                                n->pool[l + 1].ptr));
+        PHX_TRY(layer_fwd_more(n, 2 * l + 1, v(n->A[l], LEVEL_CH[l]), v(n->cat[l], CAT_CH[l], UP_CH[l]), s, l, nullptr,
+                               0, n->pool[l + 1].ptr));
         x = v(n->pool[l + 1], LEVEL_CH[l]);
     }
     PHX_TRY(layer_fwd(n, 8, x, v(n->A[4], 160), s, 4));
@@ -192,9 +201,14 @@ int32_t forward(phx_unet_s* n, const void* feat, const Shape& s, bool with_head 
     View below = v(n->B4, 160);
     int below_ch = 160;
     for (int l = 3; l >= 0; l--) {
-        PHX_TRY(phx_nn_up_fwd(n->handle, below.p, below_ch, s.B, s.H >> l, s.W >> l, n->cat[l].ptr, CAT_CH[l], 0));
         const int d = 10 + 2 * (3 - l);
-        PHX_TRY(layer_fwd(n, d, v(n->cat[l], CAT_CH[l]), v(n->Da[l], LEVEL_CH[l]), s, l));
+        if (with_head) {
+            PHX_TRY(phx_nn_up_fwd(n->handle, below.p, below_ch, s.B, s.H >> l, s.W >> l, n->cat[l].ptr, CAT_CH[l], 0));
+            PHX_TRY(layer_fwd(n, d, v(n->cat[l], CAT_CH[l]), v(n->Da[l], LEVEL_CH[l]), s, l));
+        } else {
+            PHX_TRY(layer_fwd_more(n, d, v(n->cat[l], CAT_CH[l], UP_CH[l]), v(n->Da[l], LEVEL_CH[l]), s, l, below.p,
+                                   below_ch, nullptr));
+        }
         PHX_TRY(layer_fwd(n, d + 1, v(n->Da[l], LEVEL_CH[l]), v(n->Db[l], LEVEL_CH[l]), s, l));
         below = v(n->Db[l], LEVEL_CH[l]);
         below_ch = LEVEL_CH[l];
