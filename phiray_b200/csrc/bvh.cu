@@ -20,9 +20,10 @@
 //                   cand = (last - first < leaf) || depth + 1 >= STACK; cand
 //                   holds for every descendant of a cand node, so that rule
 //                   reproduces the DFS exactly. Depth = climb of parents.
-//   k_refit         Bvh::refit (build.rs:180-194) as one atomic bottom-up
-//                   pass: reachable leaves compute their box, the second
-//                   child to arrive at a parent computes the parent's.
+//   k_refit         Bvh::refit (build.rs:180-194) bottom up: subtrees that
+//                   lie in a block's sorted slots in shared memory, what is
+//                   above them by atomic arrivals, the second child to arrive
+//                   at a parent computing the parent's box.
 //
 // min/max add no rounding, so codes, order, links, depth and bounds match
 // the CPU builder exactly.
@@ -403,7 +404,8 @@ __global__ void __launch_bounds__(256) k_pack(const uint4* __restrict__ links, c
                                               const uint32_t* __restrict__ anc, const uint32_t* __restrict__ dist,
                                               uint32_t n, uint32_t leaf, float4* __restrict__ nodes,
                                               uint32_t* __restrict__ starts, uint32_t* __restrict__ nstarts,
-                                              uint32_t* __restrict__ depth_out, Gate gate) {
+                                              uint32_t* __restrict__ owner, uint32_t* __restrict__ depth_out,
+                                              Gate gate) {
     if (gate.off()) return;
     const uint32_t total = 2 * n - 1;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -449,6 +451,8 @@ __global__ void __launch_bounds__(256) k_pack(const uint4* __restrict__ links, c
                 start = true;
             }
         }
+        if (start)  // the leaves share the slots out, each slot one leaf's
+            for (uint32_t k = lo_i & ~LEAF; k < hi_i; k++) owner[k] = k == (lo_i & ~LEAF) ? i : NO_OWNER;
         nodes[2 * (size_t)i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(lo_i));
         nodes[2 * (size_t)i + 1] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(hi_i));
     }
@@ -478,36 +482,32 @@ __global__ void __launch_bounds__(256) k_pack(const uint4* __restrict__ links, c
     if (start) starts[s_base + s_cnt[warp] + __popc(m & ((1u << lane) - 1u))] = i;
 }
 
-// ---- refit: atomic bottom-up (Bvh::refit's bounds, Warp's refit pattern) ----
+// ---- refit: bottom-up by blocks of slots (Bvh::refit's bounds) ----
 
 // `order` NULL: boxes are given by sorted slot (Bvh::refit_slots,
 // build.rs:172-177). counters[] start even; each reachable inner node gets
-// exactly two arrivals per refit, so no reset is needed between refits.
-__global__ void __launch_bounds__(256) k_refit(const float4* __restrict__ prims, const uint32_t* __restrict__ order,
-                                               const uint32_t* __restrict__ parent, float4* nodes,
-                                               const uint32_t* __restrict__ starts,
-                                               const uint32_t* __restrict__ nstarts, uint32_t* counters,
-                                               uint32_t* status, Gate gate) {
+// two arrivals a refit or (made inside a block) none, so no reset is needed
+// between refits.
+__global__ void __launch_bounds__(REFIT_SLOTS) k_refit(const float4* __restrict__ prims,
+                                                       const uint32_t* __restrict__ order, uint32_t n,
+                                                       const uint32_t* __restrict__ parent, float4* nodes,
+                                                       const uint32_t* __restrict__ owner, uint32_t* counters,
+                                                       uint32_t* status, uint32_t* list, Gate gate) {
     if (gate.off()) return;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= *nstarts) return;
-    uint32_t i = starts[t];
-    const float4 a = nodes[2 * (size_t)i], b = nodes[2 * (size_t)i + 1];
-    const uint32_t first = __float_as_uint(a.w) & ~LEAF, end = __float_as_uint(b.w);
-    float lx = FLT_MAX, ly = FLT_MAX, lz = FLT_MAX, hx = -FLT_MAX, hy = -FLT_MAX, hz = -FLT_MAX;
-    for (uint32_t s = first; s < end; s++) {
+    refit_block(n, owner, parent, nodes, counters, status, list, [&](uint32_t s, bool, bool) {
         const uint32_t p = order ? __ldg(order + s) : s;
-        const float4 pa = __ldg(prims + 2 * (size_t)p), pb = __ldg(prims + 2 * (size_t)p + 1);
-        lx = fminf(lx, pa.x);
-        ly = fminf(ly, pa.y);
-        lz = fminf(lz, pa.z);
-        hx = fmaxf(hx, pb.x);
-        hy = fmaxf(hy, pb.y);
-        hz = fmaxf(hz, pb.z);
-    }
-    nodes[2 * (size_t)i] = make_float4(lx, ly, lz, a.w);
-    nodes[2 * (size_t)i + 1] = make_float4(hx, hy, hz, b.w);
-    refit_climb(i, lx, ly, lz, hx, hy, hz, parent, nodes, counters, status);
+        const float4 a = __ldg(prims + 2 * (size_t)p), b = __ldg(prims + 2 * (size_t)p + 1);
+        return RefitBox{a.x, a.y, a.z, b.x, b.y, b.z};
+    });
+}
+
+__global__ void __launch_bounds__(256) k_refit_climbs(const uint32_t* __restrict__ list, uint32_t count,
+                                                      const uint32_t* __restrict__ parent, float4* nodes,
+                                                      uint32_t* counters, uint32_t* status, Gate gate) {
+    if (gate.off()) return;
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t id = k < count ? __ldg(list + k) : NO_OWNER;
+    if (id != NO_OWNER) refit_climb_from(id, parent, nodes, counters, status);
 }
 
 // The reference's Jacobi Refit step (kernel.rs:130-170), for Pass replay.
@@ -673,20 +673,25 @@ int32_t enqueue_build(Ctx* c, BvhWork& w, uint32_t n, uint32_t leaf, Gate gate, 
     k_pack<<<grid_for(2ull * n - 1, 256, 1u << 30), 256, 0, s>>>((const uint4*)w.links.ptr,
                                                                 (const uint32_t*)w.parent.ptr, anc_a, dist_a, n, leaf,
                                                                 (float4*)w.nodes.ptr, (uint32_t*)w.starts.ptr,
-                                                                w.nstarts(), w.depth(), gate);
+                                                                w.nstarts(), w.owner(), w.depth(), gate);
     if (!refit) return cuda_check(cudaGetLastError(), "bvh build");
-    k_refit<<<grid_for(n, 256, 1u << 30), 256, 0, s>>>(prims, (const uint32_t*)w.order.ptr,
-                                                       (const uint32_t*)w.parent.ptr, (float4*)w.nodes.ptr,
-                                                       (const uint32_t*)w.starts.ptr, w.nstarts(),
-                                                       (uint32_t*)w.counters.ptr, c->status, gate);
-    return cuda_check(cudaGetLastError(), "bvh build");
+    return enqueue_refit(c, w, n, false, gate);
 }
 
 int32_t enqueue_refit(Ctx* c, BvhWork& w, uint32_t n, bool slots, Gate gate) {
     if (n == 0) return PHX_OK;
-    k_refit<<<grid_for(n, 256, 1u << 30), 256, 0, c->stream>>>(
-        (const float4*)w.prims.ptr, slots ? nullptr : (const uint32_t*)w.order.ptr, (const uint32_t*)w.parent.ptr,
-        (float4*)w.nodes.ptr, (const uint32_t*)w.starts.ptr, w.nstarts(), (uint32_t*)w.counters.ptr, c->status, gate);
+    k_refit<<<grid_for(n, REFIT_SLOTS, 1u << 30), REFIT_SLOTS, 0, c->stream>>>(
+        (const float4*)w.prims.ptr, slots ? nullptr : (const uint32_t*)w.order.ptr, n, (const uint32_t*)w.parent.ptr,
+        (float4*)w.nodes.ptr, w.owner(), (uint32_t*)w.counters.ptr, c->status, w.climbs(n), gate);
+    PHX_CUDA(cudaGetLastError());
+    return enqueue_climbs(c, w, n, gate);
+}
+
+int32_t enqueue_climbs(Ctx* c, BvhWork& w, uint32_t n, Gate gate) {
+    if (!w.climbs(n)) return PHX_OK;
+    const uint32_t count = grid_for(n, REFIT_SLOTS, 1u << 30) * REFIT_OPEN;
+    k_refit_climbs<<<grid_for(count, 256, 1u << 30), 256, 0, c->stream>>>(
+        w.climbs(n), count, (const uint32_t*)w.parent.ptr, (float4*)w.nodes.ptr, (uint32_t*)w.counters.ptr, c->status, gate);
     return cuda_check(cudaGetLastError(), "bvh refit");
 }
 

@@ -92,45 +92,35 @@ __global__ void k_mark_ends(const float4* __restrict__ nodes, const uint32_t* __
     c->w = __uint_as_float(__float_as_uint(c->w) | FLAG_END);
 }
 
-// The refit (k_refit's leaf part and climb) fused with the triangle gather
-// for a single-mesh LBVH tree: the thread of each reachable leaf computes
-// its faces' boxes from the vertices (Aabb::of_tri, as k_face_boxes), writes
-// their slots' triangle records (as k_gather) with the last slot marked (as
-// k_mark_ends), stores the leaf's box and climbs. The nodes, triangles and
-// flags are those of the separate kernels; the vertices are read once.
-__global__ void __launch_bounds__(256) k_refit_gather(const uint32_t* __restrict__ order,
-                                                      const uint4* __restrict__ faces,
-                                                      const float4* __restrict__ verts,
-                                                      const float4* __restrict__ vnorm,
-                                                      const float4* __restrict__ mats, uint32_t nmats,
-                                                      float4* __restrict__ tris, float4* __restrict__ tnorm,
-                                                      const uint32_t* __restrict__ parent, float4* nodes,
-                                                      const uint32_t* __restrict__ starts,
-                                                      const uint32_t* __restrict__ nstarts, uint32_t* counters,
-                                                      uint32_t* status) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= *nstarts) return;
-    const uint32_t i = starts[t];
-    const float4 na = nodes[2 * (size_t)i], nb = nodes[2 * (size_t)i + 1];
-    const uint32_t first = __float_as_uint(na.w) & ~LEAF, end = __float_as_uint(nb.w);
-    float lx = FLT_MAX, ly = FLT_MAX, lz = FLT_MAX, hx = -FLT_MAX, hy = -FLT_MAX, hz = -FLT_MAX;
-    for (uint32_t s = first; s < end; s++) {
+// The refit fused with the triangle gather for a single-mesh LBVH tree: each
+// slot's thread computes its face's box from the vertices (Aabb::of_tri, as
+// k_face_boxes) and writes the slot's triangle record (as k_gather), the last
+// slot of a leaf marked (as k_mark_ends); the boxes rise as in k_refit. The
+// nodes, triangles and flags are those of the separate kernels; the vertices
+// are read once.
+__global__ void __launch_bounds__(REFIT_SLOTS) k_refit_gather(const uint32_t* __restrict__ order, uint32_t n,
+                                                              const uint4* __restrict__ faces,
+                                                              const float4* __restrict__ verts,
+                                                              const float4* __restrict__ vnorm,
+                                                              const float4* __restrict__ mats, uint32_t nmats,
+                                                              float4* __restrict__ tris, float4* __restrict__ tnorm,
+                                                              const uint32_t* __restrict__ parent, float4* nodes,
+                                                              const uint32_t* __restrict__ owner, uint32_t* counters,
+                                                              uint32_t* status, uint32_t* list) {
+    refit_block(n, owner, parent, nodes, counters, status, list, [&](uint32_t s, bool last, bool write) {
         const uint32_t f = __ldg(order + s);
         const uint4 v = __ldg(faces + f);
         const float4 a = __ldg(verts + v.x), b = __ldg(verts + v.y), c = __ldg(verts + v.z);
-        lx = fminf(lx, fminf(fminf(a.x, b.x), c.x));
-        ly = fminf(ly, fminf(fminf(a.y, b.y), c.y));
-        lz = fminf(lz, fminf(fminf(a.z, b.z), c.z));
-        hx = fmaxf(hx, fmaxf(fmaxf(a.x, b.x), c.x));
-        hy = fmaxf(hy, fmaxf(fmaxf(a.y, b.y), c.y));
-        hz = fmaxf(hz, fmaxf(fmaxf(a.z, b.z), c.z));
+        const RefitBox box{fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z),
+                           fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z)};
+        if (!write) return box;
         uint32_t m = v.w;
         if (m >= nmats) {
             atomicOr(status, STATUS_BAD_INDEX);
             m = 0;
         }
         const float4 m0 = __ldg(mats + 8 * (size_t)m), m1 = __ldg(mats + 8 * (size_t)m + 1);
-        const uint32_t flags = ((m1.z > 0.5f || m0.w < 0.5f) ? FLAG_PASS : 0u) | (s + 1 == end ? FLAG_END : 0u);
+        const uint32_t flags = ((m1.z > 0.5f || m0.w < 0.5f) ? FLAG_PASS : 0u) | (last ? FLAG_END : 0u);
         tris[3 * (size_t)s] = make_float4(a.x, a.y, a.z, __uint_as_float(f));
         tris[3 * (size_t)s + 1] = make_float4(b.x, b.y, b.z, __uint_as_float(m));
         tris[3 * (size_t)s + 2] = make_float4(c.x, c.y, c.z, __uint_as_float(flags));
@@ -139,10 +129,8 @@ __global__ void __launch_bounds__(256) k_refit_gather(const uint32_t* __restrict
             tnorm[3 * (size_t)s + 1] = __ldg(vnorm + v.y);
             tnorm[3 * (size_t)s + 2] = __ldg(vnorm + v.z);
         }
-    }
-    nodes[2 * (size_t)i] = make_float4(lx, ly, lz, na.w);
-    nodes[2 * (size_t)i + 1] = make_float4(hx, hy, hz, nb.w);
-    refit_climb(i, lx, ly, lz, hx, hy, hz, parent, nodes, counters, status);
+        return box;
+    });
 }
 
 // Marks the last slot of every leaf of a tree whose nodes are all reachable
@@ -784,12 +772,14 @@ int32_t refit_gather(phx_tracer tr) {
     const uint32_t n = tr->nfaces;
     BvhWork& w = tr->bvh;
     if (n > 0) {
-        k_refit_gather<<<(n + 255) / 256, 256, 0, c->stream>>>(
-            (const uint32_t*)w.order.ptr, (const uint4*)tr->faces.ptr, (const float4*)tr->verts.ptr,
+        k_refit_gather<<<(n + REFIT_SLOTS - 1) / REFIT_SLOTS, REFIT_SLOTS, 0, c->stream>>>(
+            (const uint32_t*)w.order.ptr, n, (const uint4*)tr->faces.ptr, (const float4*)tr->verts.ptr,
             tr->has_normals ? (const float4*)tr->vnorm.ptr : nullptr, (const float4*)tr->mats.ptr, tr->nmats,
             (float4*)tr->tris.ptr, tr->has_normals ? (float4*)tr->tnorm.ptr : nullptr, (const uint32_t*)w.parent.ptr,
-            (float4*)w.nodes.ptr, (const uint32_t*)w.starts.ptr, w.nstarts(), (uint32_t*)w.counters.ptr, c->status);
+            (float4*)w.nodes.ptr, w.owner(), (uint32_t*)w.counters.ptr, c->status,
+            w.climbs(n));
         PHX_CUDA(cudaGetLastError());
+        PHX_TRY(enqueue_climbs(c, w, n));
     }
     return prepare_nodes(tr);
 }
