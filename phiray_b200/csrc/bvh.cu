@@ -24,6 +24,7 @@
 //                   lie in a block's sorted slots in shared memory, what is
 //                   above them by atomic arrivals, the second child to arrive
 //                   at a parent computing the parent's box.
+//   k_build_small   all of these for a small tree in one block.
 //
 // min/max add no rounding, so codes, order, links, depth and bounds match
 // the CPU builder exactly.
@@ -63,6 +64,22 @@ __device__ __forceinline__ uint32_t spread(float v) {
 __device__ __forceinline__ uint32_t morton3(float ux, float uy, float uz) {
     return (spread(ux) << 2) | (spread(uy) << 1) | spread(uz);
 }
+
+// Boxes to codes in a scene box s[0..6) (low, high corner).
+struct Quant {
+    float lo[3], inv[3];
+    __device__ __forceinline__ explicit Quant(const float* s) {
+        for (int k = 0; k < 3; k++) {
+            const float e = s[3 + k] - s[k];
+            lo[k] = s[k];
+            inv[k] = e > 0.0f ? 1.0f / e : 0.0f;
+        }
+    }
+    __device__ __forceinline__ uint32_t code(const float4& a, const float4& b) const {
+        const float cx = 0.5f * (a.x + b.x), cy = 0.5f * (a.y + b.y), cz = 0.5f * (a.z + b.z);
+        return morton3((cx - lo[0]) * inv[0], (cy - lo[1]) * inv[1], (cz - lo[2]) * inv[2]);
+    }
+};
 
 // ---- scene box ----
 
@@ -139,19 +156,14 @@ __global__ void __launch_bounds__(256) k_morton_hist(const float4* __restrict__ 
     }
     for (int k = threadIdx.x; k < PASSES * 256; k += blockDim.x) s_hist[k] = 0;
     block_minmax(v, s);
-    const float lo0 = s[0], lo1 = s[1], lo2 = s[2];
-    const float e0 = s[3] - s[0], e1 = s[4] - s[1], e2 = s[5] - s[2];
-    const float inv0 = e0 > 0.0f ? 1.0f / e0 : 0.0f;
-    const float inv1 = e1 > 0.0f ? 1.0f / e1 : 0.0f;
-    const float inv2 = e2 > 0.0f ? 1.0f / e2 : 0.0f;
+    const Quant quant(s);
     if (blockIdx.x == 0 && threadIdx.x == 0 && scene_out) {
         scene_out[0] = make_float4(s[0], s[1], s[2], 0.0f);
         scene_out[1] = make_float4(s[3], s[4], s[5], 0.0f);
     }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 a = __ldg(prims + 2 * (size_t)i), b = __ldg(prims + 2 * (size_t)i + 1);
-        const float cx = 0.5f * (a.x + b.x), cy = 0.5f * (a.y + b.y), cz = 0.5f * (a.z + b.z);
-        const uint32_t c = morton3((cx - lo0) * inv0, (cy - lo1) * inv1, (cz - lo2) * inv2);
+        const uint32_t c = quant.code(a, b);
         codes[i] = c;
         atomicAdd(&s_hist[0 * 256 + (c & 255)], 1u);
         atomicAdd(&s_hist[1 * 256 + ((c >> 8) & 255)], 1u);
@@ -321,36 +333,39 @@ __global__ void __launch_bounds__(RADIX_THREADS) k_radix_pass(const uint32_t* __
 
 // ---- Karras (build.rs:28-60, kernel.rs:65-117) ----
 
-__device__ __forceinline__ int kdelta(const uint32_t* __restrict__ codes, long long n, long long i, long long j) {
+// I: a signed index type that holds 2 n; code(i): the i-th sorted code.
+template <class I, class Code>
+__device__ __forceinline__ int kdelta(const Code& code, I n, I i, I j) {
     if (j < 0 || j >= n) return -1;
-    const uint32_t a = __ldg(codes + i), b = __ldg(codes + j);
+    const uint32_t a = code(i), b = code(j);
     if (a != b) return __clz(a ^ b);
     return 32 + __clz((uint32_t)i ^ (uint32_t)j);
 }
 
-__device__ __forceinline__ uint4 karras_link(const uint32_t* __restrict__ codes, long long n, long long i) {
-    const long long d = (kdelta(codes, n, i, i + 1) - kdelta(codes, n, i, i - 1) > 0) ? 1 : -1;
-    const int dmin = kdelta(codes, n, i, i - d);
-    long long lmax = 2;
-    while (kdelta(codes, n, i, i + lmax * d) > dmin) lmax *= 2;
-    long long l = 0, t = lmax / 2;
+template <class I, class Code>
+__device__ __forceinline__ uint4 karras_link(const Code& code, I n, I i) {
+    const I d = (kdelta<I>(code, n, i, i + 1) - kdelta<I>(code, n, i, i - 1) > 0) ? 1 : -1;
+    const int dmin = kdelta<I>(code, n, i, i - d);
+    I lmax = 2;
+    while (kdelta<I>(code, n, i, i + lmax * d) > dmin) lmax *= 2;
+    I l = 0, t = lmax / 2;
     while (t >= 1) {
-        if (kdelta(codes, n, i, i + (l + t) * d) > dmin) l += t;
+        if (kdelta<I>(code, n, i, i + (l + t) * d) > dmin) l += t;
         t /= 2;
     }
-    const long long j = i + l * d;
-    const int dnode = kdelta(codes, n, i, j);
-    long long s = 0;
+    const I j = i + l * d;
+    const int dnode = kdelta<I>(code, n, i, j);
+    I s = 0;
     t = l;
     for (;;) {
         t = (t + 1) >> 1;
-        if (kdelta(codes, n, i, i + (s + t) * d) > dnode) s += t;
+        if (kdelta<I>(code, n, i, i + (s + t) * d) > dnode) s += t;
         if (t <= 1) break;
     }
-    const long long g = i + s * d + (d < 0 ? d : 0);
-    const long long first = i < j ? i : j, last = i < j ? j : i;
-    const long long left = (first == g) ? n - 1 + g : g;
-    const long long right = (last == g + 1) ? n + g : g + 1;
+    const I g = i + s * d + (d < 0 ? d : 0);
+    const I first = i < j ? i : j, last = i < j ? j : i;
+    const I left = (first == g) ? n - 1 + g : g;
+    const I right = (last == g + 1) ? n + g : g + 1;
     return make_uint4((uint32_t)left, (uint32_t)right, (uint32_t)first, (uint32_t)last);
 }
 
@@ -360,7 +375,7 @@ __global__ void __launch_bounds__(256) k_karras(const uint32_t* __restrict__ cod
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0 && parent) parent[0] = NONE;
     if (i + 1 >= n) return;
-    const uint4 L = karras_link(codes, n, i);
+    const uint4 L = karras_link<long long>([&](long long k) { return __ldg(codes + k); }, n, i);
     links[i] = L;
     if (parent) {
         parent[L.x] = i;
@@ -510,6 +525,236 @@ __global__ void __launch_bounds__(256) k_refit_climbs(const uint32_t* __restrict
     if (id != NO_OWNER) refit_climb_from(id, parent, nodes, counters, status);
 }
 
+// ---- the whole build of a small tree in one block ----
+
+// Up to SMALL_MAX boxes are built by one block: the codes and the order sorted
+// in shared memory, the tree's parents and depths kept there, the boxes raised
+// by arrivals counted there. As launches of their own the stages are bound by
+// their number and their latencies (eighteen launches, 80 us of them on the
+// device at 1,000 boxes); the one block is bound by the latency of its steps.
+// A build and the wait for it, launches against one block: 64 boxes 104 and 46
+// us, 1,000 120 and 56, 2,000 134 and 67, 4,096 134 and 93. Past that its
+// 16-bit indices and its share of the chip (one SM) end.
+constexpr uint32_t SMALL_MAX = 4096;
+constexpr int SMALL_THREADS = 1024, SMALL_WARPS = SMALL_THREADS / 32, SMALL_ITEMS = SMALL_MAX / SMALL_THREADS;
+
+struct SmallTree {
+    uint32_t key[2][SMALL_MAX];  // a radix pass reads one half and writes the other
+    uint16_t val[2][SMALL_MAX];
+    union {
+        uint32_t digit[SMALL_WARPS][256];  // a pass's counts, then offsets
+        uint32_t arrived[SMALL_MAX];       // at an inner node, in the refit
+    };
+    uint16_t parent[2 * SMALL_MAX];
+    uint16_t width[SMALL_MAX];  // last - first slot of an inner node
+    uint8_t depth[SMALL_MAX];   // of an inner node, at most STACK
+    float part[SMALL_WARPS][6], scene[6];
+    uint32_t digit_base[256], scan[8];
+    uint32_t nstarts, max_depth;
+};
+
+struct SmallOut {
+    float4* scene;
+    uint32_t *sorted, *order, *parent, *starts, *owner, *counters, *scalars;
+    uint4* links;
+    float4* nodes;
+};
+
+__global__ void __launch_bounds__(SMALL_THREADS) k_build_small(const float4* __restrict__ prims, uint32_t n,
+                                                               uint32_t leaf, SmallOut out, bool refit, Gate gate) {
+    if (gate.off()) return;
+    extern __shared__ __align__(16) uint8_t smem[];
+    SmallTree& S = *(SmallTree*)smem;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t ninner = n - 1, total = 2 * n - 1;
+
+    // the scene box
+    float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (uint32_t i = tid; i < n; i += SMALL_THREADS) {
+        const float4 a = __ldg(prims + 2 * i), b = __ldg(prims + 2 * i + 1);
+        v[0] = fminf(v[0], a.x);
+        v[1] = fminf(v[1], a.y);
+        v[2] = fminf(v[2], a.z);
+        v[3] = fmaxf(v[3], b.x);
+        v[4] = fmaxf(v[4], b.y);
+        v[5] = fmaxf(v[5], b.z);
+    }
+    warp_minmax(v);
+    if (lane == 0)
+        for (int k = 0; k < 6; k++) S.part[warp][k] = v[k];
+    if (tid == 0) S.nstarts = S.max_depth = 0;
+    __syncthreads();
+    if (warp == 0) {
+        for (int k = 0; k < 6; k++) v[k] = S.part[lane][k];
+        warp_minmax(v);
+        if (lane == 0) {
+            for (int k = 0; k < 6; k++) S.scene[k] = v[k];
+            out.scene[0] = make_float4(v[0], v[1], v[2], 0.0f);
+            out.scene[1] = make_float4(v[3], v[4], v[5], 0.0f);
+        }
+    }
+    __syncthreads();
+    const Quant quant(S.scene);
+    for (uint32_t i = tid; i < n; i += SMALL_THREADS) {
+        S.key[0][i] = quant.code(__ldg(prims + 2 * i), __ldg(prims + 2 * i + 1));
+        S.val[0][i] = (uint16_t)i;
+    }
+
+    // k_radix_pass's ranks, one tile: a warp's keys are a run of `items` x 32
+    const uint32_t items = (n + SMALL_THREADS - 1) / SMALL_THREADS, wbase = warp * items * 32u;
+    for (int pass = 0; pass < PASSES; pass++) {
+        const uint32_t from = pass & 1, shift = 8 * pass;
+        for (int k = 0; k < 8; k++) S.digit[warp][lane + 32 * k] = 0;
+        __syncthreads();  // the keys too
+        uint32_t key[SMALL_ITEMS], rank[SMALL_ITEMS];
+        uint16_t val[SMALL_ITEMS];
+#pragma unroll
+        for (uint32_t j = 0; j < (uint32_t)SMALL_ITEMS; j++) {
+            const uint32_t idx = wbase + j * 32u + lane;
+            const bool ok = j < items && idx < n;
+            key[j] = ok ? S.key[from][idx] : 0u;
+            val[j] = ok ? S.val[from][idx] : 0u;
+            const uint32_t d = (key[j] >> shift) & 255u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, ok ? d : 256u + lane);
+            const uint32_t before = ok ? S.digit[warp][d] : 0u;
+            __syncwarp();
+            if (ok && lane == 31u - __clz(peers)) S.digit[warp][d] = before + __popc(peers);
+            __syncwarp();
+            rank[j] = before + __popc(peers & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        uint32_t run = 0, inc = 0;
+        if (tid < 256) {
+#pragma unroll 8
+            for (int w = 0; w < SMALL_WARPS; w++) {
+                const uint32_t c = S.digit[w][tid];
+                S.digit[w][tid] = run;
+                run += c;
+            }
+            inc = run;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            if (lane == 31) S.scan[warp] = inc;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            for (uint32_t w = 0; w < warp; w++) inc += S.scan[w];
+            S.digit_base[tid] = inc - run;
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < (uint32_t)SMALL_ITEMS; j++) {
+            if (j < items && wbase + j * 32u + lane < n) {
+                const uint32_t d = (key[j] >> shift) & 255u;
+                const uint32_t pos = S.digit_base[d] + S.digit[warp][d] + rank[j];
+                S.key[from ^ 1][pos] = key[j];
+                S.val[from ^ 1][pos] = val[j];
+            }
+        }
+        __syncthreads();
+    }
+    static_assert(PASSES % 2 == 0, "the sorted keys end where they began");
+
+    // k_karras
+    for (uint32_t i = tid; i < n; i += SMALL_THREADS) {
+        out.sorted[i] = S.key[0][i];
+        out.order[i] = S.val[0][i];
+        out.counters[i] = 0;
+        S.arrived[i] = 0;
+        if (i >= ninner) continue;
+        const uint4 L = karras_link<int>([&](int k) { return S.key[0][k]; }, (int)n, (int)i);
+        out.links[i] = L;
+        S.width[i] = (uint16_t)(L.w - L.z);
+        S.parent[L.x] = S.parent[L.y] = (uint16_t)i;
+        out.parent[L.x] = i;
+        out.parent[L.y] = i;
+    }
+    if (tid == 0) out.parent[0] = NONE;
+    __syncthreads();
+    for (uint32_t i = tid; i < ninner; i += SMALL_THREADS) {
+        uint32_t a = i, hops = 0;
+        for (; a != 0 && hops < STACK; hops++) a = S.parent[a];
+        S.depth[i] = (uint8_t)(a == 0 ? hops : STACK);
+    }
+    __syncthreads();
+
+    // k_pack
+    uint32_t deepest = 0;
+    for (uint32_t base = 0; base < total; base += SMALL_THREADS) {
+        const uint32_t i = base + tid;
+        bool start = false;
+        if (i < total) {
+            const bool internal = i < ninner;
+            uint32_t lo = (i - ninner) | LEAF, hi = i - ninner + 1;
+            uint2 span = make_uint2(0, 0);
+            if (internal) {
+                const uint4 L = out.links[i];
+                lo = L.x;
+                hi = L.y;
+                span = make_uint2(L.z, L.w);
+            }
+            bool reach = i == 0;
+            uint32_t dep = 0;
+            if (i != 0) {
+                const uint32_t p = S.parent[i];
+                dep = S.depth[p] + 1u;
+                reach = S.width[p] >= leaf && dep < STACK;
+            }
+            if (reach) {
+                deepest = dep > deepest ? dep : deepest;
+                start = !internal || span.y - span.x < leaf || dep + 1 >= STACK;
+                if (start && internal) {
+                    lo = span.x | LEAF;
+                    hi = span.y + 1;
+                }
+            }
+            if (start)
+                for (uint32_t k = lo & ~LEAF; k < hi; k++) out.owner[k] = k == (lo & ~LEAF) ? i : NO_OWNER;
+            out.nodes[2 * i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(lo));
+            out.nodes[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(hi));
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, start);
+        uint32_t at = 0;
+        if (lane == 0 && m) at = atomicAdd(&S.nstarts, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (start) out.starts[at + __popc(m & ((1u << lane) - 1u))] = i;
+    }
+    deepest = __reduce_max_sync(0xffffffffu, deepest);
+    if (lane == 0 && deepest) atomicMax(&S.max_depth, deepest);
+    __syncthreads();
+    if (tid < 16) out.scalars[tid] = tid == 0 ? S.max_depth : (tid == 1 ? S.nstarts : 0u);
+    if (!refit) return;
+
+    // the refit: a leaf a thread, then up while this thread is the second to arrive
+    for (uint32_t k = tid; k < S.nstarts; k += SMALL_THREADS) {
+        uint32_t i = out.starts[k];
+        uint32_t lo = __float_as_uint(out.nodes[2 * i].w), hi = __float_as_uint(out.nodes[2 * i + 1].w);
+        RefitBox box{FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+        for (uint32_t s = lo & ~LEAF; s < hi; s++) {
+            const uint32_t p = S.val[0][s];
+            const float4 a = __ldg(prims + 2 * p), b = __ldg(prims + 2 * p + 1);
+            grow(box, RefitBox{a.x, a.y, a.z, b.x, b.y, b.z});
+        }
+        for (;;) {
+            out.nodes[2 * i] = make_float4(box.lx, box.ly, box.lz, __uint_as_float(lo));
+            out.nodes[2 * i + 1] = make_float4(box.hx, box.hy, box.hz, __uint_as_float(hi));
+            if (i == 0) break;
+            const uint32_t p = S.parent[i];
+            lo = __float_as_uint(out.nodes[2 * p].w);
+            hi = __float_as_uint(out.nodes[2 * p + 1].w);
+            __threadfence_block();
+            if (atomicAdd(&S.arrived[p], 1u) == 0) break;  // the sibling finishes p
+            __threadfence_block();
+            const uint32_t sib = lo == i ? hi : lo;
+            const float4 a = out.nodes[2 * sib], b = out.nodes[2 * sib + 1];
+            grow(box, RefitBox{a.x, a.y, a.z, b.x, b.y, b.z});
+            i = p;
+        }
+    }
+}
+
 // The reference's Jacobi Refit step (kernel.rs:130-170), for Pass replay.
 __global__ void k_refit_jacobi(const float4* __restrict__ prims, const uint32_t* __restrict__ order,
                                const float4* __restrict__ src, float4* __restrict__ dst, uint32_t n) {
@@ -640,6 +885,16 @@ int32_t enqueue_sort_raw(Ctx* c, const uint32_t* codes, uint32_t n, uint32_t* or
 // Every stage of Bvh::build over w.prims[0..n) on the context's stream.
 int32_t enqueue_build(Ctx* c, BvhWork& w, uint32_t n, uint32_t leaf, Gate gate, bool refit) {
     cudaStream_t s = c->stream;
+    if (n > 0 && n <= SMALL_MAX) {
+        static std::atomic<uint64_t> done{0};
+        PHX_TRY(smem_limit(k_build_small, (int)sizeof(SmallTree), c->device, done));
+        const SmallOut out{(float4*)w.scene.ptr,      (uint32_t*)w.sorted.ptr, (uint32_t*)w.order.ptr,
+                           (uint32_t*)w.parent.ptr,   (uint32_t*)w.starts.ptr, w.owner(),
+                           (uint32_t*)w.counters.ptr, (uint32_t*)w.scalars.ptr, (uint4*)w.links.ptr,
+                           (float4*)w.nodes.ptr};
+        k_build_small<<<1, SMALL_THREADS, sizeof(SmallTree), s>>>((const float4*)w.prims.ptr, n, leaf, out, refit, gate);
+        return cuda_check(cudaGetLastError(), "bvh build");
+    }
     PHX_TRY(zero(c, w.scalars.ptr, 64, gate));
     if (n == 0) return PHX_OK;
     const float4* prims = (const float4*)w.prims.ptr;

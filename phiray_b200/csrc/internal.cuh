@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <mutex>
 #include <string>
@@ -137,3 +138,19 @@ struct phx_buf_s {
     } while (0)
 
 #define PHX_CUDA(expr) PHX_TRY(phx::cuda_check((expr), #expr))
+
+namespace phx {
+
+// Raises a kernel's dynamic shared-memory limit (and carveout) once per device.
+template <typename F>
+int32_t smem_limit(F* kernel, int bytes, int device, std::atomic<uint64_t>& done) {
+    const uint64_t bit = 1ull << (device & 63);
+    if (done.load(std::memory_order_acquire) & bit) return PHX_OK;
+    PHX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    // the largest shared-memory carveout, so that several blocks fit an SM
+    PHX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    done.fetch_or(bit, std::memory_order_release);
+    return PHX_OK;
+}
+
+}  // namespace phx

@@ -313,10 +313,10 @@ int32_t enqueue_sort_raw(Ctx* c, const uint32_t* codes, uint32_t n, uint32_t* or
 // refit = false leaves out the last one, the bounds (the caller runs a
 // refit of its own, which must climb as refit_climb does).
 int32_t enqueue_build(Ctx* c, BvhWork& w, uint32_t n, uint32_t leaf, Gate gate = Gate{}, bool refit = true);
-// Bvh::refit (slots = false: prims through order; true: prims already in
-// slot order, Bvh::refit_slots).
 // The climbs a large refit_block left in w.climbs(n).
 int32_t enqueue_climbs(Ctx* c, BvhWork& w, uint32_t n, Gate gate = Gate{});
+// Bvh::refit (slots = false: prims through order; true: prims already in
+// slot order, Bvh::refit_slots).
 int32_t enqueue_refit(Ctx* c, BvhWork& w, uint32_t n, bool slots, Gate gate = Gate{});
 
 }  // namespace phx

@@ -32,18 +32,6 @@ struct Plan {
     static constexpr int TOTAL = B_OFF + B_BYTES + B_ROOM;
 };
 
-// Raises a kernel's dynamic shared-memory limit (and carveout) once per device.
-template <typename F>
-int32_t smem_limit(F* kernel, int bytes, int device, std::atomic<uint64_t>& done) {
-    const uint64_t bit = 1ull << (device & 63);
-    if (done.load(std::memory_order_acquire) & bit) return PHX_OK;
-    PHX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    // the largest shared-memory carveout, so that several blocks fit an SM
-    PHX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    done.fetch_or(bit, std::memory_order_release);
-    return PHX_OK;
-}
-
 __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
