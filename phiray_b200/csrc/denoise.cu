@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256) k_prep(const uint32_t* __restrict__ px, u
     const f3 demod = v3at(px, 1 * n, i) * k / vmax(albedo, mk(0.05f));
     g0[i] = make_float4(albedo.x, albedo.y, albedo.z, depth);
     g1[i] = make_float4(normal.x, normal.y, normal.z, k);
-    a[i] = make_float4(demod.x, demod.y, demod.z, 0.0f);
+    a[i] = make_float4(demod.x, demod.y, demod.z, luma_of(demod));
 }
 
 struct RoundArgs {
@@ -61,16 +61,49 @@ struct RoundArgs {
     float exposure, gamma;
 };
 
-// denoise.wgsl:47-134, one round, guides from the prep planes.
+// a / b for one b and many a: two corrected steps with y = RN(1 / b), exactly
+// rounded by Markstein's theorem (IBM J. Res. Dev. 34, 1990) while nothing
+// under- or overflows, which the caller checks (plain).
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+    float q = a * y;
+    q = fmaf(fmaf(-q, b, a), y, q);
+    return fmaf(fmaf(-q, b, a), y, q);
+}
+
+// Of 0 or 2^-60 .. 2^60: two such have a quotient whose remainders are normal.
+__device__ __forceinline__ bool plain(float a) {
+    const uint32_t u = __float_as_uint(a);
+    return u == 0u || u - 0x21800000u <= 0x5D800000u - 0x21800000u;
+}
+
+// A tap's weight as written, for values div_by or the scaling below does not take.
+__device__ __noinline__ float stop_any(float dn, float da, float nd, float cd, float nl, float lc, float s0, float s1,
+                                       float s2, float s3) {
+    const float dd = nd / cd, dl = nl / lc;
+    return pm_exp(-dn * s0 - da * s1 - dd * s2 - dl * dl * s3);
+}
+
+// denoise.wgsl:47-134, one round, guides from the prep planes; the w of `in`
+// and `out` is the colour's luma. Bound by instructions (some 200 issue slots a
+// tap, 25 taps a pixel, DRAM under a tenth of its rate). The two divisions
+// have one divisor each a pixel, whose reciprocal is taken once; pm_exp's
+// scaling is one addition to the exponent where the result is normal; a
+// luma is worked out once a pixel instead of once a tap. At 1920 x 1080 the four
+// rounds took 299 / 288 / 288 / 325 us, now 227 / 238 / 241 / 292 (the last one
+// with the view transform). Six blocks an SM are the best of 4, 6 and 8 but in
+// the first round, which spills then (250 us); rows unrolled too, 271 / 269 /
+// 265 / 332; 16 x 16 blocks 239 / 249 / 253 / 296.
 template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(256) k_round(const float4* __restrict__ g0, const float4* __restrict__ g1,
+__global__ void __launch_bounds__(256, FIRST ? 1 : 6) k_round(const float4* __restrict__ g0, const float4* __restrict__ g1,
                                                const float4* __restrict__ in, float4* __restrict__ out, uint32_t* px,
                                                RoundArgs p) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= (int)p.w || y >= (int)p.h) return;
     const uint32_t i = (uint32_t)y * p.w + (uint32_t)x;
-    f3 centre = xyz(__ldg(in + i));
+    const float4 own = __ldg(in + i);
+    f3 centre = xyz(own);
+    float lc = own.w;
     if (FIRST) {
         float near_top = 0.0f;
         f3 near_sum = mk(0.0f);
@@ -79,44 +112,70 @@ __global__ void __launch_bounds__(256) k_round(const float4* __restrict__ g0, co
             for (int dx = -1; dx <= 1; dx++) {
                 const int sx = x + dx, sy = y + dy;
                 if ((dx == 0 && dy == 0) || sx < 0 || sy < 0 || sx >= (int)p.w || sy >= (int)p.h) continue;
-                const f3 c = xyz(__ldg(in + (uint32_t)sy * p.w + (uint32_t)sx));
-                near_top = fmaxf(near_top, luma_of(c));
-                near_sum += c;
+                const float4 c = __ldg(in + (uint32_t)sy * p.w + (uint32_t)sx);
+                near_top = fmaxf(near_top, c.w);
+                near_sum += xyz(c);
                 near_n += 1.0f;
             }
         }
-        if (near_n > 0.0f && luma_of(centre) > 1.5f * near_top + 0.05f) centre = near_sum / near_n;
+        if (near_n > 0.0f && lc > 1.5f * near_top + 0.05f) {
+            centre = near_sum / near_n;
+            lc = luma_of(centre);
+        }
     }
     const float4 c0 = __ldg(g0 + i), c1 = __ldg(g1 + i);
     const f3 cn = xyz(c1), ca = xyz(c0);
     const float cd = c0.w;
-    const float lc = luma_of(centre);
+    const float bd = fmaxf(fabsf(cd), 1e-3f), bl = 0.08f + lc;  // the divisors
+    const float yd = 1.0f / bd, yl = 1.0f / bl;
+    const bool divisors = bl > 0.0f && plain(bd) && plain(bl);
     f3 sum = mk(0.0f);
     float weight = 0.0f;
+#pragma unroll 1
     for (int dy = -2; dy <= 2; dy++) {
         const int sy = y + dy * (int)p.step;
         if (sy < 0 || sy >= (int)p.h) continue;
+        const float ky = KERNEL3[dy < 0 ? -dy : dy];
+#pragma unroll
         for (int dx = -2; dx <= 2; dx++) {
             const int sx = x + dx * (int)p.step;
             if (sx < 0 || sx >= (int)p.w) continue;
             const uint32_t j = (uint32_t)sy * p.w + (uint32_t)sx;
             const float4 j0 = __ldg(g0 + j);
             if ((j0.w < 0.0f) != (cd < 0.0f)) continue;
-            const f3 tap = (j == i) ? centre : xyz(__ldg(in + j));
+            const bool same = dx == 0 && dy == 0;
+            const float4 tin = __ldg(in + j);
+            const f3 tap = same ? centre : xyz(tin);
             const float4 j1 = __ldg(g1 + j);
             const float dn = fmaxf(0.0f, 1.0f - dot(cn, xyz(j1)));
             const float da = length(xyz(j0) - ca);
-            const float dd = fabsf(j0.w - cd) / fmaxf(fabsf(cd), 1e-3f);
-            const float dl = fabsf(luma_of(tap) - lc) / (0.08f + lc);
-            const float stop = pm_exp(-dn * p.s0 - da * p.s1 - dd * p.s2 - dl * dl * p.s3);
-            const float k = KERNEL3[dx < 0 ? -dx : dx] * KERNEL3[dy < 0 ? -dy : dy];
+            const float nd = fabsf(j0.w - cd), nl = fabsf((same ? lc : tin.w) - lc);
+            const float dd = div_by(nd, bd, yd), dl = div_by(nl, bl, yl);
+            const float e = (-dn * p.s0 - da * p.s1 - dd * p.s2 - dl * dl * p.s3) * 1.44269502f;
+            // pm_exp2(e): 2^k (e rounded, in the low bits of e + 1.5 * 2^23) times a polynomial
+            const float big = e + 12582912.0f;
+            const float t = (e - (big - 12582912.0f)) * 0.693147182f;
+            float q = 1.98412701e-4f;
+            q = q * t + 1.38888892e-3f;
+            q = q * t + 8.33333377e-3f;
+            q = q * t + 4.16666679e-2f;
+            q = q * t + 1.66666672e-1f;
+            q = q * t + 0.5f;
+            q = q * t + 1.0f;
+            q = q * t + 1.0f;
+            float stop = __uint_as_float(__float_as_uint(q) + (__float_as_uint(big) << 23));
+            if (e < -150.0f) stop = 0.0f;
+            // (a result of exponent k >= -120 is normal)
+            if (!(divisors && plain(nd) && plain(nl) && (e < -150.0f || fabsf(e) < 120.0f)))
+                stop = stop_any(dn, da, nd, bd, nl, bl, p.s0, p.s1, p.s2, p.s3);
+            const float k = (dx == 0 ? 0.375f : (dx == 1 || dx == -1 ? 0.25f : 0.0625f)) * ky;
             sum += tap * k * stop;
             weight += k * stop;
         }
     }
     const f3 o = weight > 0.0f ? sum / weight : centre;
     if (!LAST) {
-        out[i] = make_float4(o.x, o.y, o.z, 0.0f);
+        out[i] = make_float4(o.x, o.y, o.z, luma_of(o));
         return;
     }
     const uint32_t n = p.n;
