@@ -226,7 +226,7 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
 
 /* GpuBvh::build (gpu.rs:23-74) from HOST prims: upload, then every stage on
  * the device — bounds, Morton codes, stable radix sort, Karras links, leaf
- * packing and depth, atomic bottom-up refit. No readback. n may be 0. */
+ * packing and depth, bottom-up refit. No readback. n may be 0. */
 int32_t phx_bvh_build(phx_ctx ctx, const phx_aabb* host_prims, uint32_t n, uint32_t leaf, phx_bvh* out);
 /* The same from prims already in device memory (copied into the BVH). */
 int32_t phx_bvh_build_device(phx_ctx ctx, const phx_aabb* device_prims, uint32_t n, uint32_t leaf, phx_bvh* out);
@@ -823,7 +823,7 @@ int32_t phx_batch_trace(phx_batch b);
 /* The autotuner: times the persistent launch at each block size and stack
  * placement, the dense persistent launch at 128 and 256 threads, and
  * per-scene launches of the megakernel (4 and 16 resident blocks) and of the
- * state machine, on the batch; keeps the fastest. ms (>= 11 floats, may be NULL)
+ * pooled render, on the batch; keeps the fastest. ms (>= 11 floats, may be NULL)
  * gets each configuration's time, *nconfigs their number. Waits. */
 int32_t phx_batch_autotune(phx_batch b, uint32_t* kind, uint32_t* threads, uint32_t* stack, float* ms,
                            uint32_t* nconfigs);
