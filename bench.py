@@ -41,7 +41,7 @@ WORKLOAD = ("c2_mesh: icosphere L8 (1,310,722 tris) + 4 area lights, 1920x1080, 
             "tree rebuild (the autotuner's pick of LBVH or binned SAH) + trace + denoise per frame")
 
 
-KERNEL_NAMES = ["megakernel", "state-machine/4", "state-machine/6", "state-machine/8", "megakernel/3", "megakernel/2",
+KERNEL_NAMES = ["megakernel", "pooled/512", "pooled/256", "pooled/128", "megakernel/3", "megakernel/2",
                 "megakernel/sync", "megakernel/2/sync", "megakernel/5", "megakernel/6", "megakernel/6/sync", "megakernel/8", "megakernel/8/sync",
                 "megakernel/10/sync", "megakernel/12/sync", "megakernel/16/sync", "wavefront",
                 "megakernel/reg8", "megakernel/8/sync/reg1", "megakernel/16/sync/reg1"]
@@ -819,7 +819,8 @@ def main() -> None:
     pk = peaks()
     achieved = alg_bytes / (trace_ms * 1e-3) / 1e9
     traffic = None
-    tpath = os.path.join(ROOT, "profiles", "trace_render_traffic.json")
+    pooled = KERNEL_NAMES[chosen].startswith("pooled")
+    tpath = os.path.join(ROOT, "profiles", "pool_render_traffic.json" if pooled else "trace_render_traffic.json")
     if os.path.exists(tpath):
         with open(tpath) as f:
             tinfo = json.load(f)
@@ -902,7 +903,8 @@ def main() -> None:
                                 "achieved_gbs": round(inc_bytes / (inc_ms * 1e-3) / 1e9, 1),
                                 "frac_of_hbm": round(inc_bytes / (inc_ms * 1e-3) / 1e9 / pk["hbm_gbs"], 4)},
             "primary_grays": round(n / (prim_ms * 1e-3) / 1e9, 3),
-            "roofline": {"bound": "hbm", "kernel": "k_render (path-trace megakernel)", "achieved": round(achieved, 1),
+            "roofline": {"bound": "hbm", "kernel": "k_render_pool (pooled render)" if pooled else "k_render (path-trace megakernel)",
+                         "achieved": round(achieved, 1),
                          "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": round(achieved / pk["hbm_gbs"], 4),
                          "traffic": traffic, "peak_source": pk["source"],
                          "algorithmic": f"{counts[1]} node steps x 64 B + {counts[2]} triangle tests x 48 B per launch"},
