@@ -127,10 +127,15 @@ __device__ __forceinline__ void refit_climb(uint32_t i, float lx, float ly, floa
 // order. The subtrees rise in rounds: a node whose children were made in
 // earlier rounds takes the union of their boxes (one barrier a round, `stamp`
 // holds the round). What has no parent made here climbs through memory as
-// refit_climb. A climb from every leaf had two atomics, two fences and three
-// dependent reads a node, all through L2: 89 us at 1M boxes, and 21 us of
-// latency at 1,000. The smallest bytes are the boxes, the inner nodes' links
-// and all the nodes written, 0.14 GB at 1M or 22 us.
+// refit_climb does. A climb from every leaf had two atomics, two fences and
+// three dependent reads a node, all through L2: 89 us at 1M boxes, 137 at 2M
+// and 21 of latency at 1,000; now 70, 114 and 16. The smallest bytes are the
+// boxes, the inner nodes' links and all the nodes written, 0.14 GB at 1M or 22
+// us; what keeps it from that is the climbs' chain (29 us), shared memory's
+// pipe and the rounds' barriers. A box is one 16- and one 8-byte word there: six
+// words of 4 took 45 us at 1M without the climbs, this takes 41. With the six
+// words: blocks of 256 slots 41 + 30 us at 1M, 83 + 43 at 2M. Steps of a warp
+// alone between barriers cost more than the barriers: two 47, four 56, six 65.
 //
 // `slot(s, last, write)` gives slot s's box; write: also what goes with the
 // slot (once a slot), last: the slot ends its leaf. owner[s]: the leaf (an
@@ -174,22 +179,21 @@ __device__ __forceinline__ void refit_block(uint32_t n, const uint32_t* __restri
                                             const uint32_t* __restrict__ parent, float4* nodes, uint32_t* counters,
                                             uint32_t* status, uint32_t* list, const Slot& slot) {
     constexpr uint32_t SB = REFIT_SLOTS, CUT = 0x80000000u;  // CUT: a record's leaf bit
-    __shared__ float box[6][2 * SB];        // inner nodes, then leaf nodes
+    __shared__ float4 box4[2 * SB];         // lx ly lz hx of inner nodes, then of leaf nodes
+    __shared__ float2 box2[2 * SB];         // hy hz
     __shared__ uint8_t stamp[2 * SB];       // the round a node was made in; 0: not here
     __shared__ uint8_t taken[2 * SB];       // its parent was made here
     __shared__ uint32_t open[REFIT_OPEN], nopen;  // the nodes to climb from
     const uint32_t t = threadIdx.x, s0 = blockIdx.x * SB, s = s0 + t;
     const uint32_t first_leaf = n - 1;      // node ids below are inner nodes
     auto put = [&](uint32_t k, const RefitBox& b) {
-        box[0][k] = b.lx;
-        box[1][k] = b.ly;
-        box[2][k] = b.lz;
-        box[3][k] = b.hx;
-        box[4][k] = b.hy;
-        box[5][k] = b.hz;
+        box4[k] = make_float4(b.lx, b.ly, b.lz, b.hx);
+        box2[k] = make_float2(b.hy, b.hz);
     };
     auto get = [&](uint32_t k) {
-        return RefitBox{box[0][k], box[1][k], box[2][k], box[3][k], box[4][k], box[5][k]};
+        const float4 a = box4[k];
+        const float2 b = box2[k];
+        return RefitBox{a.x, a.y, a.z, a.w, b.x, b.y};
     };
     auto store = [&](uint32_t id, const RefitBox& b, uint32_t lo, uint32_t hi) {
         nodes[2 * (size_t)id] = make_float4(b.lx, b.ly, b.lz, __uint_as_float(lo));
