@@ -216,7 +216,8 @@ typedef struct phx_bvh_s* phx_bvh;
  * costs more than testing what the node holds or at depth 31, the
  * reference's in-place partition of each node's slots and its node
  * numbering, bounds refit bottom up. All pointers are DEVICE memory:
- * prims (n phx_aabb), nodes (room for 2n - 1), order (n). Writes the node
+ * prims (n phx_aabb), nodes (room for 2n - 1), order (n), each aligned to 4
+ * bytes (prims and nodes fastest at a multiple of 16). Writes the node
  * count and depth; stream-ordered, waits once or twice per tree level.
  * A node under 128 slots and its whole subtree are a warp's, 128-2,047 slots
  * a block's, larger ones are cut over blocks of 2,048 slots (1.3 M prims:

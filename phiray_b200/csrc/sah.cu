@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "rules.cuh"
 #include "sah_core.cuh"
 
 namespace phx {
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree(const uint32_t* 
                                                                 const float* __restrict__ centres, uint32_t* order,
                                                                 uint32_t leaf, uint4* __restrict__ loc,
                                                                 uint32_t* __restrict__ loc_count, uint32_t* inner,
-                                                                uint32_t* max_depth) {
+                                                                uint32_t* max_depth, bool vec_prims) {
     __shared__ SubShared shared[SUB_WARPS];
     const uint32_t lane = threadIdx.x & 31u, k0 = blockIdx.x * SUB_WARPS + (threadIdx.x >> 5);
     if (k0 >= nseeds) return;
@@ -491,13 +492,20 @@ __global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree(const uint32_t* 
         const uint32_t i = order[seed.start + j];
         w.slot[j] = i;
         w.idx[j] = (uint8_t)j;
-        const float4 a = __ldg((const float4*)prims + 2 * (uint64_t)i), b = __ldg((const float4*)prims + 2 * (uint64_t)i + 1);
-        w.lo[0][j] = a.x;
-        w.lo[1][j] = a.y;
-        w.lo[2][j] = a.z;
-        w.hi[0][j] = b.x;
-        w.hi[1][j] = b.y;
-        w.hi[2][j] = b.z;
+        if (vec_prims) {
+            const float4 a = __ldg((const float4*)prims + 2 * (uint64_t)i), b = __ldg((const float4*)prims + 2 * (uint64_t)i + 1);
+            w.lo[0][j] = a.x;
+            w.lo[1][j] = a.y;
+            w.lo[2][j] = a.z;
+            w.hi[0][j] = b.x;
+            w.hi[1][j] = b.y;
+            w.hi[2][j] = b.z;
+        } else {
+            for (int k = 0; k < 3; k++) {
+                w.lo[k][j] = __ldg(prims + 8 * (uint64_t)i + k);
+                w.hi[k][j] = __ldg(prims + 8 * (uint64_t)i + 4 + k);
+            }
+        }
         for (int k = 0; k < 3; k++) w.c[k][j] = __ldg(centres + 3 * (uint64_t)i + k);
     }
     __syncwarp();
@@ -658,7 +666,8 @@ __global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree(const uint32_t* 
 __global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree_emit(
     const uint32_t* __restrict__ seeds, uint32_t nseeds, const TNode* __restrict__ tn, const uint4* __restrict__ loc,
     const uint32_t* __restrict__ loc_count, const uint32_t* __restrict__ rank, const uint32_t* __restrict__ final_index,
-    const float* __restrict__ prims, const uint32_t* __restrict__ order, sah::Box* boxes, float* nodes) {
+    const float* __restrict__ prims, const uint32_t* __restrict__ order, sah::Box* boxes, float* nodes,
+    bool vec_nodes) {
     __shared__ float s_box[SUB_WARPS][6][2 * SUB];  // 24 KB
     __shared__ uint8_t s_child[SUB_WARPS][2 * SUB];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, k0 = blockIdx.x * SUB_WARPS + warp;
@@ -713,9 +722,19 @@ __global__ void __launch_bounds__(32 * SUB_WARPS) k_sah_subtree_emit(
         const bool is_leaf = r == SUB_LEAF;
         const uint32_t lo_i = is_leaf ? mine[q].x | sah::LEAF_BIT : 2u * (R + r) + 1u;
         const uint32_t hi_i = is_leaf ? mine[q].y : 2u * (R + r) + 2u;
-        float4* o = (float4*)nodes + 2 * (uint64_t)at;
-        o[0] = make_float4(box[0][k], box[1][k], box[2][k], __uint_as_float(lo_i));
-        o[1] = make_float4(box[3][k], box[4][k], box[5][k], __uint_as_float(hi_i));
+        if (vec_nodes) {
+            float4* o = (float4*)nodes + 2 * (uint64_t)at;
+            o[0] = make_float4(box[0][k], box[1][k], box[2][k], __uint_as_float(lo_i));
+            o[1] = make_float4(box[3][k], box[4][k], box[5][k], __uint_as_float(hi_i));
+        } else {
+            float* o = nodes + 8 * (uint64_t)at;
+            for (int f = 0; f < 3; f++) {
+                o[f] = box[f][k];
+                o[4 + f] = box[3 + f][k];
+            }
+            o[3] = __uint_as_float(lo_i);
+            o[7] = __uint_as_float(hi_i);
+        }
         if (code == sah::NONE) {
             sah::Box b;
             for (int f = 0; f < 3; f++) {
@@ -1120,6 +1139,9 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     PHX_TRY(loc.reserve((size_t)2 * n * sizeof(uint4)));
     PHX_TRY(loc_count.reserve((size_t)cap * 4));
     const float* P = (const float*)prims;
+    // The caller's arrays are of floats and may start at any of them, in a
+    // packed buffer for instance: 16-byte accesses only where they start at one.
+    const bool vec_prims = aligned16(prims), vec_nodes = aligned16(nodes);
     TNode* T = (TNode*)tn.ptr;
     uint32_t* L = (uint32_t*)lists.ptr;
     uint32_t* cnt = (uint32_t*)counters.ptr;  // [0] temporary ids handed out, [1] next level's length
@@ -1229,7 +1251,7 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     if (nseeds)
         k_sah_subtree<<<sub_blocks, 32 * SUB_WARPS, 0, s>>>(SD, nseeds, T, P, (const float*)centres.ptr, order, leaf,
                                                             (uint4*)loc.ptr, (uint32_t*)loc_count.ptr,
-                                                            (uint32_t*)inner.ptr, LC + LC_DEPTH);
+                                                            (uint32_t*)inner.ptr, LC + LC_DEPTH, vec_prims);
     for (uint32_t lv = levels; lv-- > 0;)
         k_sah_count<<<blocks_of(len[lv], 256), 256, 0, s>>>(L + off[lv], len[lv], T, (uint32_t*)inner.ptr);
     for (uint32_t lv = 0; lv < levels; lv++)
@@ -1238,7 +1260,7 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     if (nseeds)
         k_sah_subtree_emit<<<sub_blocks, 32 * SUB_WARPS, 0, s>>>(
             SD, nseeds, T, (const uint4*)loc.ptr, (const uint32_t*)loc_count.ptr, (const uint32_t*)rank.ptr,
-            (const uint32_t*)final_index.ptr, P, order, (sah::Box*)boxes.ptr, (float*)nodes);
+            (const uint32_t*)final_index.ptr, P, order, (sah::Box*)boxes.ptr, (float*)nodes, vec_nodes);
     for (uint32_t lv = levels; lv-- > 0;)
         k_sah_emit<<<blocks_of(len[lv], 256), 256, 0, s>>>(L + off[lv], len[lv], T, (const uint32_t*)final_index.ptr, P,
                                                            order, (sah::Box*)boxes.ptr, (float*)nodes);
