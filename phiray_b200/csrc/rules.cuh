@@ -5,9 +5,99 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <numeric>
+#include <vector>
+
+#include "../../include/phiray_cuda.h"
+
 namespace phx {
 
 // Whether a kernel may read or write `p` by 16-byte words.
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0u; }
+
+// ---- which kernel traces a frame ----
+
+// A tracer whose render kernel was neither set nor autotuned.
+constexpr uint32_t KERNEL_UNSET = 0xFFFFFFFFu;
+
+// What a frame asks of the kernel that traces it.
+struct FrameForm {
+    uint32_t kernel;  // the tracer's (set or autotuned, or KERNEL_UNSET)
+    bool full;        // instances, or the floor grid
+    bool adaptive;
+    bool transmits;   // some material transmits light
+    bool capturing;   // the launches are recorded into a graph
+};
+
+inline bool pooled_id(uint32_t kernel) {
+    return kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8;
+}
+
+// The id of the kernel that traces the frame. The default is the pooled render
+// where it can run, which on a 65,536-face cloud at 256 x 256, 16 spp took 4.9
+// ms against the 4-block megakernel's 27 ms, on the 1.3 M-face mesh at 1080p,
+// 16 spp, 28 ms against 57, and on 64 x 48 pixels 0.6 against 0.8; else that
+// megakernel. All compute the same image. Adaptive Sampling runs on the
+// megakernel forms (the others take pixels by index, not from the open list);
+// the pooled render shades a path's one opaque camera hit, so it takes scenes
+// whose materials transmit no light; the wavefront's host polls its queues
+// between passes, which a recorded graph cannot.
+inline uint32_t frame_kernel(const FrameForm& f) {
+    uint32_t k = f.kernel;
+    if (k == KERNEL_UNSET) k = f.full ? PHX_KERNEL_MEGAKERNEL : PHX_KERNEL_STATE_MACHINE;
+    if (k == PHX_KERNEL_WAVEFRONT && (f.adaptive || f.capturing)) return PHX_KERNEL_MEGAKERNEL;
+    if (pooled_id(k) && (f.adaptive || (f.transmits && !f.full))) return PHX_KERNEL_MEGAKERNEL;
+    return k;
+}
+
+// Whether that is the pooled render, which needs buffers (under the same ids a
+// frame with `full` runs the state machine, which needs none).
+inline bool frame_pooled(const FrameForm& f) { return !f.full && pooled_id(frame_kernel(f)); }
+
+// ---- a batch's launches scene by scene, on side streams ----
+
+struct LaneJob {
+    uint64_t work;      // its samples
+    bool pooled;        // it runs on the pooled render, whose buffers these are
+    size_t state, out;  // bytes
+};
+
+struct LanePlan {
+    std::vector<uint32_t> order, lane;  // jobs, the largest first; the lane of each job
+    std::vector<uint8_t> buffers;       // job: the lane's buffers hold it (else it runs without)
+};
+
+// Jobs in order of their work, each on the lane with the least so far. A lane's
+// buffers are reserved once, by reserve(lane, state, out), for the largest need
+// of its pooled jobs; no buffer changes hands or size after that, since the
+// memory is ordered on the context's stream and the jobs run beside it. The
+// jobs of a lane without buffers run on a megakernel.
+template <class Reserve>
+LanePlan plan_lanes(const std::vector<LaneJob>& jobs, uint32_t lanes, const Reserve& reserve) {
+    LanePlan p;
+    p.order.resize(jobs.size());
+    std::iota(p.order.begin(), p.order.end(), 0u);
+    std::stable_sort(p.order.begin(), p.order.end(), [&](uint32_t x, uint32_t y) { return jobs[x].work > jobs[y].work; });
+    p.lane.resize(jobs.size());
+    p.buffers.assign(jobs.size(), 0);
+    std::vector<uint64_t> load(lanes, 0);
+    for (uint32_t j : p.order) {
+        p.lane[j] = (uint32_t)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[p.lane[j]] += jobs[j].work;
+    }
+    for (uint32_t l = 0; l < lanes; l++) {
+        size_t state = 0, out = 0;
+        for (uint32_t j : p.order)
+            if (p.lane[j] == l && jobs[j].pooled) {
+                state = std::max(state, jobs[j].state);
+                out = std::max(out, jobs[j].out);
+            }
+        if (!state || !reserve(l, state, out)) continue;
+        for (uint32_t j : p.order)
+            if (p.lane[j] == l) p.buffers[j] = jobs[j].pooled;
+    }
+    return p;
+}
 
 }  // namespace phx

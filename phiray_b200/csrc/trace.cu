@@ -17,6 +17,7 @@
 
 #include "lbvh.cuh"
 #include "render.cuh"
+#include "rules.cuh"
 
 namespace phx {
 
@@ -695,9 +696,6 @@ struct Forest {
     DevMem rec, flags, mesh_of, placed_dev, mesh_rec, slots, order_all, lamp_inst, slot_mesh, mesh_off, mesh_list;
 };
 
-// A tracer whose render kernel was neither set nor autotuned (launch_frame).
-constexpr uint32_t KERNEL_UNSET = 0xFFFFFFFFu;
-
 struct phx_tracer_s {
     Ctx* ctx = nullptr;
     uint32_t nverts = 0, nfaces = 0, nmats = 0, leaf = 4;
@@ -1129,22 +1127,28 @@ int32_t wf_buffers(phx_tracer tr, uint32_t count, WfBuffers& B) {
 constexpr size_t POOL_OUT_BYTES = (size_t)1 << 30;
 constexpr uint64_t POOL_SM_SLOTS = 8192;
 
-int32_t pool_buffers(Ctx* c, PoolScratch& scratch, uint32_t count, uint32_t spp, PoolBuffers& B) {
+struct PoolNeed {
+    uint64_t slots;
+    uint32_t spp;
+    size_t state, out;  // bytes
+};
+
+PoolNeed pool_need(Ctx* c, uint32_t count, uint32_t spp) {
+    PoolNeed p;
     const size_t sample = (size_t)count * pool_out_words() * 4;
     const uint32_t fit = (uint32_t)std::max<size_t>(POOL_OUT_BYTES / sample, 1);
     const uint32_t launches = (spp + fit - 1) / fit;
-    B.slots = (uint64_t)c->sms * POOL_SM_SLOTS;
-    B.spp = (spp + launches - 1) / launches;
-    PHX_TRY(scratch.state.reserve(B.slots * pool_slot_bytes()));
-    PHX_TRY(scratch.out.reserve(sample * B.spp));
-    B.pools = (uint32_t*)scratch.state.ptr;
-    B.out = (uint32_t*)scratch.out.ptr;
-    return PHX_OK;
+    p.slots = (uint64_t)c->sms * POOL_SM_SLOTS;
+    p.spp = (spp + launches - 1) / launches;
+    p.state = p.slots * pool_slot_bytes();
+    p.out = sample * p.spp;
+    return p;
 }
 
-// Launches the tracer's render kernel over pixels [first_px, first_px +
-// count_px) of frame F, whose camera is already in tr->cam (no host copy:
-// the launch can be recorded into a graph).
+PoolBuffers pool_buffers(const PoolScratch& scratch, const PoolNeed& p) {
+    return PoolBuffers{(uint32_t*)scratch.state.ptr, p.slots, (uint32_t*)scratch.out.ptr, p.spp};
+}
+
 // The wide tree of the binary tree the tracer walks now (collapsed on the
 // device when the tree changed since the last collapse; waits).
 int32_t ensure_wide(phx_tracer tr) {
@@ -1170,62 +1174,72 @@ int32_t ensure_wide(phx_tracer tr) {
     return read_status(c);
 }
 
-int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, uint32_t count_px, bool stats,
-                     PoolScratch* scratch = nullptr, cudaStream_t stream = nullptr) {
-    Ctx* c = tr->ctx;
-    if (!stream) stream = c->stream;
-    const bool full = tr->forest || F.grid > 0.0f;
-    // The default: the pooled render where it can run (below), which on a
-    // 65,536-face cloud at 256 x 256, 16 spp took 4.9 ms against the 4-block
-    // megakernel's 27 ms, on the 1.3 M-face mesh at 1080p, 16 spp, 28 ms
-    // against 57, and on 64 x 48 pixels 0.6 against 0.8; else that megakernel.
-    uint32_t kernel = tr->kernel;
-    if (kernel == KERNEL_UNSET) kernel = full ? PHX_KERNEL_MEGAKERNEL : PHX_KERNEL_STATE_MACHINE;
-    const Scene S = scene_of(tr);
-    // Adaptive Sampling runs on the megakernel forms (the others take pixels
-    // by index, not from the open list); they all compute the same image, so
-    // an adaptive frame takes the 4-block form instead.
-    if (F.adapt_on && kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8)
-        kernel = PHX_KERNEL_MEGAKERNEL;
-    const RenderLaunch L{S,        F,       sun,    (uint32_t*)tr->px.ptr, first_px, count_px,
-                         (unsigned long long*)tr->rays.ptr, (uint32_t*)tr->next.ptr, c->sms, stream};
-    if (kernel == PHX_KERNEL_WAVEFRONT) {
-        // the host polls its queues between passes: not while a graph is recorded
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        PHX_CUDA(cudaStreamIsCapturing(stream, &cap));
-        if (cap != cudaStreamCaptureStatusNone || F.adapt_on) {
-            kernel = PHX_KERNEL_MEGAKERNEL;
-        } else {
-            WfBuffers B;
-            PHX_TRY(wf_buffers(tr, count_px, B));
-            return render_wavefront(full, stats, L, B);
-        }
-    }
-    if (full) return render_full(kernel, stats, L);
-    if (kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8) {
-        // The pooled render shades a path's one opaque camera hit, so it takes
-        // scenes whose materials transmit no light. Its buffers are the
-        // context's, which a recorded graph must not hold (they may grow
-        // before it is replayed), or the caller's `scratch`. Otherwise, and
-        // where there is no memory for them, the 4-block megakernel.
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        PHX_CUDA(cudaStreamIsCapturing(stream, &cap));
-        if (!tr->transmits && count_px && (scratch || cap == cudaStreamCaptureStatusNone)) {
-            std::unique_lock<std::mutex> lock(c->path_pool_lock, std::defer_lock);
-            if (!scratch) lock.lock();
-            PoolBuffers B;
-            const int32_t rc = pool_buffers(c, scratch ? *scratch : c->path_pool, count_px, F.spp, B);
-            if (rc >= 0) return render_pooled(kernel, stats, L, B);
-            if (rc != PHX_ERR_OOM && cap == cudaStreamCaptureStatusNone) return rc;
-        }
-        kernel = PHX_KERNEL_MEGAKERNEL;
-    }
+FrameForm form_of(phx_tracer tr, const Frame& F, bool capturing) {
+    return FrameForm{tr->kernel, tr->forest || F.grid > 0.0f, F.adapt_on != 0u, tr->transmits, capturing};
+}
+
+int32_t capturing(cudaStream_t s, bool& on) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PHX_CUDA(cudaStreamIsCapturing(s, &cap));
+    on = cap != cudaStreamCaptureStatusNone;
+    return PHX_OK;
+}
+
+int32_t launch_megakernel(uint32_t kernel, bool stats, const RenderLaunch& L) {
     if (kernel >= PHX_KERNEL_MEGAKERNEL_6 && kernel <= PHX_KERNEL_MEGAKERNEL_8_SYNC) return render_flat_b(kernel, stats, L);
     if (kernel >= PHX_KERNEL_MEGAKERNEL_10_SYNC && kernel <= PHX_KERNEL_MEGAKERNEL_16_SYNC)
         return render_flat_c(kernel, stats, L);
     if (kernel >= PHX_KERNEL_MEGAKERNEL_REG && kernel <= PHX_KERNEL_MEGAKERNEL_16_SYNC_REG)
         return render_flat_r(kernel, stats, L);
     return render_flat_a(kernel, stats, L);
+}
+
+RenderLaunch launch_of(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, uint32_t count_px, cudaStream_t s) {
+    return RenderLaunch{scene_of(tr), F, sun, (uint32_t*)tr->px.ptr, first_px, count_px,
+                        (unsigned long long*)tr->rays.ptr, (uint32_t*)tr->next.ptr, tr->ctx->sms, s};
+}
+
+// Launches the tracer's render kernel over pixels [first_px, first_px +
+// count_px) of frame F, whose camera is already in tr->cam (no host copy: the
+// launch can be recorded into a graph), on the context's stream.
+int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, uint32_t count_px, bool stats) {
+    Ctx* c = tr->ctx;
+    bool recorded = false;
+    PHX_TRY(capturing(c->stream, recorded));
+    const FrameForm form = form_of(tr, F, recorded);
+    const uint32_t kernel = frame_kernel(form);
+    const RenderLaunch L = launch_of(tr, F, sun, first_px, count_px, c->stream);
+    if (kernel == PHX_KERNEL_WAVEFRONT) {
+        WfBuffers B;
+        PHX_TRY(wf_buffers(tr, count_px, B));
+        return render_wavefront(form.full, stats, L, B);
+    }
+    if (form.full) return render_full(kernel, stats, L);
+    if (!pooled_id(kernel)) return launch_megakernel(kernel, stats, L);
+    // The pooled render's buffers are the context's, which a recorded graph
+    // must not hold (they may grow before it is replayed). There, and where
+    // there is no memory for them, the 4-block megakernel.
+    if (count_px && !recorded) {
+        const PoolNeed need = pool_need(c, count_px, F.spp);
+        std::lock_guard<std::mutex> lock(c->path_pool_lock);
+        int32_t rc = c->path_pool.state.reserve(need.state);
+        if (rc >= 0) rc = c->path_pool.out.reserve(need.out);
+        if (rc >= 0) return render_pooled(kernel, stats, L, pool_buffers(c->path_pool, need));
+        if (rc != PHX_ERR_OOM) return rc;
+    }
+    return launch_megakernel(PHX_KERNEL_MEGAKERNEL, stats, L);
+}
+
+// A frame of a batch on a side stream, with the side stream's buffers for the
+// pooled render, or null: nothing is allocated here. (Not the wavefront.)
+int32_t launch_frame_on(cudaStream_t s, const PoolBuffers* buffers, phx_tracer tr, const Frame& F, f3 sun) {
+    const FrameForm form = form_of(tr, F, true);
+    const uint32_t kernel = frame_kernel(form);
+    const RenderLaunch L = launch_of(tr, F, sun, 0, F.n, s);
+    if (form.full) return render_full(kernel, false, L);
+    if (!pooled_id(kernel)) return launch_megakernel(kernel, false, L);
+    if (buffers) return render_pooled(kernel, false, L, *buffers);
+    return launch_megakernel(PHX_KERNEL_MEGAKERNEL, false, L);
 }
 
 // The frame record of `cam` for tr, whose lights the kernels read from tr->cam.
@@ -2126,60 +2140,70 @@ int32_t batch_prepare(phx_batch b) {
     return wait_stream(c->stream, BATCH_WAIT_MS);  // the pageable sources are released on return
 }
 
-// One launch a scene, the largest first, each on the side stream with the
-// least work so far. The serving frame of six 256^2-512^2 scenes traced in
-// 26.1 ms on one stream, 22.5 on three.
+// One launch a scene on the side streams (plan_lanes). The serving frame of six
+// 256^2-512^2 scenes traced in 26.1 ms on one stream, 22.5 on three. A tracer
+// set to the wavefront follows on the context's stream: its host polls.
 int32_t trace_per_scene(phx_batch b) {
     Ctx* c = b->ctx;
+    if (!b->fork) PHX_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    for (auto& lane : b->lanes) {
+        if (!lane.stream) PHX_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
+        if (!lane.done) PHX_CUDA(cudaEventCreateWithFlags(&lane.done, cudaEventDisableTiming));
+    }
+    bool recorded = false;
+    PHX_TRY(capturing(c->stream, recorded));
     const size_t nj = b->jobs.size();
-    auto work = [&](size_t j) { return (uint64_t)b->jobs[j].w * b->jobs[j].h * b->jobs[j].spp; };
-    std::vector<uint32_t> order(nj), lane_of(nj);
-    for (size_t j = 0; j < nj; j++) order[j] = (uint32_t)j;
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return work(x) > work(y); });
-    uint64_t load[phx_batch_s::LANES] = {};
-    for (uint32_t j : order) {
-        uint32_t l = 0;
-        for (uint32_t k = 1; k < phx_batch_s::LANES; k++)
-            if (load[k] < load[l]) l = k;
-        lane_of[j] = l;
-        load[l] += work(j);
+    std::vector<Frame> frames;
+    std::vector<PoolNeed> need;
+    std::vector<LaneJob> jobs;
+    for (const BatchJob& bj : b->jobs) {
+        frames.push_back(frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp));
+        need.push_back(pool_need(c, bj.w * bj.h, bj.spp));
+        jobs.push_back(LaneJob{(uint64_t)bj.w * bj.h * bj.spp, frame_pooled(form_of(bj.tr, frames.back(), recorded)),
+                               need.back().state, need.back().out});
     }
-    if (!b->fork) {
-        PHX_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-        for (auto& lane : b->lanes) {
-            PHX_CUDA(cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking));
-            PHX_CUDA(cudaEventCreateWithFlags(&lane.done, cudaEventDisableTiming));
-        }
-    }
-    // The buffers are sized on the context's stream before the side streams
-    // start (where there is no memory for them launch_frame does without).
-    for (size_t j = 0; j < nj; j++) {
-        const BatchJob& bj = b->jobs[j];
-        PoolBuffers B;
-        if (!bj.tr->forest && !bj.tr->transmits)
-            (void)pool_buffers(c, b->lanes[lane_of[j]].path_pool, bj.w * bj.h, bj.spp, B);
-    }
+    // A captured graph holds the buffers as they are, and a frame that is
+    // recorded takes what the one before it reserved.
+    const bool keep = recorded || b->exec;
+    const LanePlan plan = plan_lanes(jobs, phx_batch_s::LANES, [&](uint32_t l, size_t state, size_t out) {
+        PoolScratch& pool = b->lanes[l].path_pool;
+        if (keep) return pool.state.bytes >= state && pool.out.bytes >= out;
+        return pool.state.reserve(state) >= 0 && pool.out.reserve(out) >= 0;
+    });
     PHX_CUDA(cudaEventRecord(b->fork, c->stream));
-    for (auto& lane : b->lanes) PHX_CUDA(cudaStreamWaitEvent(lane.stream, b->fork, 0));
     int32_t rc = PHX_OK;
-    for (uint32_t j : order) {
-        BatchJob& bj = b->jobs[j];
-        auto& lane = b->lanes[lane_of[j]];
-        const Frame F = frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp);
-        rc = cuda_check(cudaMemsetAsync(bj.tr->rays.ptr, 0, 8, lane.stream), "rays");
+    auto step = [&](int32_t r) {
+        if (rc == PHX_OK && r < 0) rc = r;
+    };
+    for (auto& lane : b->lanes) step(cuda_check(cudaStreamWaitEvent(lane.stream, b->fork, 0), "fork"));
+    auto trace = [&](uint32_t j, cudaStream_t s, bool wavefront) {
+        const BatchJob& bj = b->jobs[j];
+        auto& lane = b->lanes[plan.lane[j]];
+        const f3 sun = mk(bj.cam.sun[0], bj.cam.sun[1], bj.cam.sun[2]);
+        step(cuda_check(cudaMemsetAsync(bj.tr->rays.ptr, 0, 8, s), "rays"));
+        if (rc < 0) return;
+        if (wavefront) {
+            step(launch_frame(bj.tr, frames[j], sun, 0, frames[j].n, false));
+        } else {
+            const PoolBuffers B = pool_buffers(lane.path_pool, need[j]);
+            step(launch_frame_on(s, plan.buffers[j] ? &B : nullptr, bj.tr, frames[j], sun));
+        }
         if (rc >= 0)
-            rc = launch_frame(bj.tr, F, mk(bj.cam.sun[0], bj.cam.sun[1], bj.cam.sun[2]), 0, bj.w * bj.h, false,
-                              &lane.path_pool, lane.stream);
-        if (rc >= 0)
-            rc = cuda_check(cudaMemcpyAsync((unsigned long long*)b->counters.ptr + 3 * j, bj.tr->rays.ptr, 8,
-                                            cudaMemcpyDeviceToDevice, lane.stream), "rays");
-        if (rc < 0) break;
-    }
+            step(cuda_check(cudaMemcpyAsync((unsigned long long*)b->counters.ptr + 3 * j, bj.tr->rays.ptr, 8,
+                                            cudaMemcpyDeviceToDevice, s), "rays"));
+    };
+    auto wavefront = [&](uint32_t j) {
+        return frame_kernel(form_of(b->jobs[j].tr, frames[j], recorded)) == PHX_KERNEL_WAVEFRONT;
+    };
+    for (uint32_t j : plan.order)
+        if (rc >= 0 && !wavefront(j)) trace(j, b->lanes[plan.lane[j]].stream, false);
     // joined whatever happened: later work and frees follow all of it
     for (auto& lane : b->lanes) {
-        PHX_CUDA(cudaEventRecord(lane.done, lane.stream));
-        PHX_CUDA(cudaStreamWaitEvent(c->stream, lane.done, 0));
+        step(cuda_check(cudaEventRecord(lane.done, lane.stream), "join"));
+        step(cuda_check(cudaStreamWaitEvent(c->stream, lane.done, 0), "join"));
     }
+    for (size_t j = 0; j < nj; j++)
+        if (rc >= 0 && wavefront((uint32_t)j)) trace((uint32_t)j, c->stream, true);
     return rc;
 }
 
@@ -2201,6 +2225,14 @@ void batch_mark_traced(phx_batch b) {
         bj.tr->frame = bj.first + bj.spp - 1;
         bj.tr->last = bj.cam;
         bj.tr->have_last = true;
+    }
+}
+
+// The side streams' buffers given back (no graph may hold them).
+void release_lanes(phx_batch b) {
+    for (auto& lane : b->lanes) {
+        lane.path_pool.state.release();
+        lane.path_pool.out.release();
     }
 }
 
@@ -2253,6 +2285,7 @@ int32_t phx_batch_clear(phx_batch b) {
     b->net_of.clear();
     b->jobs.clear();
     b->ntiles = 0;
+    release_lanes(b);
     return PHX_OK;
 }
 
@@ -2295,6 +2328,7 @@ int32_t phx_batch_set_config(phx_batch b, uint32_t kind, uint32_t threads, uint3
     if (threads != 64 && threads != 128 && threads != 256) return fail(PHX_ERR_INVALID, "block size %u", threads);
     if (stack > PHX_STACK_SHARED) return fail(PHX_ERR_INVALID, "stack placement %u", stack);
     batch_drop_graph(b);
+    if (kind != PHX_BATCH_PER_SCENE) release_lanes(b);
     b->kind = kind;
     b->threads = threads;
     b->stack = stack;
@@ -2316,6 +2350,7 @@ int32_t phx_batch_autotune(phx_batch b, uint32_t* kind, uint32_t* threads, uint3
     if (!b) return fail(PHX_ERR_INVALID, "null batch");
     if (b->jobs.empty()) return fail(PHX_ERR_INVALID, "empty batch");
     PHX_TRY(use(b->ctx));
+    batch_drop_graph(b);  // the trials size the side streams' buffers
     struct Cfg {
         uint32_t kind, threads, stack, tracer_kernel;
     };
@@ -2363,7 +2398,7 @@ int32_t phx_batch_autotune(phx_batch b, uint32_t* kind, uint32_t* threads, uint3
     for (size_t j = 0; j < b->jobs.size(); j++)
         b->jobs[j].tr->kernel = cfgs[pick].kind == PHX_BATCH_PER_SCENE ? cfgs[pick].tracer_kernel : saved[j];
     PHX_TRY(rc);
-    batch_drop_graph(b);
+    if (cfgs[pick].kind != PHX_BATCH_PER_SCENE || !pooled_id(cfgs[pick].tracer_kernel)) release_lanes(b);
     b->kind = cfgs[pick].kind;
     b->threads = cfgs[pick].threads;
     b->stack = cfgs[pick].stack;

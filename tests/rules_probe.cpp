@@ -2,3 +2,31 @@
 #include "../phiray_b200/csrc/rules.cuh"
 
 extern "C" int probe_aligned16(const void* p) { return phx::aligned16(p) ? 1 : 0; }
+
+// The id of the kernel that traces a frame, and (bit 31) whether it needs the
+// pooled render's buffers. flags: full, adaptive, transmits, capturing.
+extern "C" uint32_t probe_frame_kernel(uint32_t kernel, uint32_t flags) {
+    const phx::FrameForm f{kernel, (flags & 1u) != 0, (flags & 2u) != 0, (flags & 4u) != 0, (flags & 8u) != 0};
+    return phx::frame_kernel(f) | (phx::frame_pooled(f) ? 0x80000000u : 0u);
+}
+
+// plan_lanes over n jobs of (work, pooled, state, out); the reserve calls are
+// written to calls as (lane, state, out), and call `fails` (from 0) fails.
+// Returns the number of calls.
+extern "C" uint32_t probe_lanes(const uint64_t* jobs, uint32_t n, uint32_t lanes, uint32_t fails, uint64_t* calls,
+                                uint32_t* order, uint32_t* lane, uint8_t* buffers) {
+    std::vector<phx::LaneJob> in;
+    for (uint32_t j = 0; j < n; j++)
+        in.push_back({jobs[4 * j], jobs[4 * j + 1] != 0, (size_t)jobs[4 * j + 2], (size_t)jobs[4 * j + 3]});
+    uint32_t made = 0;
+    const phx::LanePlan p = phx::plan_lanes(in, lanes, [&](uint32_t l, size_t state, size_t out) {
+        calls[3 * made] = l;
+        calls[3 * made + 1] = state;
+        calls[3 * made + 2] = out;
+        return made++ != fails;
+    });
+    std::copy(p.order.begin(), p.order.end(), order);
+    std::copy(p.lane.begin(), p.lane.end(), lane);
+    std::copy(p.buffers.begin(), p.buffers.end(), buffers);
+    return made;
+}

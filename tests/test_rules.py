@@ -5,7 +5,10 @@ import ctypes as C
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
+
+from phiray_b200.tracer import Tracer
 
 HERE = Path(__file__).resolve().parent
 
@@ -22,3 +25,56 @@ def test_wide_accesses_only_at_their_alignment(rules):
     rules.probe_aligned16.argtypes = [C.c_void_p]
     for p in range(0x7F0000000000, 0x7F0000000000 + 64):
         assert rules.probe_aligned16(p) == (p % 16 == 0)
+
+
+FULL, ADAPTIVE, TRANSMITS, CAPTURING = 1, 2, 4, 8
+POOLED = (Tracer.STATE_MACHINE, Tracer.STATE_MACHINE_6, Tracer.STATE_MACHINE_8)
+UNSET = 0xFFFFFFFF
+
+
+@pytest.mark.parametrize("flags", range(16))
+def test_every_frame_has_a_kernel_that_can_trace_it(rules, flags):
+    rules.probe_frame_kernel.restype = C.c_uint32
+    for kernel in [*range(20), UNSET]:
+        r = rules.probe_frame_kernel(C.c_uint32(kernel), flags)
+        got, buffers = r & 0x7FFFFFFF, bool(r >> 31)
+        wavefront_can = not flags & (ADAPTIVE | CAPTURING)
+        pooled_can = not flags & ADAPTIVE and (flags & FULL or not flags & TRANSMITS)
+        if kernel == UNSET:
+            want = Tracer.STATE_MACHINE if pooled_can and not flags & FULL else Tracer.MEGAKERNEL
+        elif kernel == Tracer.WAVEFRONT and not wavefront_can or kernel in POOLED and not pooled_can:
+            want = Tracer.MEGAKERNEL
+        else:
+            want = kernel
+        assert got == want
+        assert buffers == (got in POOLED and not flags & FULL)
+
+
+@pytest.mark.parametrize("fails", [0, 1, 2, 99])
+@pytest.mark.parametrize("seed", range(6))
+def test_lanes_reserve_once_for_their_pooled_jobs(rules, seed, fails):
+    """A lane's buffers are asked for once, before its first launch, for the
+    largest need of its pooled jobs; where that fails none of its jobs has any."""
+    rng = np.random.default_rng(seed)
+    n, lanes = int(rng.integers(1, 12)), 3
+    jobs = np.zeros((n, 4), np.uint64)
+    jobs[:, 0] = rng.integers(1, 1000, n)
+    jobs[:, 1] = rng.integers(0, 2, n) if seed else 0  # (seed 0: none runs pooled)
+    # the larger job need not be the one with the larger buffers
+    jobs[:, 2:] = rng.integers(1, 1000, (n, 2))
+    calls, order, lane = np.zeros((8, 3), np.uint64), np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+    buffers = np.zeros(n, np.uint8)
+    made = rules.probe_lanes(*(a.ctypes.data_as(C.c_void_p) if isinstance(a, np.ndarray) else a
+                               for a in (jobs, n, lanes, fails, calls, order, lane, buffers)))
+    assert sorted(order) == list(range(n)) and (np.diff(jobs[order, 0].astype(int)) <= 0).all()
+    assert (lane < lanes).all()
+    calls = calls[:made]
+    assert len(set(calls[:, 0])) == made  # once a lane
+    for k in range(lanes):
+        mine = (lane == k) & (jobs[:, 1] != 0)
+        at = np.flatnonzero(calls[:, 0] == k)
+        assert len(at) == int(mine.any())
+        if mine.any():
+            assert (calls[at[0], 1:] == jobs[mine, 2:].max(0)).all()
+            assert (buffers[mine] == (at[0] != fails)).all()
+    assert not buffers[jobs[:, 1] == 0].any()
