@@ -443,8 +443,8 @@ int32_t phx_tracer_destroy(phx_tracer tr);
  * paths in device memory and alternates between tracing all of their rays
  * and shading all of their hits by kind. It runs single-instance scenes whose
  * materials transmit no light, not inside a graph capture (but for a batch's
- * own) nor with adaptive sampling; PHX_KERNEL_MEGAKERNEL runs the other
- * frames. Scenes of instances and frames with the floor grid take a
+ * own) nor with adaptive sampling; the other frames run on the megakernel
+ * form an autotuning found fastest, or PHX_KERNEL_MEGAKERNEL. Scenes of instances and frames with the floor grid take a
  * persistent kernel under these ids, whose lanes take pixels from a counter
  * and run the bounce loop as a state machine around one walk.
  * phx_tracer_autotune times them on the scene and keeps the fastest. */
@@ -477,7 +477,7 @@ int32_t phx_tracer_destroy(phx_tracer tr);
  * (primary, extension, shadow) with ballot compaction, each queue walked by a
  * kernel of its own (closest or any hit) between passes of the shading
  * logic; the host polls the queues every fourth pass. Not inside a graph
- * capture nor with adaptive sampling (the megakernel runs those frames). */
+ * capture nor with adaptive sampling (a megakernel runs those frames). */
 #define PHX_KERNEL_WAVEFRONT 16u
 /* The megakernel whose walk keeps the top of its 32-entry stack in
  * registers (older entries spill to local memory, a pop refilling the
@@ -492,7 +492,8 @@ int32_t phx_tracer_destroy(phx_tracer tr);
 int32_t phx_tracer_set_kernel(phx_tracer tr, uint32_t kernel);
 /* The autotuner: times every render kernel (and register budget) above on
  * `spp` samples of this scene and camera, keeps the fastest for the tracer
- * and returns its id; ms (PHX_KERNEL_COUNT floats, may be NULL) gets each one's time. The
+ * (and the fastest megakernel form for frames that one cannot trace) and
+ * returns its id; ms (PHX_KERNEL_COUNT floats, may be NULL) gets each one's time. The
  * image is overwritten (the next sample starts over). Waits. */
 int32_t phx_tracer_autotune(phx_tracer tr, const phx_camera* cam, uint32_t w, uint32_t h, uint32_t spp,
                             uint32_t* chosen, float* ms);

@@ -24,6 +24,7 @@ constexpr uint32_t KERNEL_UNSET = 0xFFFFFFFFu;
 // What a frame asks of the kernel that traces it.
 struct FrameForm {
     uint32_t kernel;  // the tracer's (set or autotuned, or KERNEL_UNSET)
+    uint32_t mega;    // its megakernel form for frames that `kernel` cannot trace
     bool full;        // instances, or the floor grid
     bool adaptive;
     bool transmits;   // some material transmits light
@@ -32,6 +33,17 @@ struct FrameForm {
 
 inline bool pooled_id(uint32_t kernel) {
     return kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8;
+}
+
+// The fastest megakernel form by the times of an autotuning: what a tracer
+// whose fastest kernel is another one traces adaptive frames, recorded ones and
+// those without memory for the pools with. (The 1.3 M-face mesh at 1080p, 16
+// spp: 46 ms in the 16-block form, 57 in the 4-block one.)
+inline uint32_t fastest_megakernel(const float* ms) {
+    uint32_t best = PHX_KERNEL_MEGAKERNEL;
+    for (uint32_t k = 0; k < PHX_KERNEL_COUNT; k++)
+        if (!pooled_id(k) && k != PHX_KERNEL_WAVEFRONT && ms[k] < ms[best]) best = k;
+    return best;
 }
 
 // The id of the kernel that traces the frame. The default is the pooled render
@@ -45,9 +57,9 @@ inline bool pooled_id(uint32_t kernel) {
 // between passes, which a recorded graph cannot.
 inline uint32_t frame_kernel(const FrameForm& f) {
     uint32_t k = f.kernel;
-    if (k == KERNEL_UNSET) k = f.full ? PHX_KERNEL_MEGAKERNEL : PHX_KERNEL_STATE_MACHINE;
-    if (k == PHX_KERNEL_WAVEFRONT && (f.adaptive || f.capturing)) return PHX_KERNEL_MEGAKERNEL;
-    if (pooled_id(k) && (f.adaptive || (f.transmits && !f.full))) return PHX_KERNEL_MEGAKERNEL;
+    if (k == KERNEL_UNSET) k = f.full ? f.mega : PHX_KERNEL_STATE_MACHINE;
+    if (k == PHX_KERNEL_WAVEFRONT && (f.adaptive || f.capturing)) return f.mega;
+    if (pooled_id(k) && (f.adaptive || (f.transmits && !f.full))) return f.mega;
     return k;
 }
 

@@ -716,6 +716,7 @@ struct phx_tracer_s {
     uint32_t w = 0, h = 0;
     uint32_t frame = 0, target = 32;  // Tracer::SAMPLE_COUNT (src/trace/mod.rs:129) until set_samples
     uint32_t kernel = KERNEL_UNSET;  // which render kernel traces a frame (set or autotuned)
+    uint32_t mega = PHX_KERNEL_MEGAKERNEL;  // the megakernel form (autotuned) of frames that one cannot trace
     DevMem next;                                 // the pooled and state-machine kernels' work counter
     uint32_t stack_place = PHX_STACK_LOCAL;      // where thread-per-ray walks keep their stack
     uint32_t walk = PHX_WALK_THREAD;             // ray walks: a thread per ray, persistent warps, sorted first
@@ -1175,7 +1176,7 @@ int32_t ensure_wide(phx_tracer tr) {
 }
 
 FrameForm form_of(phx_tracer tr, const Frame& F, bool capturing) {
-    return FrameForm{tr->kernel, tr->forest || F.grid > 0.0f, F.adapt_on != 0u, tr->transmits, capturing};
+    return FrameForm{tr->kernel, tr->mega, tr->forest || F.grid > 0.0f, F.adapt_on != 0u, tr->transmits, capturing};
 }
 
 int32_t capturing(cudaStream_t s, bool& on) {
@@ -1218,7 +1219,7 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
     if (!pooled_id(kernel)) return launch_megakernel(kernel, stats, L);
     // The pooled render's buffers are the context's, which a recorded graph
     // must not hold (they may grow before it is replayed). There, and where
-    // there is no memory for them, the 4-block megakernel.
+    // there is no memory for them, a megakernel.
     if (count_px && !recorded) {
         const PoolNeed need = pool_need(c, count_px, F.spp);
         std::lock_guard<std::mutex> lock(c->path_pool_lock);
@@ -1227,7 +1228,7 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
         if (rc >= 0) return render_pooled(kernel, stats, L, pool_buffers(c->path_pool, need));
         if (rc != PHX_ERR_OOM) return rc;
     }
-    return launch_megakernel(PHX_KERNEL_MEGAKERNEL, stats, L);
+    return launch_megakernel(tr->mega, stats, L);
 }
 
 // A frame of a batch on a side stream, with the side stream's buffers for the
@@ -1239,7 +1240,7 @@ int32_t launch_frame_on(cudaStream_t s, const PoolBuffers* buffers, phx_tracer t
     if (form.full) return render_full(kernel, false, L);
     if (!pooled_id(kernel)) return launch_megakernel(kernel, false, L);
     if (buffers) return render_pooled(kernel, false, L, *buffers);
-    return launch_megakernel(PHX_KERNEL_MEGAKERNEL, false, L);
+    return launch_megakernel(tr->mega, false, L);
 }
 
 // The frame record of `cam` for tr, whose lights the kernels read from tr->cam.
@@ -1610,9 +1611,8 @@ int32_t phx_tracer_autotune(phx_tracer tr, const phx_camera* cam, uint32_t w, ui
     PHX_TRY(use(tr->ctx));
     PHX_TRY(ensure_image(tr, w, h));
     Ctx* c = tr->ctx;
-    float best = 0.0f;
-    uint32_t pick = PHX_KERNEL_STATE_MACHINE;
-    const uint32_t keep = tr->kernel;
+    float all[PHX_KERNEL_COUNT] = {};
+    uint32_t pick = 0;
     for (uint32_t k = 0; k < PHX_KERNEL_COUNT; k++) {
         tr->kernel = k;
         PHX_TRY(launch_render(tr, cam, w, h, 0, spp ? spp : 1, 0, w * h));  // warm-up
@@ -1620,16 +1620,12 @@ int32_t phx_tracer_autotune(phx_tracer tr, const phx_camera* cam, uint32_t w, ui
         PHX_TRY(launch_render(tr, cam, w, h, 0, spp ? spp : 1, 0, w * h));
         PHX_CUDA(cudaEventRecord(tr->ev1, c->stream));
         PHX_TRY(wait_stream(c->stream, 60000));
-        float t = 0.0f;
-        PHX_CUDA(cudaEventElapsedTime(&t, tr->ev0, tr->ev1));
-        if (ms) ms[k] = t;
-        if (k == 0 || t < best) {
-            best = t;
-            pick = k;
-        }
+        PHX_CUDA(cudaEventElapsedTime(&all[k], tr->ev0, tr->ev1));
+        if (all[k] < all[pick]) pick = k;
     }
     tr->kernel = pick;
-    (void)keep;
+    tr->mega = fastest_megakernel(all);
+    if (ms) std::memcpy(ms, all, sizeof all);
     tr->have_last = false;  // the image holds the tuning frames: start over
     if (chosen) *chosen = pick;
     return read_status(c);
@@ -2370,8 +2366,9 @@ int32_t phx_batch_autotune(phx_batch b, uint32_t* kind, uint32_t* threads, uint3
         cudaEventDestroy(e0);
         return fail(PHX_ERR_DEVICE, "event create");
     }
-    float best = 3.0e38f;
+    float best = 3.0e38f, mega_best = 3.0e38f;
     size_t pick = 0;
+    uint32_t mega = PHX_KERNEL_MEGAKERNEL;
     int32_t rc = PHX_OK;
     for (size_t k = 0; k < cfgs.size() && rc == PHX_OK; k++) {
         const Cfg& cf = cfgs[k];
@@ -2392,11 +2389,18 @@ int32_t phx_batch_autotune(phx_batch b, uint32_t* kind, uint32_t* threads, uint3
             best = t;
             pick = k;
         }
+        if (cf.kind == PHX_BATCH_PER_SCENE && !pooled_id(cf.tracer_kernel) && t < mega_best) {
+            mega_best = t;
+            mega = cf.tracer_kernel;
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    for (size_t j = 0; j < b->jobs.size(); j++)
-        b->jobs[j].tr->kernel = cfgs[pick].kind == PHX_BATCH_PER_SCENE ? cfgs[pick].tracer_kernel : saved[j];
+    const bool per_scene = cfgs[pick].kind == PHX_BATCH_PER_SCENE;
+    for (size_t j = 0; j < b->jobs.size(); j++) {
+        b->jobs[j].tr->kernel = per_scene ? cfgs[pick].tracer_kernel : saved[j];
+        if (per_scene && rc >= 0) b->jobs[j].tr->mega = mega;
+    }
     PHX_TRY(rc);
     if (cfgs[pick].kind != PHX_BATCH_PER_SCENE || !pooled_id(cfgs[pick].tracer_kernel)) release_lanes(b);
     b->kind = cfgs[pick].kind;

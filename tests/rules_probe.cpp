@@ -3,10 +3,12 @@
 
 extern "C" int probe_aligned16(const void* p) { return phx::aligned16(p) ? 1 : 0; }
 
+extern "C" uint32_t probe_fastest_megakernel(const float* ms) { return phx::fastest_megakernel(ms); }
+
 // The id of the kernel that traces a frame, and (bit 31) whether it needs the
 // pooled render's buffers. flags: full, adaptive, transmits, capturing.
-extern "C" uint32_t probe_frame_kernel(uint32_t kernel, uint32_t flags) {
-    const phx::FrameForm f{kernel, (flags & 1u) != 0, (flags & 2u) != 0, (flags & 4u) != 0, (flags & 8u) != 0};
+extern "C" uint32_t probe_frame_kernel(uint32_t kernel, uint32_t mega, uint32_t flags) {
+    const phx::FrameForm f{kernel, mega, (flags & 1u) != 0, (flags & 2u) != 0, (flags & 4u) != 0, (flags & 8u) != 0};
     return phx::frame_kernel(f) | (phx::frame_pooled(f) ? 0x80000000u : 0u);
 }
 

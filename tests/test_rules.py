@@ -32,22 +32,35 @@ POOLED = (Tracer.STATE_MACHINE, Tracer.STATE_MACHINE_6, Tracer.STATE_MACHINE_8)
 UNSET = 0xFFFFFFFF
 
 
+@pytest.mark.parametrize("mega", [Tracer.MEGAKERNEL, Tracer.MEGAKERNEL_16_SYNC])
 @pytest.mark.parametrize("flags", range(16))
-def test_every_frame_has_a_kernel_that_can_trace_it(rules, flags):
+def test_every_frame_has_a_kernel_that_can_trace_it(rules, flags, mega):
     rules.probe_frame_kernel.restype = C.c_uint32
-    for kernel in [*range(20), UNSET]:
-        r = rules.probe_frame_kernel(C.c_uint32(kernel), flags)
+    for kernel in [*range(Tracer.KERNELS), UNSET]:
+        r = rules.probe_frame_kernel(C.c_uint32(kernel), mega, flags)
         got, buffers = r & 0x7FFFFFFF, bool(r >> 31)
         wavefront_can = not flags & (ADAPTIVE | CAPTURING)
         pooled_can = not flags & ADAPTIVE and (flags & FULL or not flags & TRANSMITS)
         if kernel == UNSET:
-            want = Tracer.STATE_MACHINE if pooled_can and not flags & FULL else Tracer.MEGAKERNEL
+            want = Tracer.STATE_MACHINE if pooled_can and not flags & FULL else mega
         elif kernel == Tracer.WAVEFRONT and not wavefront_can or kernel in POOLED and not pooled_can:
-            want = Tracer.MEGAKERNEL
+            want = mega
         else:
             want = kernel
         assert got == want
         assert buffers == (got in POOLED and not flags & FULL)
+
+
+def test_autotuning_keeps_the_fastest_megakernel_beside_its_pick(rules):
+    """A tracer whose fastest kernel is the pooled render traces its adaptive
+    frames with the fastest megakernel form, not with the 4-block one."""
+    rng = np.random.default_rng(5)
+    others = {*POOLED, Tracer.WAVEFRONT}
+    for _ in range(50):
+        ms = rng.uniform(1.0, 9.0, Tracer.KERNELS).astype(np.float32)
+        ms[list(others)] -= 5.0
+        got = rules.probe_fastest_megakernel(ms.ctypes.data_as(C.c_void_p))
+        assert got not in others and ms[got] == min(ms[k] for k in range(Tracer.KERNELS) if k not in others)
 
 
 @pytest.mark.parametrize("fails", [0, 1, 2, 99])
