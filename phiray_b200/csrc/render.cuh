@@ -11,6 +11,7 @@
 #include <cstddef>
 #include <cstring>
 
+#include "rules.cuh"
 #include "shade.cuh"
 
 namespace phx {
@@ -42,19 +43,10 @@ struct WfBuffers {
     uint32_t* host_lens;  // pinned, 3 words
 };
 
-// The pooled render's buffers (render_pool.cuh): the state of `slots` paths,
-// and the terms of `spp` samples of every pixel of the launch.
-struct PoolBuffers {
-    uint32_t* pools;
-    uint64_t slots;
-    uint32_t* out;
-    uint32_t spp;
-};
-// Bytes of one path's state; words of one sample's terms.
-size_t pool_slot_bytes();
-uint32_t pool_out_words();
-// The pooled render, by kernel id 1-3 (render_pool.cu).
-int32_t render_pooled(uint32_t kernel, bool stats, const RenderLaunch& L, const PoolBuffers& B);
+// The pooled render by kernel id 1-3 (render_pool.cu): a frame's plan, and its
+// launch over buffers of the plan's sizes (the paths' states, the samples' terms).
+int32_t plan_pooled(uint32_t kernel, bool stats, int sms, uint32_t count, uint32_t spp, PoolPlan& plan);
+int32_t render_pooled(uint32_t kernel, bool stats, const RenderLaunch& L, const PoolPlan& plan, void* state, void* out);
 
 constexpr uint32_t WF_SLOTS = 1u << 20;  // path slots of the wavefront render (at most)
 // 32-bit words of one wavefront path slot (Path, Sums, phase).
@@ -62,7 +54,7 @@ uint32_t wf_slot_words();
 
 // The single-instance render kernels by id: ids 0 and 4-8 (render_flat_a.cu),
 // 9-12 (render_flat_b.cu), 13-15 (render_flat_c.cu), 17-19 (render_flat_r.cu);
-// 1-3 are render_pooled below.
+// 1-3 are render_pooled above.
 int32_t render_flat_a(uint32_t kernel, bool stats, const RenderLaunch& L);
 int32_t render_flat_b(uint32_t kernel, bool stats, const RenderLaunch& L);
 int32_t render_flat_c(uint32_t kernel, bool stats, const RenderLaunch& L);

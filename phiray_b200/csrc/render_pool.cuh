@@ -42,8 +42,9 @@
 namespace phx {
 namespace {
 
-// Words of a path's state, one after another for all of a pool's slots
-// (word k of slot s at st[k * P + s]).
+// Words of a path's state. A pool's slots lie in groups of 32, a group's words
+// one after another for its slots (Pool::w), so that a pool takes the memory of
+// the slots it uses.
 enum : uint32_t {
     PW_SEED = 0,
     PW_PIX,       // pixel
@@ -82,11 +83,6 @@ constexpr uint32_t RAY_SLOT = 4095u;
 constexpr uint32_t RAY_KIND = 12;  // bits 12-13: 0 the path's ray, 1-3 shadow ray k - 1
 constexpr uint32_t RAY_AO = 1u << 14;  // the path's ray is an any-hit ray of range F.ao
 
-// Fills of a pool a frame is cut into at least (fewer slots, so that a small
-// frame's last paths do not leave most of a pool empty, against fewer and
-// larger phases): the cloud above took 7.0, 4.9, 5.0, 5.3 and 6.3 ms at 1, 2,
-// 3, 4 and 8 fills.
-constexpr uint32_t POOL_FILLS = 2;
 constexpr int POOL_STEPS = 6;    // node visits between looks at the warp's other lanes (2: 29.9 ms, 4: 28.1, 6: 28.0)
 constexpr int POOL_REFILL = 12;  // idle lanes that make a refill (8: 28.4 ms, 12: 28.1)
 // A leaf's triangles are tested once this share of the lanes that hold an
@@ -117,10 +113,12 @@ struct Pool {
     PoolShared<P>* sh;
     uint32_t lane;
 
-    __device__ __forceinline__ uint32_t& w(uint32_t k, uint32_t s) const { return st[k * P + s]; }
-    __device__ __forceinline__ float f(uint32_t k, uint32_t s) const { return __uint_as_float(st[k * P + s]); }
+    __device__ __forceinline__ uint32_t& w(uint32_t k, uint32_t s) const {
+        return st[(s >> 5) * (PW_WORDS * 32u) + (s & 31u) + k * 32u];
+    }
+    __device__ __forceinline__ float f(uint32_t k, uint32_t s) const { return __uint_as_float(w(k, s)); }
     __device__ __forceinline__ f3 f3at(uint32_t k, uint32_t s) const { return mk(f(k, s), f(k + 1, s), f(k + 2, s)); }
-    __device__ __forceinline__ void put(uint32_t k, uint32_t s, float v) const { st[k * P + s] = __float_as_uint(v); }
+    __device__ __forceinline__ void put(uint32_t k, uint32_t s, float v) const { w(k, s) = __float_as_uint(v); }
     __device__ __forceinline__ void put(uint32_t k, uint32_t s, f3 v) const {
         put(k, s, v.x);
         put(k + 1, s, v.y);
@@ -768,7 +766,7 @@ __global__ void __launch_bounds__(T, MINB) k_render_pool(const __grid_constant__
     }
     const Scene& S = sh.S;
     const Frame& F = sh.F;
-    const Pool<P> pool{pools + (size_t)blockIdx.x * PW_WORDS * P, &sh, threadIdx.x & 31u};
+    const Pool<P> pool{pools + (size_t)blockIdx.x * PW_WORDS * slots, &sh, threadIdx.x & 31u};
     for (uint32_t s = threadIdx.x; s < P; s += T) sh.stage[s] = s < slots ? ST_FREE : ST_UNUSED;
     __syncthreads();
     Count cnt{0, 0, 0};
@@ -827,32 +825,36 @@ __global__ void __launch_bounds__(128) k_pool_resolve(Frame F, PoolFrame J, uint
     store_sums(px, F.n, i, F.frame0 == 0u, acc, F);
 }
 
+// The host's side of one form: its plan of a frame, and the frame's launches.
 template <int M, int MINB, int P, int T>
-int32_t launch_pool(const RenderLaunch& L, const PoolBuffers& B) {
-    auto kernel = k_render_pool<M, MINB, P, T>;
-    constexpr int smem = (int)sizeof(PoolShared<P>);
-    int per_sm = 0;
-    PHX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, T, smem));
-    uint32_t blocks = (uint32_t)std::max(per_sm, 1) * (uint32_t)L.sms;
-    blocks = std::min<uint32_t>(blocks, (uint32_t)(B.slots / P));
-    RenderLaunch R = L;
-    uint32_t left = L.F.spp;
-    while (left) {
-        PoolFrame J{L.first, L.count, std::min(left, B.spp), PoolOut{B.out, (uint64_t)L.count * B.spp}};
-        R.F.spp = J.spp;
-        // several fills of every pool: a small frame's last paths would
-        // otherwise end with most slots empty, or on a few blocks
-        const uint64_t share = (uint64_t)L.count * J.spp / blocks / POOL_FILLS / 32u * 32u;
-        const uint32_t slots = (uint32_t)std::min<uint64_t>(P, std::max<uint64_t>(share, 32u));
-        PHX_CUDA(cudaMemsetAsync(L.next, 0, 4, L.s));
-        kernel<<<blocks, T, smem, L.s>>>(L.S, R.F, L.sun, J, slots, B.pools, L.next, L.counters);
-        k_pool_resolve<<<(L.count + 127) / 128, 128, 0, L.s>>>(R.F, J, L.px);
-        left -= J.spp;
-        R.F.frame0 += J.spp;
+struct PoolForm {
+    static constexpr int SMEM = (int)sizeof(PoolShared<P>);
+
+    int32_t plan(int sms, uint32_t count, uint32_t spp, PoolPlan& p) const {
+        auto kernel = k_render_pool<M, MINB, P, T>;
+        int per_sm = 0;
+        PHX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, T, SMEM));
+        p = pool_plan(count, spp, (uint32_t)std::max(per_sm, 1) * (uint32_t)sms, P, PW_WORDS * 4, PO_WORDS * 4);
+        return PHX_OK;
     }
-    return cuda_check(cudaGetLastError(), "pooled render");
-}
+
+    int32_t launch(const RenderLaunch& L, const PoolPlan& p, uint32_t* state, uint32_t* out) const {
+        RenderLaunch R = L;
+        uint32_t left = L.F.spp;
+        while (left) {
+            PoolFrame J{L.first, L.count, std::min(left, p.spp), PoolOut{out, (uint64_t)L.count * p.spp}};
+            R.F.spp = J.spp;
+            const uint32_t slots = pool_slots((uint64_t)L.count * J.spp, p.blocks, P);
+            PHX_CUDA(cudaMemsetAsync(L.next, 0, 4, L.s));
+            k_render_pool<M, MINB, P, T><<<p.blocks, T, SMEM, L.s>>>(L.S, R.F, L.sun, J, slots, state, L.next, L.counters);
+            k_pool_resolve<<<(L.count + 127) / 128, 128, 0, L.s>>>(R.F, J, L.px);
+            left -= J.spp;
+            R.F.frame0 += J.spp;
+        }
+        return cuda_check(cudaGetLastError(), "pooled render");
+    }
+};
 
 }  // namespace
 }  // namespace phx

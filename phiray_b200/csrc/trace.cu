@@ -1121,35 +1121,6 @@ int32_t wf_buffers(phx_tracer tr, uint32_t count, WfBuffers& B) {
     return PHX_OK;
 }
 
-// The pooled render's buffers for `count` pixels and `spp` samples, out of
-// `scratch`: 8,192 path slots an SM (240 bytes each), and the terms of as
-// many samples as POOL_OUT_BYTES hold (one at least; the rest of the samples
-// run in further launches).
-constexpr size_t POOL_OUT_BYTES = (size_t)1 << 30;
-constexpr uint64_t POOL_SM_SLOTS = 8192;
-
-struct PoolNeed {
-    uint64_t slots;
-    uint32_t spp;
-    size_t state, out;  // bytes
-};
-
-PoolNeed pool_need(Ctx* c, uint32_t count, uint32_t spp) {
-    PoolNeed p;
-    const size_t sample = (size_t)count * pool_out_words() * 4;
-    const uint32_t fit = (uint32_t)std::max<size_t>(POOL_OUT_BYTES / sample, 1);
-    const uint32_t launches = (spp + fit - 1) / fit;
-    p.slots = (uint64_t)c->sms * POOL_SM_SLOTS;
-    p.spp = (spp + launches - 1) / launches;
-    p.state = p.slots * pool_slot_bytes();
-    p.out = sample * p.spp;
-    return p;
-}
-
-PoolBuffers pool_buffers(const PoolScratch& scratch, const PoolNeed& p) {
-    return PoolBuffers{(uint32_t*)scratch.state.ptr, p.slots, (uint32_t*)scratch.out.ptr, p.spp};
-}
-
 // The wide tree of the binary tree the tracer walks now (collapsed on the
 // device when the tree changed since the last collapse; waits).
 int32_t ensure_wide(phx_tracer tr) {
@@ -1221,11 +1192,12 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
     // must not hold (they may grow before it is replayed). There, and where
     // there is no memory for them, a megakernel.
     if (count_px && !recorded) {
-        const PoolNeed need = pool_need(c, count_px, F.spp);
+        PoolPlan plan;
+        PHX_TRY(plan_pooled(kernel, stats, c->sms, count_px, F.spp, plan));
         std::lock_guard<std::mutex> lock(c->path_pool_lock);
-        int32_t rc = c->path_pool.state.reserve(need.state);
-        if (rc >= 0) rc = c->path_pool.out.reserve(need.out);
-        if (rc >= 0) return render_pooled(kernel, stats, L, pool_buffers(c->path_pool, need));
+        int32_t rc = c->path_pool.state.reserve(plan.state);
+        if (rc >= 0) rc = c->path_pool.out.reserve(plan.out);
+        if (rc >= 0) return render_pooled(kernel, stats, L, plan, c->path_pool.state.ptr, c->path_pool.out.ptr);
         if (rc != PHX_ERR_OOM) return rc;
     }
     return launch_megakernel(tr->mega, stats, L);
@@ -1233,13 +1205,14 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
 
 // A frame of a batch on a side stream, with the side stream's buffers for the
 // pooled render, or null: nothing is allocated here. (Not the wavefront.)
-int32_t launch_frame_on(cudaStream_t s, const PoolBuffers* buffers, phx_tracer tr, const Frame& F, f3 sun) {
+int32_t launch_frame_on(cudaStream_t s, const PoolPlan& plan, const PoolScratch* buffers, phx_tracer tr, const Frame& F,
+                        f3 sun) {
     const FrameForm form = form_of(tr, F, true);
     const uint32_t kernel = frame_kernel(form);
     const RenderLaunch L = launch_of(tr, F, sun, 0, F.n, s);
     if (form.full) return render_full(kernel, false, L);
     if (!pooled_id(kernel)) return launch_megakernel(kernel, false, L);
-    if (buffers) return render_pooled(kernel, false, L, *buffers);
+    if (buffers) return render_pooled(kernel, false, L, plan, buffers->state.ptr, buffers->out.ptr);
     return launch_megakernel(tr->mega, false, L);
 }
 
@@ -1345,6 +1318,7 @@ int32_t create_tracer(phx_ctx ctx, const phx_scene* sc, const phx_mesh* meshes, 
     tr->leaf = sc->leaf ? sc->leaf : 4;
     tr->has_normals = sc->normals != nullptr;
     ctx->c.live++;
+    ctx->c.tracers++;
     cudaStream_t s = ctx->c.stream;
     const size_t n = sc->nfaces;
     int32_t rc = PHX_OK;
@@ -1592,8 +1566,14 @@ int32_t phx_tracer_destroy(phx_tracer tr) {
     if (tr->ev0) cudaEventDestroy(tr->ev0);
     if (tr->ev1) cudaEventDestroy(tr->ev1);
     if (tr->wf_host_lens) cudaFreeHost(tr->wf_host_lens);
-    tr->ctx->live--;
+    Ctx* c = tr->ctx;
+    c->live--;
     delete tr;
+    if (--c->tracers == 0) {  // nobody is left to use them
+        std::lock_guard<std::mutex> lock(c->path_pool_lock);
+        c->path_pool.state.release();
+        c->path_pool.out.release();
+    }
     return PHX_OK;
 }
 
@@ -2150,13 +2130,16 @@ int32_t trace_per_scene(phx_batch b) {
     PHX_TRY(capturing(c->stream, recorded));
     const size_t nj = b->jobs.size();
     std::vector<Frame> frames;
-    std::vector<PoolNeed> need;
+    std::vector<PoolPlan> pools;
     std::vector<LaneJob> jobs;
     for (const BatchJob& bj : b->jobs) {
-        frames.push_back(frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp));
-        need.push_back(pool_need(c, bj.w * bj.h, bj.spp));
-        jobs.push_back(LaneJob{(uint64_t)bj.w * bj.h * bj.spp, frame_pooled(form_of(bj.tr, frames.back(), recorded)),
-                               need.back().state, need.back().out});
+        const Frame F = frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp);
+        const FrameForm form = form_of(bj.tr, F, recorded);
+        PoolPlan p{};
+        if (frame_pooled(form)) PHX_TRY(plan_pooled(frame_kernel(form), false, c->sms, F.n, F.spp, p));
+        frames.push_back(F);
+        pools.push_back(p);
+        jobs.push_back(LaneJob{(uint64_t)F.n * F.spp, frame_pooled(form), p.state, p.out});
     }
     // A captured graph holds the buffers as they are, and a frame that is
     // recorded takes what the one before it reserved.
@@ -2181,8 +2164,7 @@ int32_t trace_per_scene(phx_batch b) {
         if (wavefront) {
             step(launch_frame(bj.tr, frames[j], sun, 0, frames[j].n, false));
         } else {
-            const PoolBuffers B = pool_buffers(lane.path_pool, need[j]);
-            step(launch_frame_on(s, plan.buffers[j] ? &B : nullptr, bj.tr, frames[j], sun));
+            step(launch_frame_on(s, pools[j], plan.buffers[j] ? &lane.path_pool : nullptr, bj.tr, frames[j], sun));
         }
         if (rc >= 0)
             step(cuda_check(cudaMemcpyAsync((unsigned long long*)b->counters.ptr + 3 * j, bj.tr->rays.ptr, 8,

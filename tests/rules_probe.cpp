@@ -32,3 +32,16 @@ extern "C" uint32_t probe_lanes(const uint64_t* jobs, uint32_t n, uint32_t lanes
     std::copy(p.buffers.begin(), p.buffers.end(), buffers);
     return made;
 }
+
+// pool_plan as (blocks, slots, spp, state, out), and the slots of a launch.
+extern "C" void probe_pool_plan(uint32_t count, uint32_t spp, uint32_t blocks, uint32_t most, uint64_t* plan) {
+    const phx::PoolPlan p = phx::pool_plan(count, spp, blocks, most, 244, 40);
+    plan[0] = p.blocks;
+    plan[1] = p.slots;
+    plan[2] = p.spp;
+    plan[3] = p.state;
+    plan[4] = p.out;
+}
+extern "C" uint32_t probe_pool_slots(uint64_t samples, uint32_t blocks, uint32_t most) {
+    return phx::pool_slots(samples, blocks, most);
+}

@@ -91,3 +91,25 @@ def test_lanes_reserve_once_for_their_pooled_jobs(rules, seed, fails):
             assert (calls[at[0], 1:] == jobs[mine, 2:].max(0)).all()
             assert (buffers[mine] == (at[0] != fails)).all()
     assert not buffers[jobs[:, 1] == 0].any()
+
+
+@pytest.mark.parametrize("count", [1, 33, 64 * 48, 256 * 256, 1920 * 1080, 120_000_000])
+@pytest.mark.parametrize("spp", [1, 3, 16, 64, 4000])
+@pytest.mark.parametrize("blocks,most", [(296, 4096), (592, 2048), (1184, 1024), (2, 4096)])
+def test_pooled_render_memory_follows_the_frame(rules, count, spp, blocks, most):
+    plan = (C.c_uint64 * 5)()
+    rules.probe_pool_plan(count, spp, blocks, most, plan)
+    got_blocks, slots, per, state, out = plan
+    assert got_blocks == blocks and 32 <= slots <= most and slots % 32 == 0
+    assert 1 <= per <= spp and out == count * per * 40
+    assert out <= max(1 << 30, count * 40)
+    # all blocks' slots, no more than the frame has paths (or a group of 32 each)
+    assert state == blocks * slots * 244
+    assert blocks * slots <= max(count * per, 32 * blocks)
+    left = spp
+    while left:  # no launch needs more slots than the plan holds
+        now = min(left, per)
+        rules.probe_pool_slots.argtypes = [C.c_uint64, C.c_uint32, C.c_uint32]
+        assert rules.probe_pool_slots(count * now, blocks, most) <= slots
+        left -= now
+    assert -(-spp // per) == -(-spp // min(max((1 << 30) // (count * 40), 1), spp))  # as many launches as it takes
