@@ -697,6 +697,11 @@ __global__ void __launch_bounds__(128, 4) k_conv_ws(const bf16* __restrict__ X, 
 // taps, a block each. The bias gradient is one more MMA with a B of ones. The
 // blocks' partial sums meet in dWt by fp32 atomics, consecutive lanes at
 // consecutive output channels.
+//
+// Where the image ends inside a tile, an MMA takes pixels past its edge with dY
+// = 0. At the taps left of and above them they meet the image's last column and
+// row of X, and 0 times a value that is not finite is NaN: such a sum is made
+// again over the image's pixels alone (wgrad_again). A finite one met none.
 struct WgradPlan {
     int n;             // input channels a block (the last chunk may hold fewer)
     int taps;          // 9 or 3
@@ -726,10 +731,36 @@ WgradPlan wgrad_plan(int cin, int cout) {
     return p;
 }
 
+// A block's part of one weight's gradient, over the pixels of its tiles `first`,
+// first + step, ..; the first product that is not finite is the answer.
+__device__ __forceinline__ float wgrad_again(const bf16* __restrict__ X, const bf16* __restrict__ dY, int dys, const Geo& g,
+                                          int tap, int ci, int co, int first, int step) {
+    const int tiles_x = (g.W + TX - 1) / TX, tiles_y = (g.H + TY - 1) / TY;
+    float sum = 0.0f;
+    for (int t = first; t < g.B * tiles_x * tiles_y; t += step) {
+        const int img = t / (tiles_x * tiles_y), y0 = (t / tiles_x) % tiles_y * TY, x0 = t % tiles_x * TX;
+        for (int y = y0; y < min(y0 + TY, g.H); y++) {
+            for (int x = x0; x < min(x0 + TX, g.W); x++) {
+                const int sy = y + tap / 3 - 1, sx = x + tap % 3 - 1;
+                if (sy < 0 || sy >= g.H || sx < 0 || sx >= g.W) continue;
+                const float d = __bfloat162float(dY[((size_t)(img * g.H + y) * g.W + x) * dys + co]);
+                const float v = d * __bfloat162float(X[((size_t)(img * g.H + sy) * g.W + sx) * g.xs + g.xo + ci]);
+                if (!isfinite(v)) return v;
+                sum += v;
+            }
+        }
+    }
+    return sum;
+}
+
 __host__ __device__ constexpr uint32_t instr_desc_mn(int N) {
     return tc::instr_desc_bf16(tc::BM, N) | (1u << 15) | (1u << 16);  // A and B MN-major
 }
 
+// RAGGED: the image ends inside a tile. The look at the sums costs these launches
+// up to 1.2 us (of 8 to 13); in one kernel for both it cost every launch 1.3 and
+// the 96-channel ones at full resolution 12 of 110.
+template <bool RAGGED>
 __global__ void __launch_bounds__(128) k_conv_wgrad(const bf16* __restrict__ X, const bf16* __restrict__ dY, int dys,
                                                     int dyo, float* __restrict__ dWt, float* __restrict__ db, Geo g,
                                                     WgradPlan pl, uint32_t* status) {
@@ -841,6 +872,26 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(const bf16* __restrict__ X, 
                 float v[16];
                 tc::tmem_ld16(row + (uint32_t)t * pl.acc + (uint32_t)c, v);
                 float* o = dWt + (size_t)((tap0 + t) * g.cin + c0 + c) * g.cout + m0 + co;
+                if (RAGGED) {
+                    float z = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 16; j++) z += v[j] * 0.0f;
+                    if (__any_sync(0xffffffffu, z != 0.0f)) {
+                        uint32_t odd = 0;
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            if (!isfinite(v[j])) odd |= 1u << j;
+                            else if (co < cm) atomicAdd(o + (size_t)j * g.cout, v[j]);
+                        }
+#pragma unroll 1
+                        for (; odd && co < cm; odd &= odd - 1u) {
+                            const int j = __ffs(odd) - 1;
+                            atomicAdd(o + (size_t)j * g.cout,
+                                      wgrad_again(X, dY, dys, g, tap0 + t, c0 + c + j, dyo + m0 + co, first, step));
+                        }
+                        continue;
+                    }
+                }
                 if (co < cm) {
 #pragma unroll
                     for (int j = 0; j < 16; j++) atomicAdd(o + (size_t)j * g.cout, v[j]);
@@ -1452,14 +1503,16 @@ int32_t conv_fwd_any(Ctx* c, const bf16* X, const bf16* W, const float* bias, vo
 // dWt (and db, unless null) += the gradients of one convolution.
 int32_t conv_wgrad(Ctx* c, const bf16* X, const bf16* dY, int dys, int dyo, float* dWt, float* db, const Geo& g) {
     const WgradPlan p = wgrad_plan(g.cin, g.cout);
-    static std::atomic<uint64_t> done{0};
-    PHX_TRY(smem_limit(k_conv_wgrad, 224 * 1024, c->device, done));
+    const bool ragged = g.W % TX || g.H % TY;
+    const auto kernel = ragged ? k_conv_wgrad<true> : k_conv_wgrad<false>;
+    static std::atomic<uint64_t> done[2];
+    PHX_TRY(smem_limit(kernel, 224 * 1024, c->device, done[ragged]));
     const int ntiles = g.B * ((g.H + TY - 1) / TY) * ((g.W + TX - 1) / TX);
     const int gy = 9 / p.taps * ((g.cin + p.n - 1) / p.n), gz = (g.cout + 127) / 128;
     // the tiles are split so that the blocks fill the SMs once (a block's
     // accumulators take most of an SM's TMEM)
     const int splits = std::max(1, std::min(ntiles, c->sms / (gy * gz)));
-    k_conv_wgrad<<<dim3(splits, gy, gz), 128, p.smem, c->stream>>>(X, dY, dys, dyo, dWt, db, g, p, c->status);
+    kernel<<<dim3(splits, gy, gz), 128, p.smem, c->stream>>>(X, dY, dys, dyo, dWt, db, g, p, c->status);
     return cuda_check(cudaGetLastError(), "conv wgrad");
 }
 
