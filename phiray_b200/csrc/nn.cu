@@ -9,6 +9,7 @@
 #include <atomic>
 
 #include "../../include/phiray_math.h"
+#include "conv_index.cuh"
 #include "internal.cuh"
 #include "tc.cuh"
 #include "vec.cuh"
@@ -527,19 +528,14 @@ __global__ void __launch_bounds__(128, 4) k_conv_ws(const bf16* __restrict__ X, 
         cp_async_cg16(wsm + tap * BTAP + tc::tile_off(r, kg * 8, N), Wt + (size_t)r * g.Kp + tap * g.cin + kg * 8);
     }
     cp_async_commit();
-    // This thread's vectors of every patch, worked out once: the patch pixel
-    // (row py, column px), its offset in the image's pixels from the patch's
-    // first, and its places in shared memory and among the channels.
+    // This thread's vectors of every patch, worked out once (but for the
+    // kernel-prediction head's pixels, whose registers its epilogue needs: 243 us
+    // so, 280 with them kept).
     constexpr int NV = 12;  // 18 x 10 pixels of 8 groups (64 channels) over 128 threads
-    int rel[NV], at[NV];    // rel: pixel offset; at: shared offset | py << 20 | px << 26
+    PatchVec vec[NV];
     const int nv = PY * PX * KG;
 #pragma unroll
-    for (int j = 0; j < NV; j++) {
-        const int v = tid + 128 * j;
-        const int kg = v % KG, q = v / KG, py = q / PX, px = q - py * PX;
-        rel[j] = (py * g.W + px) * 8 + kg;  // the group beside it (at most 8 of them)
-        at[j] = (kg * LBO_A + q * 16) | py << 20 | px << 26;
-    }
+    for (int j = 0; j < NV; j++) vec[j] = PatchVec(tid + 128 * j, KG, PX, LBO_A, g.W);
     // A block's tiles are consecutive, so that a tile's place is one step from
     // the last one's (two divisions a tile and use cost a third of the loop: the
     // 1080p layers of 32 channels 95 / 147 / 115 us so, 85 / 144 / 109 with
@@ -578,11 +574,11 @@ __global__ void __launch_bounds__(128, 4) k_conv_ws(const bf16* __restrict__ X, 
             if (tid + 128 * j >= nv) continue;
             bool ok = true;
             if (!inside) {
-                const int y = y0 + ((at[j] >> 20) & 31), x = x0 + (at[j] >> 26);
+                const int y = y0 + vec[j].row(), x = x0 + vec[j].column();
                 ok = y >= 0 && y < g.H && x >= 0 && x < g.W;
             }
-            const bf16* src = ok ? base + (size_t)(rel[j] >> 3) * g.xs + (rel[j] & 7) * 8 : X;
-            cp_async_ca16_at(patch + (uint32_t)(at[j] & 0xFFFFF), src, ok ? 16u : 0u);
+            const bf16* src = ok ? base + (size_t)(KPN ? vec[j].pixel_in(g.W) : vec[j].pixel) * g.xs + vec[j].channel() : X;
+            cp_async_ca16_at(patch + vec[j].shared_bytes(), src, ok ? 16u : 0u);
         }
         cp_async_commit();
     };

@@ -1,4 +1,6 @@
-// A host build of the library's path decisions (phiray_b200/csrc/rules.cuh).
+// A host build of the library's path decisions (phiray_b200/csrc/rules.cuh) and
+// of a kernel's index arithmetic (conv_index.cuh).
+#include "../phiray_b200/csrc/conv_index.cuh"
 #include "../phiray_b200/csrc/rules.cuh"
 
 extern "C" int probe_aligned16(const void* p) { return phx::aligned16(p) ? 1 : 0; }
@@ -44,4 +46,14 @@ extern "C" void probe_pool_plan(uint32_t count, uint32_t spp, uint32_t blocks, u
 }
 extern "C" uint32_t probe_pool_slots(uint64_t samples, uint32_t blocks, uint32_t most) {
     return phx::pool_slots(samples, blocks, most);
+}
+
+// A patch vector as (pixel, shared bytes, channel, row, column).
+extern "C" void probe_patch_vec(int v, int groups, int px, int lbo, int width, int64_t* out) {
+    const phx::PatchVec p(v, groups, px, lbo, width);
+    out[0] = p.pixel;
+    out[1] = p.shared_bytes();
+    out[2] = p.channel();
+    out[3] = p.row();
+    out[4] = p.column();
 }

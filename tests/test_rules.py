@@ -1,5 +1,6 @@
 """The host's decisions between paths (phiray_b200/csrc/rules.cuh), built for
-the host: which calls take which path, over the forms that they accept."""
+the host: which calls take which path, over the forms that they accept. And the
+index arithmetic of the convolutions' copies (conv_index.cuh)."""
 
 import ctypes as C
 import subprocess
@@ -113,3 +114,19 @@ def test_pooled_render_memory_follows_the_frame(rules, count, spp, blocks, most)
         assert rules.probe_pool_slots(count * now, blocks, most) <= slots
         left -= now
     assert -(-spp // per) == -(-spp // min(max((1 << 30) // (count * 40), 1), spp))  # as many launches as it takes
+
+
+# 15.8 M pixels wide is where (row W + column) 8 passes 2^31, 126 M where row W does
+@pytest.mark.parametrize("width", [1, 8, 1920, 15_790_320, 15_800_000, 67_108_864, 126_000_000])
+@pytest.mark.parametrize("groups", [2, 4, 6, 8])
+def test_patch_vectors_of_wide_images(rules, width, groups):
+    PX, PY = 10, 18
+    lbo, seen = PX * PY * 16, set()
+    out = (C.c_int64 * 5)()
+    for v in range(PX * PY * groups):
+        rules.probe_patch_vec(v, groups, PX, lbo, width, out)
+        q, g = divmod(v, groups)
+        row, col = divmod(q, PX)
+        assert list(out) == [row * width + col, g * lbo + q * 16, 8 * g, row, col]
+        seen.add(out[1])
+    assert len(seen) == PX * PY * groups
