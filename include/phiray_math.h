@@ -77,12 +77,8 @@ PM_HD float pm_rint(float x) {
 #endif
 }
 
-PM_HD float pm_exp2(float x) {
-    if (x != x) return x;
-    if (x >= 128.0f) return pm_float(0x7f800000u);
-    if (x < -150.0f) return 0.0f;
-    float k = pm_rint(x);
-    float f = x - k;
+/* 2^f for |f| <= 0.5. */
+PM_HD float pm_exp2_part(float f) {
     float t = f * 0.693147182f;
     float p = 1.98412701e-4f;
     p = p * t + 1.38888892e-3f;
@@ -92,6 +88,15 @@ PM_HD float pm_exp2(float x) {
     p = p * t + 0.5f;
     p = p * t + 1.0f;
     p = p * t + 1.0f;
+    return p;
+}
+
+PM_HD float pm_exp2(float x) {
+    if (x != x) return x;
+    if (x >= 128.0f) return pm_float(0x7f800000u);
+    if (x < -150.0f) return 0.0f;
+    float k = pm_rint(x);
+    float p = pm_exp2_part(x - k);
     int ki = (int)k;
     int k1 = ki / 2;
     int k2 = ki - k1;

@@ -154,15 +154,7 @@ __global__ void __launch_bounds__(256, FIRST ? 1 : 6) k_round(const float4* __re
             const float e = (-dn * p.s0 - da * p.s1 - dd * p.s2 - dl * dl * p.s3) * 1.44269502f;
             // pm_exp2(e): 2^k (e rounded, in the low bits of e + 1.5 * 2^23) times a polynomial
             const float big = e + 12582912.0f;
-            const float t = (e - (big - 12582912.0f)) * 0.693147182f;
-            float q = 1.98412701e-4f;
-            q = q * t + 1.38888892e-3f;
-            q = q * t + 8.33333377e-3f;
-            q = q * t + 4.16666679e-2f;
-            q = q * t + 1.66666672e-1f;
-            q = q * t + 0.5f;
-            q = q * t + 1.0f;
-            q = q * t + 1.0f;
+            const float q = pm_exp2_part(e - (big - 12582912.0f));
             float stop = __uint_as_float(__float_as_uint(q) + (__float_as_uint(big) << 23));
             if (e < -150.0f) stop = 0.0f;
             // (a result of exponent k >= -120 is normal)
