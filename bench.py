@@ -214,6 +214,16 @@ def cpu_baseline(scene, cam) -> dict:
                       "oracle/ C++ OpenMP"}
 
 
+def frame_traffic(kernel: int, w: int, h: int, spp: int) -> int | None:
+    """DRAM bytes a traced frame moved when it was captured with this kernel,
+    size and sample count (all its launches), or None."""
+    with open(os.path.join(ROOT, "profiles", "pool_render_traffic.json")) as f:
+        info = json.load(f)
+    if (w, h, spp) != (info["width"], info["height"], info["spp"]):
+        return None
+    return info["kernels"].get(str(kernel), {}).get("dram_bytes_per_frame")
+
+
 def profile_phase(args, tr, gpu, cam, verts_dev, W, H, n, local) -> None:
     """Warm-up and steps of one kernel family alone (for ncu launch lists and
     captures): the frame render, the incoherent ray walk, or the LBVH build."""
@@ -818,13 +828,8 @@ def main() -> None:
     alg_bytes = counts[1] * 64 + counts[2] * 48
     pk = peaks()
     achieved = alg_bytes / (trace_ms * 1e-3) / 1e9
-    traffic = None
     pooled = KERNEL_NAMES[chosen].startswith("pooled")
-    tpath = os.path.join(ROOT, "profiles", "pool_render_traffic.json" if pooled else "trace_render_traffic.json")
-    if os.path.exists(tpath):
-        with open(tpath) as f:
-            tinfo = json.load(f)
-        traffic = tinfo.get("dram_bytes_per_launch_full")
+    traffic = frame_traffic(chosen, W, H, args.spp)
 
     rays = torch.empty((n, 8), dtype=torch.float32, device=f"cuda:{local}")
     hits = torch.empty((n, 4), dtype=torch.float32, device=f"cuda:{local}")
@@ -906,8 +911,9 @@ def main() -> None:
             "roofline": {"bound": "hbm", "kernel": "k_render_pool (pooled render)" if pooled else "k_render (path-trace megakernel)",
                          "achieved": round(achieved, 1),
                          "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": round(achieved / pk["hbm_gbs"], 4),
-                         "traffic": traffic, "peak_source": pk["source"],
-                         "algorithmic": f"{counts[1]} node steps x 64 B + {counts[2]} triangle tests x 48 B per launch"},
+                         "traffic": traffic, "traffic_of": "a frame, all launches, as captured with this kernel",
+                         "peak_source": pk["source"],
+                         "algorithmic": f"{counts[1]} node steps x 64 B + {counts[2]} triangle tests x 48 B a frame"},
             "cpu_baseline": cpu,
             "e2e": {"value": round(e2e, 2), "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                     "statistic": "median step", "mean_value": round(e2e_mean, 2),
