@@ -1,8 +1,7 @@
-// The binned SAH builder's per-node steps (phiray src/bvh/sah.rs:25-189),
-// written once for the device kernels of sah.cu and for a host build of
-// the same code: every function here is plain arithmetic on one node or
-// one tree entry, so a host loop over the entries computes exactly what a
-// launch over them computes.
+// The binned SAH builder's arithmetic (phiray src/bvh/sah.rs:25-189) that its
+// device kernels (sah.cu, sah_subtree.cuh) share with host builds: a node's grid
+// and bins, an axis's sweep, the decision, and the tree's numbering and bounds;
+// for host builds also a node's whole step as one serial function.
 //
 // The tree equals the reference's node for node: the same bins, sweep and
 // leaf rule per node, the same in-place (swap) partition of the node's
@@ -92,54 +91,12 @@ SAH_HD bool grid_of(const Box& cbox, float* lo, float* scale) {
     return !flat;
 }
 
-// What split does with a node once its bins are filled (sah.rs:150-181):
-// the cheapest plane over the three axes' sweeps, then the leaf rule.
+// What becomes of a node once its bins are filled (sah.rs:150-181): the
+// cheapest plane over the three axes' sweeps, then the leaf rule.
 enum Cut : uint32_t { CUT_LEAF = 0, CUT_HALF = 1, CUT_PLANE = 2 };
 struct Decision {
     uint32_t cut, axis, at;
 };
-
-SAH_HD Decision decide(const uint32_t (*bcount)[BINS], const Box (*bbox)[BINS], const float* scale, uint32_t count,
-                       uint32_t leaf) {
-    bool have = false;
-    float best = 0.0f;
-    uint32_t best_k = 0;
-    uint32_t best_at = 0;
-    for (int k = 0; k < 3; k++) {
-        if (scale[k] == 0.0f) continue;
-        float right_area[BINS];
-        uint32_t right_count[BINS];
-        Box b = empty_box();
-        uint32_t c = 0;
-        for (uint32_t at = BINS - 1; at >= 1; at--) {
-            grow(b, bbox[k][at]);
-            c += bcount[k][at];
-            right_area[at] = area(b);
-            right_count[at] = c;
-        }
-        b = empty_box();
-        c = 0;
-        for (uint32_t at = 0; at + 1 < BINS; at++) {
-            grow(b, bbox[k][at]);
-            c += bcount[k][at];
-            const uint32_t rc = right_count[at + 1];
-            if (c == 0 || rc == 0) continue;
-            const float cost = area(b) * (float)c + right_area[at + 1] * (float)rc;
-            if (!have || cost < best) {
-                have = true;
-                best = cost;
-                best_k = (uint32_t)k;
-                best_at = at;
-            }
-        }
-    }
-    Box bounds = empty_box();
-    for (uint32_t b = 0; b < BINS; b++) grow(bounds, bbox[0][b]);
-    if (!have) return Decision{count > leaf ? (uint32_t)CUT_HALF : (uint32_t)CUT_LEAF, 0u, 0u};
-    const float parent = rmax(area(bounds), 1.17549435e-38f);  // f32::MIN_POSITIVE
-    if (count <= leaf && TRAVERSE + best / parent >= (float)count) return Decision{CUT_LEAF, 0u, 0u};
-    return Decision{CUT_PLANE, best_k, best_at};
-}
 
 SAH_HD uint32_t lowest_bit(uint32_t x) {
 #if defined(__CUDA_ARCH__)
@@ -214,17 +171,68 @@ SAH_HD Decision decide_from(const AxisBest* axes, const float* scale, const Box&
     return Decision{CUT_PLANE, best_k, best_at};
 }
 
-// decide over the occupied bins only (mask[k] for axis k).
-SAH_HD Decision decide_occupied(const uint32_t* mask, const uint32_t (*bcount)[BINS], const Box (*bbox)[BINS],
-                                const float* scale, uint32_t count, uint32_t leaf) {
-    AxisBest axes[3];
-    for (int k = 0; k < 3; k++)
-        axes[k] = scale[k] == 0.0f ? AxisBest{false, 0.0f, 0u} : sweep_axis(mask[k], bcount[k], bbox[k]);
-    Box bounds = empty_box();
-    for (uint32_t b = 0; b < BINS; b++)
-        if ((mask[0] >> b) & 1u) grow(bounds, bbox[0][b]);
-    return decide_from(axes, scale, bounds, count, leaf);
+// One node of the tree under construction (temporary numbering).
+struct TNode {
+    uint32_t start, end, depth;
+    uint32_t left, right;  // temporary ids of the children; NONE for a leaf
+};
+
+// Inner nodes in t's subtree, t included (children's counts first).
+SAH_HD void count_inner(uint32_t t, const TNode* tn, uint32_t* inner) {
+    const TNode nd = tn[t];
+    inner[t] = nd.left == NONE ? 0u : 1u + inner[nd.left] + inner[nd.right];
 }
+
+// Top down: an inner node of depth-first rank r has its children at final
+// indices 2r + 1 and 2r + 2 (sah.rs:95-105's work stack pops the left child
+// first and hands out two indices per inner node).
+SAH_HD void place(uint32_t t, const TNode* tn, const uint32_t* inner, uint32_t* rank, uint32_t* final_index) {
+    const TNode nd = tn[t];
+    if (nd.left == NONE) return;
+    const uint32_t r = rank[t];
+    rank[nd.left] = r + 1;
+    rank[nd.right] = r + 1 + inner[nd.left];
+    final_index[nd.left] = 2 * r + 1;
+    final_index[nd.right] = 2 * r + 2;
+}
+
+// The node at its final index, bounds from its children or its primitives
+// (Bvh::refit, build.rs:180-194: unions, exact in any order). `boxes` holds
+// each temporary node's bounds for its parent; children come first.
+SAH_HD void emit(uint32_t t, const TNode* tn, const uint32_t* final_index, const float* prims, const uint32_t* order,
+                 Box* boxes, float* nodes) {
+    const TNode nd = tn[t];
+    Box b = empty_box();
+    uint32_t lo_i, hi_i;
+    if (nd.left == NONE) {
+        for (uint32_t s = nd.start; s < nd.end; s++) grow(b, prim_box(prims + 8 * (uint64_t)order[s]));
+        lo_i = nd.start | LEAF_BIT;
+        hi_i = nd.end;
+    } else {
+        b = boxes[nd.left];
+        grow(b, boxes[nd.right]);
+        lo_i = final_index[nd.left];
+        hi_i = final_index[nd.right];
+    }
+    boxes[t] = b;
+    float* o = nodes + 8 * (uint64_t)final_index[t];
+    uint32_t* u = (uint32_t*)o;
+    o[0] = b.lo[0];
+    o[1] = b.lo[1];
+    o[2] = b.lo[2];
+    u[3] = lo_i;
+    o[4] = b.hi[0];
+    o[5] = b.hi[1];
+    o[6] = b.hi[2];
+    u[7] = hi_i;
+}
+
+#ifndef __CUDACC__
+
+// ---- a node's step as one serial function, for host builds ----
+//
+// What the device's forms of the step (a warp's, a block's and a chunked one)
+// come to, from the same grid, bins, sweep, decision and partition.
 
 // sah.rs:114-189 split: the left count after reordering slots[0, count), or
 // NONE for a leaf. Serial over the node's slots; a bin's entries are set
@@ -298,12 +306,6 @@ SAH_HD uint32_t split(const float* prims, const float* centres, uint32_t* slots,
     return (m == 0 || m == count) ? count / 2 : m;
 }
 
-// One node of the tree under construction (temporary numbering).
-struct TNode {
-    uint32_t start, end, depth;
-    uint32_t left, right;  // temporary ids of the children; NONE for a leaf
-};
-
 // Where to put new nodes: a counter of temporary ids and the next level's
 // list. `add` is an atomic add on the device and a plain one on the host.
 template <class Add>
@@ -328,55 +330,7 @@ SAH_HD void process(uint32_t t, TNode* tn, const float* prims, const float* cent
     tn[t] = nd;
 }
 
-// Inner nodes in t's subtree, t included (children's counts first).
-SAH_HD void count_inner(uint32_t t, const TNode* tn, uint32_t* inner) {
-    const TNode nd = tn[t];
-    inner[t] = nd.left == NONE ? 0u : 1u + inner[nd.left] + inner[nd.right];
-}
-
-// Top down: an inner node of depth-first rank r has its children at final
-// indices 2r + 1 and 2r + 2 (sah.rs:95-105's work stack pops the left child
-// first and hands out two indices per inner node).
-SAH_HD void place(uint32_t t, const TNode* tn, const uint32_t* inner, uint32_t* rank, uint32_t* final_index) {
-    const TNode nd = tn[t];
-    if (nd.left == NONE) return;
-    const uint32_t r = rank[t];
-    rank[nd.left] = r + 1;
-    rank[nd.right] = r + 1 + inner[nd.left];
-    final_index[nd.left] = 2 * r + 1;
-    final_index[nd.right] = 2 * r + 2;
-}
-
-// The node at its final index, bounds from its children or its primitives
-// (Bvh::refit, build.rs:180-194: unions, exact in any order). `boxes` holds
-// each temporary node's bounds for its parent; children come first.
-SAH_HD void emit(uint32_t t, const TNode* tn, const uint32_t* final_index, const float* prims, const uint32_t* order,
-                 Box* boxes, float* nodes) {
-    const TNode nd = tn[t];
-    Box b = empty_box();
-    uint32_t lo_i, hi_i;
-    if (nd.left == NONE) {
-        for (uint32_t s = nd.start; s < nd.end; s++) grow(b, prim_box(prims + 8 * (uint64_t)order[s]));
-        lo_i = nd.start | LEAF_BIT;
-        hi_i = nd.end;
-    } else {
-        b = boxes[nd.left];
-        grow(b, boxes[nd.right]);
-        lo_i = final_index[nd.left];
-        hi_i = final_index[nd.right];
-    }
-    boxes[t] = b;
-    float* o = nodes + 8 * (uint64_t)final_index[t];
-    uint32_t* u = (uint32_t*)o;
-    o[0] = b.lo[0];
-    o[1] = b.lo[1];
-    o[2] = b.lo[2];
-    u[3] = lo_i;
-    o[4] = b.hi[0];
-    o[5] = b.hi[1];
-    o[6] = b.hi[2];
-    u[7] = hi_i;
-}
+#endif
 
 }  // namespace sah
 }  // namespace phx
