@@ -741,7 +741,7 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
     PHX_TRY(use(&ctx->c));
     Ctx* c = &ctx->c;
     cudaStream_t s = c->stream;
-    const uint32_t cap = 2 * n - 1;
+    const uint32_t cap = open_nodes(n);
     DevMem centres, tn, lists, counters, inner, rank, final_index, boxes, loc, loc_count;
     PHX_TRY(centres.reserve((size_t)n * 12));
     PHX_TRY(tn.reserve((size_t)cap * sizeof(TNode)));
@@ -804,12 +804,12 @@ int32_t phx_bvh_build_sah(phx_ctx ctx, const phx_aabb* prims, uint32_t n, uint32
         PHX_CUDA(cudaMemcpyAsync(lc, LC, LC_WORDS * 4, cudaMemcpyDeviceToHost, s));
         PHX_TRY(wait_stream(s, 0));
         nseeds = lc[LC_SEEDS];
-        if (nseeds > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than 2n - 1");
+        if (nseeds > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than %u slots open", n);
         if (lv > 0) {
             // the children the level before opened (this level's length)
             if (lc[LC_LEN] == 0) break;
             const uint32_t at = off[lv - 1] + len[lv - 1];
-            if (at + lc[LC_LEN] > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than 2n - 1");
+            if (at + lc[LC_LEN] > cap) return fail(PHX_ERR_DEVICE, "SAH build: more nodes than %u slots open", n);
             off.push_back(at);
             len.push_back(lc[LC_LEN]);
         }

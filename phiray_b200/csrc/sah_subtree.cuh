@@ -12,6 +12,14 @@ using sah::TNode;
 
 constexpr uint32_t SUB = 128;  // nodes under this many slots are seeds
 
+// The most nodes a build of n slots opens above and with its seeds: only nodes of
+// SUB slots or more open two others, those of a level share the slots out, and
+// no more than MAX_DEPTH - 1 levels have them.
+constexpr uint32_t open_nodes(uint32_t n) {
+    const uint64_t all = 2ull * n - 1, some = 1 + 2ull * (sah::MAX_DEPTH - 1) * (n / SUB);
+    return (uint32_t)(some < all ? some : all);
+}
+
 // Floats as words whose unsigned order is the floats' order (for atomic min
 // and max; a NaN has no place among them and is left out).
 __device__ __forceinline__ uint32_t ord(float f) {

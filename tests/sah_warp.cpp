@@ -26,3 +26,5 @@ extern "C" uint32_t warp_build_sah(const float* prims, uint32_t n, uint32_t leaf
     });
     return 2 * inner + 1;
 }
+
+extern "C" uint32_t warp_open_nodes(uint32_t n) { return phx::open_nodes(n); }

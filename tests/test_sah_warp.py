@@ -13,11 +13,15 @@ HERE = Path(__file__).resolve().parent
 
 
 @pytest.fixture(scope="module")
-def build(tmp_path_factory):
+def lib(tmp_path_factory):
     out = tmp_path_factory.mktemp("sahwarp") / "libsahwarp.so"
     subprocess.run(["g++", "-O1", "-std=c++20", "-pthread", "-shared", "-fPIC", "-ffp-contract=off", "-fno-fast-math",
                     "-Wno-unknown-pragmas", "-o", str(out), str(HERE / "sah_warp.cpp")], check=True)
-    lib = C.CDLL(str(out))
+    return C.CDLL(str(out))
+
+
+@pytest.fixture(scope="module")
+def build(lib):
     lib.warp_build_sah.restype = C.c_uint32
 
     def run(prims, leaf, vec):
@@ -66,3 +70,23 @@ def test_a_warps_subtree_is_the_reference_tree(build, orc, n, leaf, vec, kind):
     assert depth == want_depth
     assert np.array_equal(order, want_order)
     assert np.array_equal(nodes.view(np.uint32), want_nodes.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 300, 5000, 100_000])
+@pytest.mark.parametrize("cut", ["one", "half", "seed", "mixed"])
+def test_open_nodes_bounds_what_a_build_opens(lib, n, cut):
+    """Nodes opened by the build's rule (128 slots or more, up to depth 30)
+    when every node parts as unevenly, evenly or awkwardly as it can."""
+    rng = np.random.default_rng(n)
+    opened, level = 1, [n]
+    for _ in range(31):
+        children = []
+        for k in level:
+            if k < 128:
+                continue
+            kind = cut if cut != "mixed" else ("one", "half", "seed")[rng.integers(3)]
+            m = {"one": 1, "half": k // 2, "seed": min(127, k - 1)}[kind]
+            children += [m, k - m]
+        opened += len(children)
+        level = children
+    assert opened <= lib.warp_open_nodes(n) <= 2 * n - 1
