@@ -434,8 +434,9 @@ int32_t phx_tracer_create_instanced(phx_ctx ctx, const phx_scene* scene, const p
 int32_t phx_tracer_reinstance(phx_tracer tr, const phx_instance* insts, uint32_t ninsts);
 int32_t phx_tracer_destroy(phx_tracer tr);
 /* Which kernel traces a frame. All compute the same image bit for bit. A
- * tracer whose kernel was neither set nor autotuned takes the pooled render
- * where it can run and PHX_KERNEL_MEGAKERNEL elsewhere.
+ * tracer whose kernel was neither set nor autotuned takes a form of the pooled
+ * render where it can run, but for one sample of few pixels of a small scene, and
+ * PHX_KERNEL_MEGAKERNEL elsewhere.
  * PHX_KERNEL_MEGAKERNEL is shade.wgsl's main as one thread per pixel with the
  * walk called from every site that traces;
  * PHX_KERNEL_STATE_MACHINE and its _6 and _8 forms are the pooled render with

@@ -845,7 +845,7 @@ struct PoolForm {
         while (left) {
             PoolFrame J{L.first, L.count, std::min(left, p.spp), PoolOut{out, (uint64_t)L.count * p.spp}};
             R.F.spp = J.spp;
-            const uint32_t slots = pool_slots((uint64_t)L.count * J.spp, p.blocks, P);
+            const uint32_t slots = launch_slots(p, L.count, J.spp, P);
             PHX_CUDA(cudaMemsetAsync(L.next, 0, 4, L.s));
             k_render_pool<M, MINB, P, T><<<p.blocks, T, SMEM, L.s>>>(L.S, R.F, L.sun, J, slots, state, L.next, L.counters);
             k_pool_resolve<<<(L.count + 127) / 128, 128, 0, L.s>>>(R.F, J, L.px);

@@ -21,6 +21,9 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0u; }
 // A tracer whose render kernel was neither set nor autotuned.
 constexpr uint32_t KERNEL_UNSET = 0xFFFFFFFFu;
 
+// Frames of so few samples trace in one fill of the pools (see POOL_FILLS).
+constexpr uint64_t FEW_SAMPLES = 300000;
+
 // What a frame asks of the kernel that traces it.
 struct FrameForm {
     uint32_t kernel;  // the tracer's (set or autotuned, or KERNEL_UNSET)
@@ -29,6 +32,7 @@ struct FrameForm {
     bool adaptive;
     bool transmits;   // some material transmits light
     bool capturing;   // the launches are recorded into a graph
+    uint32_t pixels, spp, faces;
 };
 
 inline bool pooled_id(uint32_t kernel) {
@@ -46,18 +50,29 @@ inline uint32_t fastest_megakernel(const float* ms) {
     return best;
 }
 
-// The id of the kernel that traces the frame. The default is the pooled render
-// where it can run, which on a 65,536-face cloud at 256 x 256, 16 spp took 4.9
-// ms against the 4-block megakernel's 27 ms, on the 1.3 M-face mesh at 1080p,
-// 16 spp, 28 ms against 57, and on 64 x 48 pixels 0.6 against 0.8; else that
-// megakernel. All compute the same image. Adaptive Sampling runs on the
+// The kernel of a frame whose tracer names none, of those that compute the same
+// image: the pooled render where it can run. On a 65,536-face cloud at 256 x 256,
+// 16 spp, it took 4.9 ms against the 4-block megakernel's 27 ms, on the 1.3
+// M-face mesh at 1080p, 16 spp, 28 ms against 57. Frames of few samples take the
+// form of 256 threads (more and smaller pools end sooner): 256 x 256 at 1 spp,
+// megakernel / 512 threads / 256 threads, cloud 2.06 / 1.59 / 1.49 ms, that mesh
+// 0.76 / 0.84 / 0.73. One sample of few pixels of a small scene is a few walks
+// one after another, which the megakernel does without phases (a scene of 1,600
+// faces at 256 x 256, 1 spp 0.17 ms against 0.21; of two triangles 0.05 against
+// 0.09; from 144,000 pixels on, or with two samples, the pools are even or ahead).
+inline uint32_t default_kernel(const FrameForm& f) {
+    if (f.full || (f.spp == 1 && f.pixels < 100000 && f.faces < 10000)) return f.mega;
+    return (uint64_t)f.pixels * f.spp < FEW_SAMPLES ? PHX_KERNEL_STATE_MACHINE_6 : PHX_KERNEL_STATE_MACHINE;
+}
+
+// The id of the kernel that traces the frame. Adaptive Sampling runs on the
 // megakernel forms (the others take pixels by index, not from the open list);
 // the pooled render shades a path's one opaque camera hit, so it takes scenes
 // whose materials transmit no light; the wavefront's host polls its queues
 // between passes, which a recorded graph cannot.
 inline uint32_t frame_kernel(const FrameForm& f) {
     uint32_t k = f.kernel;
-    if (k == KERNEL_UNSET) k = f.full ? f.mega : PHX_KERNEL_STATE_MACHINE;
+    if (k == KERNEL_UNSET) k = default_kernel(f);
     if (k == PHX_KERNEL_WAVEFRONT && (f.adaptive || f.capturing)) return f.mega;
     if (pooled_id(k) && (f.adaptive || (f.transmits && !f.full))) return f.mega;
     return k;
@@ -72,7 +87,9 @@ inline bool frame_pooled(const FrameForm& f) { return !f.full && pooled_id(frame
 // Fills of a pool a frame is cut into at least (fewer slots, so that a small
 // frame's last paths do not leave most of a pool empty, against fewer and
 // larger phases): the cloud above took 7.0, 4.9, 5.0, 5.3 and 6.3 ms at 1, 2,
-// 3, 4 and 8 fills.
+// 3, 4 and 8 fills. Of few samples every phase is short, and one fill has the
+// fewest: at 1 spp and 480 x 300 2.0 ms against 2.4, the 1.3 M-face mesh 0.95
+// against 1.08; from 640 x 480 at 1 spp on two are even or ahead.
 constexpr uint32_t POOL_FILLS = 2;
 
 // Sample terms held at once; the rest of the samples run in further launches.
@@ -80,7 +97,7 @@ constexpr size_t POOL_OUT_BYTES = (size_t)1 << 30;
 
 // Slots a block for `samples` paths over `blocks` blocks of at most `most`.
 inline uint32_t pool_slots(uint64_t samples, uint32_t blocks, uint32_t most) {
-    const uint64_t share = samples / blocks / POOL_FILLS / 32u * 32u;
+    const uint64_t share = samples / blocks / (samples < FEW_SAMPLES ? 1u : POOL_FILLS) / 32u * 32u;
     return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(share, 32u));
 }
 
@@ -105,6 +122,11 @@ inline PoolPlan pool_plan(uint32_t count, uint32_t spp, uint32_t blocks, uint32_
     p.state = (size_t)blocks * p.slots * slot_bytes;
     p.out = sample * p.spp;
     return p;
+}
+
+// Slots a block of a launch of `spp` of the samples (the last may have few).
+inline uint32_t launch_slots(const PoolPlan& p, uint32_t count, uint32_t spp, uint32_t most) {
+    return std::min(p.slots, pool_slots((uint64_t)count * spp, p.blocks, most));
 }
 
 // ---- a batch's launches scene by scene, on side streams ----

@@ -1146,8 +1146,9 @@ int32_t ensure_wide(phx_tracer tr) {
     return read_status(c);
 }
 
-FrameForm form_of(phx_tracer tr, const Frame& F, bool capturing) {
-    return FrameForm{tr->kernel, tr->mega, tr->forest || F.grid > 0.0f, F.adapt_on != 0u, tr->transmits, capturing};
+FrameForm form_of(phx_tracer tr, const Frame& F, uint32_t count_px, bool capturing) {
+    return FrameForm{tr->kernel, tr->mega, tr->forest || F.grid > 0.0f, F.adapt_on != 0u, tr->transmits, capturing,
+                     count_px, F.spp, tr->nfaces};
 }
 
 int32_t capturing(cudaStream_t s, bool& on) {
@@ -1178,7 +1179,7 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
     Ctx* c = tr->ctx;
     bool recorded = false;
     PHX_TRY(capturing(c->stream, recorded));
-    const FrameForm form = form_of(tr, F, recorded);
+    const FrameForm form = form_of(tr, F, count_px, recorded);
     const uint32_t kernel = frame_kernel(form);
     const RenderLaunch L = launch_of(tr, F, sun, first_px, count_px, c->stream);
     if (kernel == PHX_KERNEL_WAVEFRONT) {
@@ -1207,7 +1208,7 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
 // pooled render, or null: nothing is allocated here. (Not the wavefront.)
 int32_t launch_frame_on(cudaStream_t s, const PoolPlan& plan, const PoolScratch* buffers, phx_tracer tr, const Frame& F,
                         f3 sun) {
-    const FrameForm form = form_of(tr, F, true);
+    const FrameForm form = form_of(tr, F, F.n, true);
     const uint32_t kernel = frame_kernel(form);
     const RenderLaunch L = launch_of(tr, F, sun, 0, F.n, s);
     if (form.full) return render_full(kernel, false, L);
@@ -2134,7 +2135,7 @@ int32_t trace_per_scene(phx_batch b) {
     std::vector<LaneJob> jobs;
     for (const BatchJob& bj : b->jobs) {
         const Frame F = frame_for(bj.tr, &bj.cam, bj.w, bj.h, bj.first, bj.spp);
-        const FrameForm form = form_of(bj.tr, F, recorded);
+        const FrameForm form = form_of(bj.tr, F, F.n, recorded);
         PoolPlan p{};
         if (frame_pooled(form)) PHX_TRY(plan_pooled(frame_kernel(form), false, c->sms, F.n, F.spp, p));
         frames.push_back(F);
@@ -2171,7 +2172,7 @@ int32_t trace_per_scene(phx_batch b) {
                                             cudaMemcpyDeviceToDevice, s), "rays"));
     };
     auto wavefront = [&](uint32_t j) {
-        return frame_kernel(form_of(b->jobs[j].tr, frames[j], recorded)) == PHX_KERNEL_WAVEFRONT;
+        return frame_kernel(form_of(b->jobs[j].tr, frames[j], frames[j].n, recorded)) == PHX_KERNEL_WAVEFRONT;
     };
     for (uint32_t j : plan.order)
         if (rc >= 0 && !wavefront(j)) trace(j, b->lanes[plan.lane[j]].stream, false);

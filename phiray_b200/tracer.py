@@ -240,8 +240,9 @@ class Tracer:
         return chosen.value, list(ms)
 
     def set_kernel(self, kind: int) -> None:
-        """Render kernel, one of the ids above (same image). Unset, the pooled
-        render (STATE_MACHINE) where it can run, else MEGAKERNEL."""
+        """Render kernel, one of the ids above (same image). Unset, a form of the
+        pooled render (the STATE_MACHINE ids) where it can run, but for one sample
+        of few pixels of a small scene; else MEGAKERNEL."""
         N.check(N.lib().phx_tracer_set_kernel(self.handle, kind))
 
     STACK_LOCAL = 0

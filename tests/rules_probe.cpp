@@ -9,8 +9,10 @@ extern "C" uint32_t probe_fastest_megakernel(const float* ms) { return phx::fast
 
 // The id of the kernel that traces a frame, and (bit 31) whether it needs the
 // pooled render's buffers. flags: full, adaptive, transmits, capturing.
-extern "C" uint32_t probe_frame_kernel(uint32_t kernel, uint32_t mega, uint32_t flags) {
-    const phx::FrameForm f{kernel, mega, (flags & 1u) != 0, (flags & 2u) != 0, (flags & 4u) != 0, (flags & 8u) != 0};
+extern "C" uint32_t probe_frame_kernel(uint32_t kernel, uint32_t mega, uint32_t flags, uint32_t pixels, uint32_t spp,
+                                       uint32_t faces) {
+    const phx::FrameForm f{kernel, mega, (flags & 1u) != 0, (flags & 2u) != 0, (flags & 4u) != 0, (flags & 8u) != 0,
+                           pixels, spp, faces};
     return phx::frame_kernel(f) | (phx::frame_pooled(f) ? 0x80000000u : 0u);
 }
 
@@ -35,17 +37,17 @@ extern "C" uint32_t probe_lanes(const uint64_t* jobs, uint32_t n, uint32_t lanes
     return made;
 }
 
-// pool_plan as (blocks, slots, spp, state, out), and the slots of a launch.
-extern "C" void probe_pool_plan(uint32_t count, uint32_t spp, uint32_t blocks, uint32_t most, uint64_t* plan) {
+// pool_plan as (blocks, slots, spp, state, out), and the slots of its launch of
+// `now` samples.
+extern "C" uint32_t probe_pool_plan(uint32_t count, uint32_t spp, uint32_t blocks, uint32_t most, uint32_t now,
+                                    uint64_t* plan) {
     const phx::PoolPlan p = phx::pool_plan(count, spp, blocks, most, 244, 40);
     plan[0] = p.blocks;
     plan[1] = p.slots;
     plan[2] = p.spp;
     plan[3] = p.state;
     plan[4] = p.out;
-}
-extern "C" uint32_t probe_pool_slots(uint64_t samples, uint32_t blocks, uint32_t most) {
-    return phx::pool_slots(samples, blocks, most);
+    return phx::launch_slots(p, count, now, most);
 }
 
 // A patch vector as (pixel, shared bytes, channel, row, column).

@@ -33,23 +33,31 @@ POOLED = (Tracer.STATE_MACHINE, Tracer.STATE_MACHINE_6, Tracer.STATE_MACHINE_8)
 UNSET = 0xFFFFFFFF
 
 
+# one sample and many, around the sizes where the default changes
+FRAMES = [(64, 1, 12), (99_999, 1, 9_999), (100_000, 1, 9_999), (99_999, 1, 10_000), (64, 2, 12), (299_999, 1, 50_000),
+          (300_000, 1, 50_000), (2_073_600, 1, 12), (65_536, 16, 65_540), (2_073_600, 64, 1_310_722)]
+
+
 @pytest.mark.parametrize("mega", [Tracer.MEGAKERNEL, Tracer.MEGAKERNEL_16_SYNC])
 @pytest.mark.parametrize("flags", range(16))
 def test_every_frame_has_a_kernel_that_can_trace_it(rules, flags, mega):
     rules.probe_frame_kernel.restype = C.c_uint32
     for kernel in [*range(Tracer.KERNELS), UNSET]:
-        r = rules.probe_frame_kernel(C.c_uint32(kernel), mega, flags)
-        got, buffers = r & 0x7FFFFFFF, bool(r >> 31)
-        wavefront_can = not flags & (ADAPTIVE | CAPTURING)
-        pooled_can = not flags & ADAPTIVE and (flags & FULL or not flags & TRANSMITS)
-        if kernel == UNSET:
-            want = Tracer.STATE_MACHINE if pooled_can and not flags & FULL else mega
-        elif kernel == Tracer.WAVEFRONT and not wavefront_can or kernel in POOLED and not pooled_can:
-            want = mega
-        else:
-            want = kernel
-        assert got == want
-        assert buffers == (got in POOLED and not flags & FULL)
+        for pixels, spp, faces in FRAMES:
+            r = rules.probe_frame_kernel(C.c_uint32(kernel), mega, flags, pixels, spp, faces)
+            got, buffers = r & 0x7FFFFFFF, bool(r >> 31)
+            wavefront_can = not flags & (ADAPTIVE | CAPTURING)
+            pooled_can = not flags & ADAPTIVE and (flags & FULL or not flags & TRANSMITS)
+            if kernel == UNSET:
+                brief = spp == 1 and pixels < 100_000 and faces < 10_000
+                form = Tracer.STATE_MACHINE_6 if pixels * spp < 300_000 else Tracer.STATE_MACHINE
+                want = form if pooled_can and not flags & FULL and not brief else mega
+            elif kernel == Tracer.WAVEFRONT and not wavefront_can or kernel in POOLED and not pooled_can:
+                want = mega
+            else:
+                want = kernel
+            assert got == want
+            assert buffers == (got in POOLED and not flags & FULL)
 
 
 def test_autotuning_keeps_the_fastest_megakernel_beside_its_pick(rules):
@@ -94,12 +102,12 @@ def test_lanes_reserve_once_for_their_pooled_jobs(rules, seed, fails):
     assert not buffers[jobs[:, 1] == 0].any()
 
 
-@pytest.mark.parametrize("count", [1, 33, 64 * 48, 256 * 256, 1920 * 1080, 120_000_000])
-@pytest.mark.parametrize("spp", [1, 3, 16, 64, 4000])
+@pytest.mark.parametrize("count", [1, 33, 64 * 48, 256 * 256, 1920 * 1080, 2400 * 1800, 120_000_000])
+@pytest.mark.parametrize("spp", [1, 3, 7, 13, 16, 64, 4000])
 @pytest.mark.parametrize("blocks,most", [(296, 4096), (592, 2048), (1184, 1024), (2, 4096)])
 def test_pooled_render_memory_follows_the_frame(rules, count, spp, blocks, most):
     plan = (C.c_uint64 * 5)()
-    rules.probe_pool_plan(count, spp, blocks, most, plan)
+    first = rules.probe_pool_plan(count, spp, blocks, most, 1, plan)
     got_blocks, slots, per, state, out = plan
     assert got_blocks == blocks and 32 <= slots <= most and slots % 32 == 0
     assert 1 <= per <= spp and out == count * per * 40
@@ -108,11 +116,11 @@ def test_pooled_render_memory_follows_the_frame(rules, count, spp, blocks, most)
     assert state == blocks * slots * 244
     assert blocks * slots <= max(count * per, 32 * blocks)
     left = spp
-    while left:  # no launch needs more slots than the plan holds
+    while left:  # no launch takes more slots than the plan holds
         now = min(left, per)
-        rules.probe_pool_slots.argtypes = [C.c_uint64, C.c_uint32, C.c_uint32]
-        assert rules.probe_pool_slots(count * now, blocks, most) <= slots
+        assert 32 <= rules.probe_pool_plan(count, spp, blocks, most, now, plan) <= slots
         left -= now
+    assert 32 <= first <= slots
     assert -(-spp // per) == -(-spp // min(max((1 << 30) // (count * 40), 1), spp))  # as many launches as it takes
 
 
