@@ -53,10 +53,9 @@ struct Ctx {
     uint32_t* status = nullptr;     // device status word
     cudaMemPool_t pool = nullptr;   // device memory of the context's objects
     DevMem denoise_scratch;         // guide and ping-pong planes of phx_denoise
-    PoolScratch path_pool;          // the pooled render's buffers, until the last tracer goes
+    PoolScratch path_pool;          // the pooled render's buffers
     std::mutex path_pool_lock;      // from sizing them to the launches that use them
     int live = 0;                   // buffers, passes, BVHs, tracers not yet freed
-    std::atomic<int> tracers{0};    // the tracers among them
 };
 
 // Sets the thread's last error text and returns `code`.

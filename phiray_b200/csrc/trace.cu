@@ -1319,7 +1319,6 @@ int32_t create_tracer(phx_ctx ctx, const phx_scene* sc, const phx_mesh* meshes, 
     tr->leaf = sc->leaf ? sc->leaf : 4;
     tr->has_normals = sc->normals != nullptr;
     ctx->c.live++;
-    ctx->c.tracers++;
     cudaStream_t s = ctx->c.stream;
     const size_t n = sc->nfaces;
     int32_t rc = PHX_OK;
@@ -1567,14 +1566,8 @@ int32_t phx_tracer_destroy(phx_tracer tr) {
     if (tr->ev0) cudaEventDestroy(tr->ev0);
     if (tr->ev1) cudaEventDestroy(tr->ev1);
     if (tr->wf_host_lens) cudaFreeHost(tr->wf_host_lens);
-    Ctx* c = tr->ctx;
-    c->live--;
+    tr->ctx->live--;
     delete tr;
-    if (--c->tracers == 0) {  // nobody is left to use them
-        std::lock_guard<std::mutex> lock(c->path_pool_lock);
-        c->path_pool.state.release();
-        c->path_pool.out.release();
-    }
     return PHX_OK;
 }
 
