@@ -39,6 +39,20 @@ inline bool pooled_id(uint32_t kernel) {
     return kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8;
 }
 
+// The pooled forms within 6 % of an autotuning's fastest time, as a mask of their
+// ids, if that time is one's: at few samples the last paths' end decides between
+// them, so such forms are timed again at POOL_TIE_SAMPLES times as many. (The 1.3
+// M-face mesh at 1080p, 512 / 256 / 128 threads: 2.71 / 2.67 / 2.83 ms at 1 spp,
+// either of the first two fastest by chance; 7.54 / 7.70 / 8.40 at 4, 27.8 / 28.6
+// / 31.5 at 16.)
+constexpr uint32_t POOL_TIE_SAMPLES = 8;
+inline uint32_t pooled_ties(const float* ms, uint32_t pick) {
+    uint32_t mask = 0;
+    for (uint32_t k = 0; k < PHX_KERNEL_COUNT && pooled_id(pick); k++)
+        if (pooled_id(k) && ms[k] <= 1.06f * ms[pick]) mask |= 1u << k;
+    return mask;
+}
+
 // The fastest megakernel form by the times of an autotuning: what a tracer
 // whose fastest kernel is another one traces adaptive frames, recorded ones and
 // those without memory for the pools with. (The 1.3 M-face mesh at 1080p, 16

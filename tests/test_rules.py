@@ -72,6 +72,22 @@ def test_autotuning_keeps_the_fastest_megakernel_beside_its_pick(rules):
         assert got not in others and ms[got] == min(ms[k] for k in range(Tracer.KERNELS) if k not in others)
 
 
+def test_pooled_forms_close_to_the_fastest_are_timed_again(rules):
+    def ties(ms, pick):
+        ms = np.array(ms, np.float32)
+        return rules.probe_pooled_ties(ms.ctypes.data_as(C.c_void_p), pick)
+
+    ms = [9.0] * Tracer.KERNELS
+    ms[1], ms[2], ms[3] = 2.71, 2.67, 2.84
+    assert ties(ms, 2) == 0b0110
+    ms[3] = 2.82
+    assert ties(ms, 2) == 0b1110
+    ms[1] = ms[3] = 5.0
+    assert ties(ms, 2) == 0b0100
+    ms[15] = 2.0  # a megakernel is fastest: nothing to decide
+    assert ties(ms, 15) == 0
+
+
 @pytest.mark.parametrize("fails", [0, 1, 2, 99])
 @pytest.mark.parametrize("seed", range(6))
 def test_lanes_reserve_once_for_their_pooled_jobs(rules, seed, fails):
