@@ -6,7 +6,7 @@
 // different lobes, and the warps of an SM run different parts of a long code
 // (on the 1.3 M-face mesh 9.7 of 32 lanes were active in an instruction, and
 // waiting for instructions was the largest stall). Here a path's state sits
-// in memory (PW words in the pool of its block; the pools stay in L2), so
+// in memory (PW_WORDS words in the pool of its block), so
 // lanes are not bound to paths: in the trace phase they take the next ray of
 // the block's list as soon as theirs is done, and the shading phase runs each
 // kind of hit over the slots that hold it, 32 at a time. A block's warps run
@@ -17,13 +17,16 @@
 // Measured (B200, against the fastest megakernel form): the 1.3 M-face mesh at
 // 1080p, 16 spp, 8 bounces on its SAH tree 48.7 -> 27.8 ms (2.72 Grays/s);
 // the 65,536-face cloud at 256 x 256, 16 spp on its LBVH 26.5 -> 4.9 ms.
-// What is left: 42 % of issue slots used in the walk and the shading alike,
-// the rest waiting on L2 (tree, triangles, path state) and instructions.
-// Blocks of 512 threads, two an SM, beat 256 x 4 and 128 x 8 (28.7, 32.0 ms)
-// and 1,024 x 1 (31.7): more warps in one phase, but two phases an SM to
-// overlap; 64 registers beat 80 (31.8, 768 threads an SM) and 40 (34.4).
-// A warp-sized pool (64-256 slots) ran 41-117 ms: groups of 15-25 lanes, and
-// an SM's warps spread over all phases.
+// What is left (that mesh at 960 x 540, 4 spp, one launch): 52 % of issue slots
+// used, 17 of 32 lanes active, the rest waiting on memory past L1 (tree,
+// triangles, path state; 5.2 of 14.7 cycles an instruction) and at the phases'
+// barriers (2.7). A large frame's pools, 296 MB, go through DRAM: 1.1 TB/s.
+// At many samples blocks of 512 threads, two an SM, beat 256 x 4 and 128 x 8
+// (27.8 against 28.6 and 31.5 ms at 16 spp; 2.71, 2.67 and 2.83 at 1) and 1,024 x
+// 1 (31.7): more warps in one phase, but two phases an SM to overlap; 64
+// registers beat 80 (31.8, 768 threads an SM) and 40 (34.4). Frames of few
+// samples take 256 (rules.cuh). A warp-sized pool (64-256 slots) ran 41-117 ms:
+// small groups, and an SM's warps spread over all phases.
 //
 // A sample's arithmetic and its draws are those of render.cuh's `sample` in
 // the same order, one exception apart: a shadow ray is traced beside the
@@ -155,9 +158,8 @@ struct Pool {
 // bit. A ray's walk is walk_tree's (shade.cuh), step by step; what the warp
 // does next is one step for the lanes at an inner node or one triangle for
 // the lanes at a leaf. Taking both for whichever lanes were there cost a leaf
-// test in nearly every step (11 of 32 lanes active on the mesh's rays); the
-// lanes at a leaf wait until they are half as many as those at inner nodes
-// (19 of 32 active, 1 spp of the mesh at 1080p 5.3 -> 3.6 ms). A ray's own
+// test in nearly every step; the lanes at a leaf wait until they are half as many
+// as those at inner nodes (1 spp of the mesh at 1080p 5.3 -> 3.6 ms). A ray's own
 // order is not changed, so ties of two triangles at one t fall as before.
 template <int STATS, int P>
 __device__ __forceinline__ void pool_trace(const Scene& S, const Frame& F, const Pool<P>& of, Count& cnt) {
