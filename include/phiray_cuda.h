@@ -497,11 +497,11 @@ int32_t phx_tracer_destroy(phx_tracer tr);
 #define PHX_KERNEL_COUNT 20u
 int32_t phx_tracer_set_kernel(phx_tracer tr, uint32_t kernel);
 /* The autotuner: times every render kernel (and register budget) above on
- * `spp` samples of this scene and camera, keeps the fastest for the tracer
- * (and the fastest megakernel form for frames that one cannot trace; pooled
- * forms within 6 % are decided at eight times the samples) and returns its id;
- * ms (PHX_KERNEL_COUNT floats, may be NULL) gets each one's time. The
- * image is overwritten (the next sample starts over). Waits. */
+ * `spp` samples of this scene and camera, keeps the fastest for the tracer (of
+ * pooled forms within 6 % the one of the largest blocks; and the fastest
+ * megakernel form for frames that one cannot trace) and returns its id; ms
+ * (PHX_KERNEL_COUNT floats, may be NULL) gets each one's time. The image is
+ * overwritten (the next sample starts over). Waits. */
 int32_t phx_tracer_autotune(phx_tracer tr, const phx_camera* cam, uint32_t w, uint32_t h, uint32_t spp,
                             uint32_t* chosen, float* ms);
 /* Where thread-per-ray walks (phx_trace_rays under PHX_WALK_THREAD) keep

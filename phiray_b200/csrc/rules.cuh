@@ -39,18 +39,18 @@ inline bool pooled_id(uint32_t kernel) {
     return kernel >= PHX_KERNEL_STATE_MACHINE && kernel <= PHX_KERNEL_STATE_MACHINE_8;
 }
 
-// The pooled forms within 6 % of an autotuning's fastest time, as a mask of their
-// ids, if that time is one's: at few samples the last paths' end decides between
-// them, so such forms are timed again at POOL_TIE_SAMPLES times as many. (The 1.3
-// M-face mesh at 1080p, 512 / 256 / 128 threads: 2.71 / 2.67 / 2.83 ms at 1 spp,
-// either of the first two fastest by chance; 7.54 / 7.70 / 8.40 at 4, 27.8 / 28.6
-// / 31.5 at 16.)
-constexpr uint32_t POOL_TIE_SAMPLES = 8;
-inline uint32_t pooled_ties(const float* ms, uint32_t pick) {
-    uint32_t mask = 0;
-    for (uint32_t k = 0; k < PHX_KERNEL_COUNT && pooled_id(pick); k++)
-        if (pooled_id(k) && ms[k] <= 1.06f * ms[pick]) mask |= 1u << k;
-    return mask;
+// An autotuning's pick (of a frame that is not `full`), `fastest` by its times: of
+// pooled forms within 6 % of one another the one of the largest blocks. At few
+// samples the last paths' end decides between them, at many that form is ahead or
+// even. (512 / 256 / 128 threads: the 1.3 M-face mesh at 1080p 2.71 / 2.67 / 2.83 ms
+// at 1 spp, either of the first two fastest by chance; 7.54 / 7.70 / 8.40 at 4, 27.8
+// / 28.6 / 31.5 at 16; a scene of 60,000 faces at 512 x 512 3.59 / 3.62 / 3.66 and
+// 25.4 / 25.5 / 26.1.)
+inline uint32_t autotuned(const float* ms, uint32_t fastest) {
+    if (!pooled_id(fastest)) return fastest;
+    uint32_t k = PHX_KERNEL_STATE_MACHINE;
+    while (ms[k] > 1.06f * ms[fastest]) k++;
+    return k;
 }
 
 // The fastest megakernel form by the times of an autotuning: what a tracer

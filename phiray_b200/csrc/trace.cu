@@ -1585,41 +1585,23 @@ int32_t phx_tracer_autotune(phx_tracer tr, const phx_camera* cam, uint32_t w, ui
     PHX_TRY(use(tr->ctx));
     PHX_TRY(ensure_image(tr, w, h));
     Ctx* c = tr->ctx;
-    auto time = [&](uint32_t kernel, uint32_t samples, float* t) -> int32_t {
-        tr->kernel = kernel;
-        PHX_TRY(launch_render(tr, cam, w, h, 0, samples, 0, w * h));  // warm-up
+    float all[PHX_KERNEL_COUNT] = {};
+    uint32_t fastest = 0;
+    for (uint32_t k = 0; k < PHX_KERNEL_COUNT; k++) {
+        tr->kernel = k;
+        PHX_TRY(launch_render(tr, cam, w, h, 0, spp ? spp : 1, 0, w * h));  // warm-up
         PHX_CUDA(cudaEventRecord(tr->ev0, c->stream));
-        PHX_TRY(launch_render(tr, cam, w, h, 0, samples, 0, w * h));
+        PHX_TRY(launch_render(tr, cam, w, h, 0, spp ? spp : 1, 0, w * h));
         PHX_CUDA(cudaEventRecord(tr->ev1, c->stream));
         PHX_TRY(wait_stream(c->stream, 60000));
-        return cuda_check(cudaEventElapsedTime(t, tr->ev0, tr->ev1), "event");
-    };
-    const uint32_t samples = spp ? spp : 1;
-    float all[PHX_KERNEL_COUNT] = {};
-    uint32_t pick = 0;
-    for (uint32_t k = 0; k < PHX_KERNEL_COUNT; k++) {
-        PHX_TRY(time(k, samples, &all[k]));
-        if (all[k] < all[pick]) pick = k;
+        PHX_CUDA(cudaEventElapsedTime(&all[k], tr->ev0, tr->ev1));
+        if (all[k] < all[fastest]) fastest = k;
     }
-    const uint32_t ties = pooled_ties(all, pick);
-    if (ties & (ties - 1u)) {
-        float best = 0.0f;
-        for (uint32_t k = 0, first = 1; k < PHX_KERNEL_COUNT; k++) {
-            if (!((ties >> k) & 1u)) continue;
-            float t = 0.0f;
-            PHX_TRY(time(k, samples < 0xFFFFFFFFu / POOL_TIE_SAMPLES ? samples * POOL_TIE_SAMPLES : samples, &t));
-            if (first || t < best) {
-                best = t;
-                pick = k;
-            }
-            first = 0;
-        }
-    }
-    tr->kernel = pick;
+    tr->kernel = tr->forest || cam->grid > 0.0f ? fastest : autotuned(all, fastest);
     tr->mega = fastest_megakernel(all);
     if (ms) std::memcpy(ms, all, sizeof all);
     tr->have_last = false;  // the image holds the tuning frames: start over
-    if (chosen) *chosen = pick;
+    if (chosen) *chosen = tr->kernel;
     return read_status(c);
 }
 

@@ -5,7 +5,7 @@
 
 extern "C" int probe_aligned16(const void* p) { return phx::aligned16(p) ? 1 : 0; }
 
-extern "C" uint32_t probe_pooled_ties(const float* ms, uint32_t pick) { return phx::pooled_ties(ms, pick); }
+extern "C" uint32_t probe_autotuned(const float* ms, uint32_t fastest) { return phx::autotuned(ms, fastest); }
 
 extern "C" uint32_t probe_fastest_megakernel(const float* ms) { return phx::fastest_megakernel(ms); }
 

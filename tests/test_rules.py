@@ -72,20 +72,17 @@ def test_autotuning_keeps_the_fastest_megakernel_beside_its_pick(rules):
         assert got not in others and ms[got] == min(ms[k] for k in range(Tracer.KERNELS) if k not in others)
 
 
-def test_pooled_forms_close_to_the_fastest_are_timed_again(rules):
-    def ties(ms, pick):
-        ms = np.array(ms, np.float32)
-        return rules.probe_pooled_ties(ms.ctypes.data_as(C.c_void_p), pick)
+def test_of_pooled_forms_close_together_the_largest_blocks(rules):
+    def pick(*pooled, mega=9.0):
+        ms = np.full(Tracer.KERNELS, 9.0, np.float32)
+        ms[list(POOLED)], ms[15] = pooled, mega
+        return rules.probe_autotuned(ms.ctypes.data_as(C.c_void_p), int(np.argmin(ms)))
 
-    ms = [9.0] * Tracer.KERNELS
-    ms[1], ms[2], ms[3] = 2.71, 2.67, 2.84
-    assert ties(ms, 2) == 0b0110
-    ms[3] = 2.82
-    assert ties(ms, 2) == 0b1110
-    ms[1] = ms[3] = 5.0
-    assert ties(ms, 2) == 0b0100
-    ms[15] = 2.0  # a megakernel is fastest: nothing to decide
-    assert ties(ms, 15) == 0
+    assert pick(2.71, 2.67, 2.83) == 1
+    assert pick(2.84, 2.67, 2.83) == 2  # 512 threads 6.4 % behind
+    assert pick(1.87, 2.12, 1.50) == 3
+    assert pick(2.5, 2.6, 2.7) == 1
+    assert pick(2.71, 2.67, 2.83, mega=2.0) == 15
 
 
 @pytest.mark.parametrize("fails", [0, 1, 2, 99])
