@@ -448,9 +448,9 @@ int32_t phx_tracer_destroy(phx_tracer tr);
  * form an autotuning found fastest, or PHX_KERNEL_MEGAKERNEL. Its memory
  * follows the frame: 244 bytes a path, at most 8,192 paths a multiprocessor
  * (296 MB on 148), and 40 bytes a sample, at most 1 GiB or one sample a pixel;
- * the context keeps it for its next frames until it is destroyed (a program
- * that makes a tracer a frame would else map a gigabyte each time), a batch has
- * its own until phx_batch_clear. Scenes of instances and frames with the floor grid take a
+ * the context keeps it for its next frames until it is destroyed or another of
+ * its allocations finds no memory (a program that makes a tracer a frame would
+ * else map a gigabyte each time), a batch has its own until phx_batch_clear. Scenes of instances and frames with the floor grid take a
  * persistent kernel under these ids, whose lanes take pixels from a counter
  * and run the bounce loop as a state machine around one walk.
  * phx_tracer_autotune times them on the scene and keeps the fastest. */

@@ -54,8 +54,19 @@ struct Ctx {
     cudaMemPool_t pool = nullptr;   // device memory of the context's objects
     DevMem denoise_scratch;         // guide and ping-pong planes of phx_denoise
     PoolScratch path_pool;          // the pooled render's buffers
-    std::mutex path_pool_lock;      // from sizing them to the launches that use them
+    std::mutex path_pool_lock;      // from sizing them to the launches that use them (PathPoolHold)
     int live = 0;                   // buffers, passes, BVHs, tracers not yet freed
+};
+
+// The context's pooled buffers, held by this thread while it sizes them and
+// launches what uses them. An allocation that finds no memory gives them back,
+// but not those made under the hold.
+class PathPoolHold {
+    std::lock_guard<std::mutex> lock_;
+
+public:
+    explicit PathPoolHold(Ctx* c);
+    ~PathPoolHold();
 };
 
 // Sets the thread's last error text and returns `code`.

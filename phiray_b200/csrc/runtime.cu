@@ -17,6 +17,8 @@ namespace phx {
 static thread_local std::string g_last_error;
 // The context of this thread's last use(): DevMem::reserve draws on its pool.
 static thread_local Ctx* t_current = nullptr;
+// This thread holds some context's pooled buffers (PathPoolHold).
+static thread_local bool t_holds_pool = false;
 // Contexts not yet destroyed (a stale t_current is never dereferenced).
 static std::mutex g_ctx_mutex;
 static std::unordered_set<Ctx*> g_ctxs;
@@ -53,16 +55,37 @@ int32_t use(Ctx* c) {
     return PHX_OK;
 }
 
+PathPoolHold::PathPoolHold(Ctx* c) : lock_(c->path_pool_lock) { t_holds_pool = true; }
+PathPoolHold::~PathPoolHold() { t_holds_pool = false; }
+
+// The pooled buffers given back to an allocation that found no memory (up to
+// 1.3 GB that only make frames faster); false when there are none to give.
+static bool give_back(Ctx* c) {
+    if (t_holds_pool) return false;
+    const PathPoolHold hold(c);
+    if (!c->path_pool.state.ptr && !c->path_pool.out.ptr) return false;
+    c->path_pool.state.release();
+    c->path_pool.out.release();
+    if (wait_stream(c->stream, 0) < 0) return false;
+    if (c->pool) cudaMemPoolTrimTo(c->pool, 0);
+    return true;
+}
+
 int32_t ctx_alloc(Ctx* c, void** p, size_t bytes) {
     *p = nullptr;
-    if (!c->pool) return cuda_check(cudaMalloc(p, bytes), "cudaMalloc");
     // An allocation recorded into a graph would belong to the graph: refuse
     // one made while the context's stream is being captured.
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    PHX_CUDA(cudaStreamIsCapturing(c->stream, &cs));
+    if (c->pool) PHX_CUDA(cudaStreamIsCapturing(c->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return fail(PHX_ERR_INVALID, "allocation of %zu bytes while the stream is captured", bytes);
-    PHX_CUDA(cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream));
+    auto get = [&] {
+        return c->pool ? cuda_check(cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream), "cudaMallocFromPoolAsync")
+                       : cuda_check(cudaMalloc(p, bytes), "cudaMalloc");
+    };
+    int32_t rc = get();
+    if (rc == PHX_ERR_OOM && give_back(c)) rc = get();
+    if (rc < 0 || !c->pool) return rc;
     // Kernels stage rows with 16-byte copies and vector loads: keep the
     // 256-byte alignment cudaMalloc gives.
     if ((uintptr_t)*p & 255u) {

@@ -1195,7 +1195,7 @@ int32_t launch_frame(phx_tracer tr, const Frame& F, f3 sun, uint32_t first_px, u
     if (count_px && !recorded) {
         PoolPlan plan;
         PHX_TRY(plan_pooled(kernel, stats, c->sms, count_px, F.spp, plan));
-        std::lock_guard<std::mutex> lock(c->path_pool_lock);
+        const PathPoolHold hold(c);
         int32_t rc = c->path_pool.state.reserve(plan.state);
         if (rc >= 0) rc = c->path_pool.out.reserve(plan.out);
         if (rc >= 0) return render_pooled(kernel, stats, L, plan, c->path_pool.state.ptr, c->path_pool.out.ptr);
